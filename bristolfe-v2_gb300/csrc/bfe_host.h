@@ -126,6 +126,21 @@ inline std::vector<unsigned char> cast_bytes(const double* v, int64_t count) {
 std::vector<unsigned char> cast_bytes(int prec, const double* v, int64_t count);
 int upload_bytes(DevBuf<unsigned char>& d, const std::vector<unsigned char>& h);
 
+// Partition of a plan's operator for the one-source march that stays on the
+// chip (bfe_onchip_host.cpp), built on the first run that can use it.
+struct Onchip {
+  int state = 0;                    // 0: not built, 1: usable, -1: does not fit
+  bfe::OnchipArgs args{};
+  std::vector<int32_t> part_slice;  // n_parts + 1
+  std::vector<int64_t> need;        // shared memory of each part without forcing and cached operator
+  std::vector<int32_t> op_bytes;    // and of its operator
+  uint32_t next_tag = 0;
+  DevBuf<int32_t> d_part, d_off, d_word, d_bytes, d_cnt, d_halo, d_vptr, d_vhalo;
+  DevBuf<uint16_t> flags, order, z_lcol;
+  DevBuf<unsigned char> blocks, xch, xchv;
+  DevBuf<ushort4> lref;
+};
+
 }  // namespace bfe_host
 
 struct bfe_plan {
@@ -141,6 +156,8 @@ struct bfe_plan {
   bfe_host::DevBuf<uint32_t> col;
   bfe_host::DevBuf<unsigned char> val;        // double or float
   bfe_host::DevBuf<unsigned char> rowc;       // double or float
+  std::vector<int32_t> h_slice_ptr;
+  std::unique_ptr<bfe_host::Onchip> onchip{new bfe_host::Onchip()};
   std::vector<uint32_t> h_base;     // node-block base per row
   std::vector<double> h_acoef;      // forcing coefficient per row (diagonal of A)
   // interface correction
@@ -149,13 +166,14 @@ struct bfe_plan {
   std::vector<int32_t> h_int_row;
   bfe_host::DevBuf<int32_t> int_row, z_ptr, z_col;
   bfe_host::DevBuf<unsigned char> z_val;
+  std::vector<int32_t> h_z_ptr, h_z_col;
   // statistics
   int64_t nnz_operator = 0;         // stored (unpadded) entries
   int64_t nnz_padded = 0;
   int64_t n_direct_rows = 0;
   bool timing = false;
   double time_limit_s = 0.0;        // wall-clock limit of a run (0 = none)
-  bfe_host::DevBuf<int> d_flag;     // non-finite flag of the last run
+  bfe_host::DevBuf<int> d_flag;     // non-finite flag of the last run, and a march's wait-ran-out flag
   bfe_stats last{};
   // autotuned batched-kernel variant per R (chosen on the first run with that R)
   std::map<int64_t, int> variant_of_R;
@@ -215,6 +233,11 @@ int prepare_run(bfe_plan* pl, std::vector<ForceEntry>& frc, const std::vector<in
                 int64_t R, int64_t n_t, int64_t n_sig, const double* d_sig64, double* d_hist,
                 cudaStream_t st, RunArrays& ra, bfe::StepArgs& a);
 int execute(bfe_plan* pl, RunSpec& rs, cudaStream_t st);
+// Builds the plan's on-chip partition if it has none yet (state says whether
+// it is usable afterwards); with the run's forced rows, its shared memory and
+// thread count are set. false: this run does not fit.
+int onchip_prepare(bfe_plan* pl, cudaStream_t st);
+bool onchip_fit(bfe_plan* pl, const std::vector<ForceEntry>& frc, bfe::OnchipArgs& o);
 bool outputs_valid(int rc);
 int64_t first_nonzero_column(const double* frcs, int64_t rows, int64_t n_t, int64_t R);
 int check_time(bfe_plan* pl, int64_t n_t, const double* time);

@@ -139,6 +139,66 @@ cudaError_t launch_frame(const StepArgs& a, int precision, double* fld, int64_t 
 cudaError_t launch_cast_f64_to_f32(const double* in, float* out, int64_t n, cudaStream_t s);
 cudaError_t launch_advance(int64_t* ti_dev, int64_t k, cudaStream_t s);
 
+// One-source march that keeps state and operator on the chip (bfe_onchip.cu).
+// Device data of a plan's partition; the forcing, monitor and interface lists
+// are those of StepArgs.
+struct OnchipArgs {
+  int32_t n_parts, threads, smem;   // CTAs, threads per CTA, dynamic shared memory
+  const int32_t* part_slice;        // first slice of each part (n_parts + 1)
+  const int32_t* halo_cnt;          // halo rows of each part ...
+  const int32_t* halo_row;          // ... halo_row[p * halo_cap + k]
+  int32_t halo_cap;
+  const uint16_t* flags;            // per row: exported, interface, number
+  const uint16_t* order;            // slices of each part in order of work
+  const void* blocks;               // operator block of each slice: coefficients, entries in chunks
+  const int32_t* block_off;         // its offset in units of 16 bytes
+  const int32_t* slice_word;        // its width and kind
+  const int32_t* op_bytes;          // bytes of each part's blocks
+  int32_t depth, slot_bytes;        // slots per warp for streamed chunks
+  const ushort4* lref;              // FP32: window indices of a cut block's reference values
+  const int32_t* vhalo_ptr;         // interface values each part reads (n_parts + 1)
+  const int32_t* vhalo;             // their interface numbers
+  const uint16_t* z_lcol;           // columns of Z as local interface numbers
+  void* xch;                        // exchange buffers of states and interface values,
+  int64_t x_stride;                 // two each, x_stride / xv_stride values apart
+  void* xchv;
+  int64_t xv_stride;
+  uint32_t tag0;                    // step ti carries tag0 + ti
+  int* err;                         // set when a wait ran out
+};
+// Inputs and outputs of building it.
+struct OnchipBuild {
+  int32_t n, n_parts, max_part_slices, max_words, max_window, halo_cap, n_int;
+  const int32_t* part_slice;
+  const int32_t* slice_ptr;
+  const int32_t* block_off;
+  const uint32_t* col;
+  const void* val;
+  const void* rowc;
+  const uint32_t* base;             // FP32: node-block base per row
+  const int32_t* int_row;
+  const uint8_t* v_exported;        // per interface number
+  int32_t* halo_cnt;
+  int32_t* halo_row;
+  uint8_t* exported;                // scratch, zeroed: n
+  uint8_t* adj;                     // scratch, zeroed: n_parts^2
+  uint16_t* flags;
+  uint16_t* order;
+  void* blocks;
+  int32_t* slice_word;
+  int32_t* op_bytes;
+  ushort4* lref;
+  uint8_t* pos;                     // FP32 scratch: n
+  int* slot_bytes;                  // of the largest chunk, zeroed
+  int* fail;                        // set when the operator does not fit the form
+};
+int onchip_block_bound(int precision, int width);    // most bytes of a slice of this width
+cudaError_t launch_onchip_build(const OnchipBuild& b, int precision, cudaStream_t s);
+// n_steps steps from ti0. fresh: from rest, else from a.u_n, a.u_prev. The
+// newest state is written to a.u_new, the one before it to a.u_prev.
+cudaError_t launch_onchip(const OnchipArgs& o, const StepArgs& a, int precision, int64_t ti0, int64_t n_steps,
+                          int fresh, cudaStream_t s);
+
 // Prescribed displacements of the v5 scheme (fn_explicit_dynamic_solver_v5.m
 // :142-188). The main step kernel advances every row with the velocity
 // u_n - u_{n-1}; the v5 kernel then handles the rows that differ from that:

@@ -1,0 +1,1036 @@
+// One-source march that stays on the chip (sm_103a).
+//
+// A march of one source (fn_explicit_dynamic_solver_v6.m:180-218 for one load
+// step) on a model of up to about 1.5 million DOFs is short work per step: a
+// kernel launch per step spends its few microseconds on the launch, on the
+// chain column index -> gathered value, and on reading the same operator
+// again. Here ONE cooperative launch marches all steps. Every CTA (one per
+// SM) owns a contiguous range of 32-row slices and keeps in shared memory
+//   * the two newest states of its rows, and the values of the rows of other
+//     CTAs that its rows couple to (halo),
+//   * as many slices of its operator as fit; the others stream from L2 by
+//     bulk copies into a slot or two per warp. The operator does not change,
+//     so a slot's next copy is issued as soon as the slot has been read, also
+//     across the end of a step.
+// Operator entries carry 16-bit indices into the CTA's shared window, so a
+// gather is one shared-memory load.
+//
+// Exchange: after computing a row that others read, its owner writes the
+// value to a global buffer together with the step number, in one store per 4
+// bytes of value and 4 of step number; readers poll the value itself. One L2
+// round trip replaces data, fence, flag, poll, read. Two buffers by step
+// parity suffice: a CTA publishes step t + 2 only after it has read step
+// t + 1 of every CTA that reads from it (reading is made symmetric when the
+// partition is built), and those publish t + 1 after having read step t.
+// Every poll is bounded in time; when one runs out the kernel sets *err and
+// all CTAs leave, and the host marches with one launch per step instead.
+//
+// The arithmetic of a row is that of step_f64_r1 / step_f32_r1 and
+// interface_fixup_r1 (bfe_kernels.cu), term for term in the same order, so
+// the results are the same bits.
+#include <cuda_runtime.h>
+#include <cstdint>
+#include <type_traits>
+
+#include "bfe_device.cuh"
+#include "bfe_internal.h"
+
+namespace bfe {
+
+namespace {
+
+// Flag word of a row (shared memory): bits 0-3; in 4-6 the row's place in its
+// node block (FP32: reference values are the block's rows), kOcCut when the
+// block is cut by the part's edge; interface number in 7-15.
+constexpr uint32_t kOcExport = 1, kOcInterface = 2, kOcForced = 4, kOcExportV = 8;
+constexpr int kOcPosShift = 4, kOcIntShift = 7;
+constexpr uint32_t kOcCut = 7, kOcMaxInt = 511;
+
+// ---------------------------------------------------------------------------
+// Exchange words: value and step number travel in the same 8 bytes.
+__device__ __forceinline__ void xput(double* base, size_t i, double v, uint32_t tag) {
+  const uint32_t lo = (uint32_t)__double2loint(v), hi = (uint32_t)__double2hiint(v);
+  asm volatile("st.volatile.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(reinterpret_cast<uint4*>(base) + i), "r"(lo),
+               "r"(tag), "r"(hi), "r"(tag)
+               : "memory");
+}
+__device__ __forceinline__ void xput(float* base, size_t i, float v, uint32_t tag) {
+  asm volatile("st.volatile.global.v2.u32 [%0], {%1,%2};" ::"l"(reinterpret_cast<uint2*>(base) + i),
+               "r"(__float_as_uint(v)), "r"(tag)
+               : "memory");
+}
+__device__ __forceinline__ bool xtry(const double* base, size_t i, uint32_t tag, double& v) {
+  uint32_t a, b, c, d;
+  asm volatile("ld.volatile.global.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(a), "=r"(b), "=r"(c), "=r"(d)
+               : "l"(reinterpret_cast<const uint4*>(base) + i)
+               : "memory");
+  v = __hiloint2double((int)c, (int)a);
+  return b == tag && d == tag;
+}
+__device__ __forceinline__ bool xtry(const float* base, size_t i, uint32_t tag, float& v) {
+  uint32_t a, b;
+  asm volatile("ld.volatile.global.v2.u32 {%0,%1}, [%2];"
+               : "=r"(a), "=r"(b)
+               : "l"(reinterpret_cast<const uint2*>(base) + i)
+               : "memory");
+  v = __uint_as_float(a);
+  return b == tag;
+}
+
+// About two seconds of the SM clock: far above any wait of a running march.
+constexpr long long kSpinClocks = 4000000000ll;
+
+// A value from exchange slot i, polled until it carries tag. false: gave up.
+template <typename T>
+__device__ __noinline__ bool xwait(const T* xbuf, uint32_t i, uint32_t tag, T& v, int* err) {
+  long long t0 = 0;
+  T x;
+  for (uint32_t spin = 1; !xtry(xbuf, i, tag, x); ++spin) {
+    if ((spin & 255u) == 0) {
+      const long long now = clock64();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > kSpinClocks) atomicExch(err, 1);
+      if (*reinterpret_cast<volatile int*>(err)) return false;
+    }
+  }
+  v = x;
+  return true;
+}
+// The values of exchange slots idx[tid], idx[tid + nt], ... into dst. The
+// thread's first N slots are held in registers (ix) and their first polls are
+// in flight together.
+template <typename T, int N>
+__device__ __forceinline__ bool receive(const T* xbuf, const int32_t* __restrict__ idx, int count, const int (&ix)[N],
+                                        uint32_t tag, T* dst, int tid, int nt, int* err) {
+  if (tid >= count) return true;
+  T v[N];
+  bool got[N], ok = true;
+#pragma unroll
+  for (int j = 0; j < N; ++j) got[j] = tid + j * nt >= count || xtry(xbuf, (uint32_t)ix[j], tag, v[j]);
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    if (!got[j]) ok &= xwait(xbuf, (uint32_t)ix[j], tag, v[j], err);
+    if (tid + j * nt < count) dst[tid + j * nt] = v[j];
+  }
+  for (int k = tid + N * nt; k < count && ok; k += nt) {
+    T x;
+    ok = xwait(xbuf, (uint32_t)__ldg(idx + k), tag, x, err);
+    dst[k] = x;
+  }
+  return ok;
+}
+
+__device__ __forceinline__ int lower_bound_sm(const int32_t* a, int n, int key) {
+  int lo = 0, hi = n;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (a[mid] < key) lo = mid + 1; else hi = mid;
+  }
+  return lo;
+}
+
+// Bulk copies of operator chunks into shared memory, completion on an
+// mbarrier (one phase per copy).
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void bar_init(uint64_t* bar) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n\tfence.mbarrier_init.release.cluster;" ::"r"(smem_addr(bar))
+               : "memory");
+}
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");    // after the warp's reads of the old contents
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_addr(dst)),
+      "l"(src), "r"(bytes), "r"(smem_addr(bar))
+      : "memory");
+}
+// Wait for the phase with this parity; false after about two seconds.
+__device__ bool bar_wait(uint64_t* bar, uint32_t parity, int* err) {
+  long long t0 = 0;
+  for (uint32_t spin = 1;; ++spin) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tmbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(done)
+        : "r"(smem_addr(bar)), "r"(parity)
+        : "memory");
+    if (done) return true;
+    if ((spin & 63u) == 0) {
+      const long long now = clock64();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > kSpinClocks) {
+        atomicExch(err, 1);
+        return false;
+      }
+    }
+  }
+}
+
+// Operator blocks. The block of a slice (32 rows, lane = row) is the rows'
+// update coefficients followed by chunks of entries; a chunk is what one bulk
+// copy moves, about 3 KB. The entries of a slice are of one kind:
+//   0, 1  single entries in pairs: values as T2 per lane, then the pair's two
+//         window indices in one word. Kind 0 is any row (FP64: all rows).
+//         FP32 kind 0 names in the index's low bits which of the row's three
+//         reference values is subtracted (3: none); kind 1 are rows whose
+//         entries all subtract the row's own value (fluid).
+//   2, 3  FP32 rows whose entries subtract the matching DOF of the row's own
+//         node, by neighbour node: the node's 2 or 3 values (absent entries
+//         as zeros), one window index for all of them.
+// FP32 indices are byte offsets into the window (4 x index, at most 64 KB).
+// An entry of kind 0 takes about 14 instructions, one of kind 2 under 4, and
+// FP32 rows are bound by instruction issue: C1's 961,641 rows took 12.4 us of
+// a step as kind 0.
+template <typename T> __host__ __device__ constexpr int coef_bytes() { return 32 * (int)sizeof(T); }
+// Units (pairs or nodes) of a full chunk, bytes of a chunk of u units.
+template <typename T>
+__host__ __device__ inline int chunk_units(int kind) { return sizeof(T) == 8 ? 4 : kind == 3 ? 6 : 8; }
+template <typename T>
+__host__ __device__ inline int units_bytes(int kind, int u) {
+  if (kind < 2) return u * 64 * ((int)sizeof(T) + 2);
+  return u * kind * 128 + ((u + 1) >> 1) * 128;
+}
+// Units of a slice of so many entries (kinds 0, 1) or nodes per row.
+__host__ __device__ inline int slice_units(int kind, int width) { return kind < 2 ? (width + 1) >> 1 : width; }
+template <typename T>
+__host__ __device__ inline int block_bytes(int kind, int units) {
+  const int cu = chunk_units<T>(kind);
+  return coef_bytes<T>() + units / cu * units_bytes<T>(kind, cu) + units_bytes<T>(kind, units % cu);
+}
+// Space kept for the block of a slice of this many entries per row; a slice
+// that would need more as kind 2 or 3 (many absent entries) stays kind 0.
+template <typename T>
+__host__ __device__ inline int block_bound(int width) {
+  const int b = block_bytes<T>(0, slice_units(0, width));
+  return sizeof(T) == 8 ? b : (b + b / 4 + 512) & ~15;
+}
+// Offset and bytes of chunk c in its block; chunk 0 includes the coefficients.
+template <typename T>
+__device__ __forceinline__ int chunk_offset(int kind, int c) {
+  return c == 0 ? 0 : coef_bytes<T>() + c * units_bytes<T>(kind, chunk_units<T>(kind));
+}
+template <typename T>
+__device__ __forceinline__ int chunk_bytes(int kind, int c, int units) {
+  const int cu = chunk_units<T>(kind);
+  return units_bytes<T>(kind, min(cu, units - c * cu)) + (c == 0 ? coef_bytes<T>() : 0);
+}
+// Slice word: width (FP64: entries, FP32: units), kind, resident, more than
+// one chunk, local slice.
+__device__ __forceinline__ int sl_width(int y) { return y & 0x7ff; }
+__device__ __forceinline__ int sl_kind(int y) { return (y >> 11) & 3; }
+template <typename T>
+__device__ __forceinline__ int sl_units(int y) { return sizeof(T) == 8 ? (sl_width(y) + 1) >> 1 : sl_width(y); }
+constexpr int kSlResident = 1 << 13, kSlChunks = 1 << 14, kSlLocalShift = 15, kSlMaxWidth = 0x7ff;
+
+// Value at a byte offset of shared memory.
+template <typename T>
+__device__ __forceinline__ T sm_at(const unsigned char* sm, uint32_t bytes) {
+  return *reinterpret_cast<const T*>(sm + bytes);
+}
+
+// Adds the entries of a chunk (blk: its first value) to a row's sum; au is
+// the byte offset of the state in shared memory, w the entries (FP64) or
+// units (FP32) of the chunk.
+__device__ __forceinline__ double row_sum(double acc, const unsigned char* blk, int lane, int, int w,
+                                          const unsigned char* sm, uint32_t au, const float*) {
+  const int np = w >> 1;
+  const double2* v = reinterpret_cast<const double2*>(blk) + lane;
+  const uint32_t* c = reinterpret_cast<const uint32_t*>(blk + ((w + 1) >> 1) * 512) + lane;
+#pragma unroll 4
+  for (int k = 0; k < np; ++k) {
+    const double2 x = v[32 * k];
+    const uint32_t cc = c[32 * k];
+    acc = fma(x.x, sm_at<double>(sm, au + 8 * (cc & 0xffffu)), acc);
+    acc = fma(x.y, sm_at<double>(sm, au + 8 * (cc >> 16)), acc);
+  }
+  if (w & 1) acc = fma(v[32 * np].x, sm_at<double>(sm, au + 8 * (c[32 * np] & 0xffffu)), acc);
+  return acc;
+}
+__device__ __forceinline__ float ref_of(uint32_t s, const float* ref) {
+  const float lo = (s & 1u) ? ref[1] : ref[0], hi = (s & 1u) ? 0.f : ref[2];
+  return (s & 2u) ? hi : lo;
+}
+__device__ __forceinline__ float row_sum(float acc, const unsigned char* blk, int lane, int kind, int u,
+                                         const unsigned char* sm, uint32_t au, const float* ref) {
+  if (kind == 2) {
+    const float2* v = reinterpret_cast<const float2*>(blk) + lane;
+    const uint32_t* c = reinterpret_cast<const uint32_t*>(blk + u * 256) + lane;
+    const float r0 = ref[0], r1 = ref[1];
+#pragma unroll 3
+    for (int k = 0; k < u >> 1; ++k, v += 64, c += 32) {
+      const uint32_t c0 = au + (*c & 0xffffu), c1 = au + (*c >> 16);
+      const float2 x = v[0], y = v[32];
+      acc = fmaf(x.x, sm_at<float>(sm, c0) - r0, acc);
+      acc = fmaf(x.y, sm_at<float>(sm, c0 + 4) - r1, acc);
+      acc = fmaf(y.x, sm_at<float>(sm, c1) - r0, acc);
+      acc = fmaf(y.y, sm_at<float>(sm, c1 + 4) - r1, acc);
+    }
+    if (u & 1) {
+      const uint32_t c0 = au + (*c & 0xffffu);
+      acc = fmaf(v->x, sm_at<float>(sm, c0) - r0, acc);
+      acc = fmaf(v->y, sm_at<float>(sm, c0 + 4) - r1, acc);
+    }
+  } else if (kind == 1) {
+    const float2* v = reinterpret_cast<const float2*>(blk) + lane;
+    const uint32_t* c = reinterpret_cast<const uint32_t*>(blk + u * 256) + lane;
+    const float r0 = ref[0];
+#pragma unroll 3
+    for (int k = 0; k < u; ++k, v += 32, c += 32) {
+      const float2 x = *v;
+      const uint32_t c0 = au + (*c & 0xffffu), c1 = au + (*c >> 16);
+      acc = fmaf(x.x, sm_at<float>(sm, c0) - r0, acc);
+      acc = fmaf(x.y, sm_at<float>(sm, c1) - r0, acc);
+    }
+  } else if (kind == 3) {
+    const float* v = reinterpret_cast<const float*>(blk) + lane;
+    const uint32_t* c = reinterpret_cast<const uint32_t*>(blk + u * 384) + lane;
+    const float r0 = ref[0], r1 = ref[1], r2 = ref[2];
+#pragma unroll 3
+    for (int k = 0; k < u >> 1; ++k, v += 192, c += 32) {
+      const uint32_t c0 = au + (*c & 0xffffu), c1 = au + (*c >> 16);
+      acc = fmaf(v[0], sm_at<float>(sm, c0) - r0, acc);
+      acc = fmaf(v[32], sm_at<float>(sm, c0 + 4) - r1, acc);
+      acc = fmaf(v[64], sm_at<float>(sm, c0 + 8) - r2, acc);
+      acc = fmaf(v[96], sm_at<float>(sm, c1) - r0, acc);
+      acc = fmaf(v[128], sm_at<float>(sm, c1 + 4) - r1, acc);
+      acc = fmaf(v[160], sm_at<float>(sm, c1 + 8) - r2, acc);
+    }
+    if (u & 1) {
+      const uint32_t c0 = au + (*c & 0xffffu);
+      acc = fmaf(v[0], sm_at<float>(sm, c0) - r0, acc);
+      acc = fmaf(v[32], sm_at<float>(sm, c0 + 4) - r1, acc);
+      acc = fmaf(v[64], sm_at<float>(sm, c0 + 8) - r2, acc);
+    }
+  } else {
+    const float2* v = reinterpret_cast<const float2*>(blk) + lane;
+    const uint32_t* c = reinterpret_cast<const uint32_t*>(blk + u * 256) + lane;
+#pragma unroll 2
+    for (int k = 0; k < u; ++k, v += 32, c += 32) {
+      const uint32_t c0 = *c & 0xffffu, c1 = *c >> 16;
+      acc = fmaf(v->x, sm_at<float>(sm, au + (c0 & 0xfffcu)) - ref_of(c0 & 3u, ref), acc);
+      acc = fmaf(v->y, sm_at<float>(sm, au + (c1 & 0xfffcu)) - ref_of(c1 & 3u, ref), acc);
+    }
+  }
+  return acc;
+}
+
+// New value r of a row from its sum, and what its interface correction
+// starts from (v).
+__device__ __forceinline__ void row_update(double acc, double ui, double up, double rc, bool forced, double f,
+                                           int base_prev, double& r, double& v) {
+  r = acc + rc * up;
+  if (forced) r += f;
+  v = base_prev ? (r - up) : (ui - up);
+}
+__device__ __forceinline__ void row_update(float acc, float ui, float up, float rc, bool forced, float f,
+                                           int base_prev, float& r, float& v) {
+  float d, err;
+  two_sum(ui, -up, d, err);
+  float inc = fmaf(rc, d, -acc);
+  if (forced) inc += f;
+  inc = fmaf(rc, err, inc);
+  r = ui + inc;
+  v = base_prev ? (d + err + inc) : (d + err);
+}
+
+__device__ __forceinline__ double round_mul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float round_mul(float a, float b) { return __fmul_rn(a, b); }
+
+// ---------------------------------------------------------------------------
+// The march, one CTA of NT threads or fewer per part.
+//
+// What bounds it: FP64 rows the FP64 pipe (2 multiply-adds per clock and SM);
+// FP32 rows of large models the stream of operator chunks from L2 (about 4.5
+// TB/s over all SMs) and instruction issue; small models the exchange of a
+// step, about a microsecond from a value's store to its use in another CTA.
+// Measured per step of a 500-step run against one launch per step from a
+// graph, GB300 (us): plate of 40,602 DOF FP64 2.9 / 6.2, FP32 2.3 / 6.0;
+// coupled 241,579 DOF FP64 8.3 / 13.1, FP32 4.5 / 9.3; coupled 961,641 DOF
+// FP32 12.5 / 17.1; bricks of 202,878 DOF FP32 15.7 / 29.8.
+//
+// Per step: rows (interface and exported slices first, so that
+// their values travel while the others are computed), interface correction,
+// halo of the new state. A monitor's sample and a frame of state t are
+// written during step t + 1, when both states are still on chip.
+template <typename T, bool INT, int NT>
+__global__ void __launch_bounds__(NT, 1) march_onchip(OnchipArgs o, StepArgs a, int64_t ti0, int64_t n_steps,
+                                                         int fresh) {
+  using T2 = typename Vec2<T>::type;
+  extern __shared__ __align__(16) unsigned char sm[];
+  const int p = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
+  const int warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
+  const int s0 = o.part_slice[p], s1 = o.part_slice[p + 1];
+  const int ns = s1 - s0, row0 = s0 * kSlice, rpad = ns * kSlice;
+  const int rows = min(a.n - row0, rpad);
+  const int H = o.halo_cnt[p];
+  const int32_t* hrow = o.halo_row + (size_t)p * o.halo_cap;
+  const int W = (rpad + H + 2 + 3) & ~3;            // two rows of slack for unused reference values
+  // this CTA's forced rows, monitors and interface rows (sorted global lists)
+  const int f0 = lower_bound_i32(a.frc_row, a.n_frc, row0);
+  const int nf = lower_bound_i32(a.frc_row, a.n_frc, row0 + rows) - f0;
+  const int m0 = lower_bound_i32(a.mon_row, a.n_mon, row0);
+  const int nm = lower_bound_i32(a.mon_row, a.n_mon, row0 + rows) - m0;
+  int t0 = 0, ni = 0, nv = 0, nz = 0, zb = 0;
+  const int32_t* vrow = nullptr;
+  if (INT) {
+    t0 = lower_bound_i32(a.int_row, a.n_int, row0);
+    ni = lower_bound_i32(a.int_row, a.n_int, row0 + rows) - t0;
+    nv = o.vhalo_ptr[p + 1] - o.vhalo_ptr[p];
+    vrow = o.vhalo + o.vhalo_ptr[p];
+    zb = __ldg(a.z_ptr + t0);
+    nz = __ldg(a.z_ptr + t0 + ni) - zb;
+  }
+  // shared memory
+  T* U0 = reinterpret_cast<T*>(sm);
+  T* U1 = U0 + W;
+  T* vs = U1 + W;                                   // interface differences: own, then halo
+  T* zv = vs + (INT ? ((ni + nv + 1) & ~1) : 0);
+  T* fs = zv + (INT ? ((nz + 1) & ~1) : 0);         // forcing terms of two steps
+  int2* sd = reinterpret_cast<int2*>(fs + ((2 * nf + 1) & ~1));   // slices in order
+  int32_t* fr = reinterpret_cast<int32_t*>(sd + ns);              // forced rows (local)
+  int32_t* zp = fr + nf;
+  uint16_t* zc = reinterpret_cast<uint16_t*>(zp + (INT ? ni + 1 : 0));
+  uint16_t* zr = zc + (INT ? ((nz + 1) & ~1) : 0);
+  uint16_t* fl = zr + (INT ? ((ni + 1) & ~1) : 0);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sm + ((reinterpret_cast<unsigned char*>(fl + rpad) - sm + 15) & ~15));
+  unsigned char* cache = reinterpret_cast<unsigned char*>(bars + ((nw * o.depth + 1) & ~1));
+
+  for (int r = tid; r < rpad; r += nt) fl[r] = r < rows ? __ldg(o.flags + row0 + r) : 0;
+  for (int k = tid; k < nf; k += nt) fr[k] = __ldg(a.frc_row + f0 + k) - row0;
+  if (INT) {
+    for (int k = tid; k <= ni; k += nt) zp[k] = __ldg(a.z_ptr + t0 + k) - zb;
+    for (int k = tid; k < ni; k += nt) zr[k] = (uint16_t)(__ldg(a.int_row + t0 + k) - row0);
+    for (int k = tid; k < nz; k += nt) {
+      zc[k] = __ldg(o.z_lcol + zb + k);
+      zv[k] = __ldg(static_cast<const T*>(a.z_val) + zb + k);
+    }
+  }
+  // slices in order: {block offset / 16, slice word}
+  for (int j = tid; j < ns; j += nt) {
+    const int ls = __ldg(o.order + s0 + j);
+    const int y = __ldg(o.slice_word + s0 + ls);
+    sd[j] = make_int2(__ldg(o.block_off + s0 + ls),
+                      y | (ls << kSlLocalShift) | (sl_units<T>(y) > chunk_units<T>(sl_kind(y)) ? kSlChunks : 0));
+  }
+  for (int k = tid; k < nw * o.depth; k += nt) bar_init(bars + k);
+  __syncthreads();
+  for (int k = tid; k < nf; k += nt) fl[fr[k]] |= (uint16_t)kOcForced;
+  // Resident slices: all of them when they fit, else what the slots leave
+  // room for, spread evenly over the order so that a warp computes a resident
+  // slice while its slot is filled.
+  const bool stream = __ldg(o.op_bytes + p) > o.smem - (int)(cache - sm);
+  unsigned char* ring = cache;
+  if (stream) cache += nw * o.depth * o.slot_bytes;
+  const unsigned char* gblk = static_cast<const unsigned char*>(o.blocks);
+  if (tid == 0) {
+    const int room = o.smem - (int)(cache - sm);
+    const float share = stream ? (float)room / (float)__ldg(o.op_bytes + p) : 1.f;
+    float due = 0.f;
+    int used = 0;
+    for (int m0 = 0; m0 < ns; m0 += nw) {               // one slice of every warp at a time
+      due += share;
+      if (stream && due < 1.f) continue;
+      due -= 1.f;
+      for (int j = m0; j < min(m0 + nw, ns); ++j) {
+        const int y = sd[j].y, bytes = block_bytes<T>(sl_kind(y), sl_units<T>(y));
+        if (used + bytes > room) break;
+        used += bytes;
+        sd[j].y = y | kSlResident;
+      }
+    }
+  }
+  __syncthreads();
+  {
+    int off = 0;
+    for (int j = 0; j < ns; ++j) {
+      const int2 d = sd[j];
+      if (!(d.y & kSlResident)) continue;
+      const int bytes = block_bytes<T>(sl_kind(d.y), sl_units<T>(d.y));
+      if (j % nw == warp) {
+        const int4* src = reinterpret_cast<const int4*>(gblk + (size_t)d.x * 16);
+        for (int k = lane; k < bytes / 16; k += 32) reinterpret_cast<int4*>(cache + off)[k] = __ldg(src + k);
+        __syncwarp();
+        if (lane == 0) sd[j].x = off;
+      }
+      off += bytes;
+    }
+  }
+  __syncthreads();
+  // this warp's slots: the chunk (ij, ic) to copy next, copies left to issue
+  int ij = warp, ic = 0;
+  int64_t to_issue = 0;
+  int waiting = 0, w_slot = 0, i_slot = 0;              // copies in flight, slot to read, slot to fill
+  uint32_t w_parity = 0;
+  if (stream)
+    for (int j = warp; j < ns; j += nw)
+      if (!(sd[j].y & kSlResident)) {
+        const int kd = sl_kind(sd[j].y), cu = chunk_units<T>(kd);
+        to_issue += max(1, (sl_units<T>(sd[j].y) + cu - 1) / cu) * n_steps;
+      }
+  auto issue = [&]() {
+    if (to_issue == 0) return;
+    while (sd[ij].y & kSlResident) {
+      ij += nw;
+      if (ij >= ns) ij = warp;
+    }
+    const int2 d = sd[ij];
+    const int kd = sl_kind(d.y), un = sl_units<T>(d.y);
+    if (lane == 0)
+      bulk_load(ring + (warp * o.depth + i_slot) * o.slot_bytes, gblk + (size_t)d.x * 16 + chunk_offset<T>(kd, ic),
+                (uint32_t)chunk_bytes<T>(kd, ic, un), bars + warp * o.depth + i_slot);
+    if (++i_slot == o.depth) i_slot = 0;
+    if (++ic * chunk_units<T>(kd) >= un) {
+      ic = 0;
+      ij += nw;
+      if (ij >= ns) ij = warp;
+    }
+    --to_issue;
+    ++waiting;
+  };
+  for (int k = 0; k < o.depth && stream; ++k) issue();
+  // the slot just read is free again: fill it, go on to the next
+  auto next_slot = [&]() {
+    --waiting;
+    if (++w_slot == o.depth) {
+      w_slot = 0;
+      w_parity ^= 1;
+    }
+    __syncwarp();
+    issue();
+  };
+  // states
+  for (int r = tid; r < W; r += nt) {
+    T un = T(0), up = T(0);
+    if (!fresh) {
+      const int g = r < rpad ? (r < rows ? row0 + r : -1) : (r < rpad + H ? __ldg(hrow + r - rpad) : -1);
+      if (g >= 0) {
+        un = static_cast<const T*>(a.u_n)[g];
+        if (r < rpad) up = static_cast<const T*>(a.u_prev)[g];
+      }
+    }
+    U0[r] = un;
+    U1[r] = up;
+  }
+  // forcing terms: those of step k are in fs[k & 1], the signal of the step
+  // after next is on its way in freg
+  T fcoef = T(0), freg = T(0);
+  const T* fsig = static_cast<const T*>(a.sig);
+  if (tid < nf) {
+    fcoef = __ldg(static_cast<const T*>(a.frc_coef) + f0 + tid);
+    fsig += (size_t)ti0 * a.n_sig + __ldg(a.frc_sig + f0 + tid);
+    fs[tid] = round_mul(fcoef, __ldg(fsig));
+    fsig += a.n_sig;
+    if (n_steps > 1) freg = __ldg(fsig);
+  }
+  // one monitor per thread from the last thread down (the rest in a loop)
+  const int mt = nt - 1 - tid;
+  int mrow = 0;
+  double* hist = a.hist;
+  if (mt < nm) {
+    mrow = __ldg(a.mon_row + m0 + mt) - row0;
+    hist += (size_t)__ldg(a.mon_slot + m0 + mt) + (size_t)a.q * (size_t)ti0;
+  }
+  // exchange buffers of even and odd steps, this thread's first slots in them
+  T* const xu0 = static_cast<T*>(o.xch);
+  T* const xu1 = xu0 + o.x_stride;
+  T* const xv0 = static_cast<T*>(o.xchv);
+  T* const xv1 = xv0 + o.xv_stride;
+  constexpr int kPolls = NT <= 512 ? 4 : 2;
+  int hx[kPolls], vx[kPolls];
+#pragma unroll
+  for (int j = 0; j < kPolls; ++j) {
+    hx[j] = tid + j * nt < H ? __ldg(hrow + tid + j * nt) : 0;
+    vx[j] = INT && tid + j * nt < nv ? __ldg(vrow + tid + j * nt) : 0;
+  }
+  // step (from ti0) after which the next frame is due
+  int64_t frame = -1;
+  double* fcol = a.fld;
+  if (a.fld) {
+    const int64_t c = (ti0 + a.fld_every - 1) / a.fld_every;
+    frame = c * a.fld_every - ti0;
+    fcol += (size_t)a.n * (size_t)c;
+  }
+  __syncthreads();
+
+  uint32_t au = 0, bu = (uint32_t)(W * sizeof(T));      // byte offsets of u_n and of u_{n-1} / u_{n+1}
+  bool bad = false;
+  for (int64_t k = 0; k <= n_steps; ++k) {
+    const T* A = reinterpret_cast<const T*>(sm + au);
+    T* B = reinterpret_cast<T*>(sm + bu);
+    const uint32_t tag = o.tag0 + (uint32_t)(ti0 + k);
+    const bool odd = (ti0 + k) & 1;
+    // state ti0 + k - 1 (A): samples and, on frame steps, the frame
+    if (k > 0) {
+      if (mt < nm) {
+        *hist = (double)A[mrow];
+        hist += a.q;
+      }
+      for (int j = mt + nt; j < nm; j += nt)
+        a.hist[(size_t)__ldg(a.mon_slot + m0 + j) + (size_t)a.q * (size_t)(ti0 + k - 1)] =
+            (double)A[__ldg(a.mon_row + m0 + j) - row0];
+      if (k - 1 == frame) {
+        for (int j = warp; j < ns; j += nw) {            // each thread the rows it will overwrite
+          const int r = (sd[j].y >> kSlLocalShift) * kSlice + lane;
+          if (r < rows)
+            fcol[row0 + r] = a.fld_is_vel ? ((double)A[r] - (double)B[r]) / a.dt : (double)A[r];
+        }
+        frame += a.fld_every;
+        fcol += a.n;
+      }
+    }
+    if (k == n_steps) break;
+    if (tid < nf) {
+      fs[((k + 1) & 1) * nf + tid] = round_mul(fcoef, freg);
+      fsig += a.n_sig;
+      if (k + 2 < n_steps) freg = __ldg(fsig);
+    }
+    T* xu = odd ? xu1 : xu0;
+    T* xv = odd ? xv1 : xv0;
+    // rows
+    for (int j = warp; j < ns; j += nw) {
+      const int2 d = sd[j];
+      const int kind = sizeof(T) == 8 ? 0 : sl_kind(d.y), r = (d.y >> kSlLocalShift) * kSlice + lane;
+      const bool resident = d.y & kSlResident;
+      const T ui = A[r], up = B[r];
+      const uint32_t f = fl[r];
+      float ref[3];
+      if (sizeof(T) == 4) {
+        const int pos = (int)(f >> kOcPosShift) & 7;
+        ref[0] = (float)ui;
+        if (kind != 1) {
+          int q0 = r - pos, q1 = q0 + 1, q2 = q0 + 2;
+          if (kind == 0 && pos == (int)kOcCut) {
+            const ushort4 x = o.lref[row0 + r];
+            q0 = x.x, q1 = x.y, q2 = x.z;
+          }
+          __syncwarp();
+          ref[0] = (float)A[q0];
+          ref[1] = (float)A[q1];
+          ref[2] = (float)A[q2];
+        }
+      }
+      const unsigned char* blk = cache + d.x;
+      if (!resident) {
+        blk = ring + (warp * o.depth + w_slot) * o.slot_bytes;
+        bad |= !bar_wait(bars + warp * o.depth + w_slot, w_parity, o.err);
+      }
+      const T rc = reinterpret_cast<const T*>(blk)[lane];
+      blk += coef_bytes<T>();
+      T acc = T(0);
+      if (!(d.y & kSlChunks)) {
+        acc = row_sum(acc, blk, lane, kind, sl_width(d.y), sm, au, ref);
+      } else {
+        // FP64 counts entries (an odd last one is not paired), FP32 units
+        const int cu = chunk_units<T>(kind), full = sizeof(T) == 8 ? 2 * cu : cu, step = units_bytes<T>(kind, cu);
+        for (int left = sl_width(d.y);;) {
+          acc = row_sum(acc, blk, lane, kind, min(left, full), sm, au, ref);
+          left -= full;
+          if (left <= 0) break;
+          blk += step;
+          if (!resident) {
+            next_slot();
+            blk = ring + (warp * o.depth + w_slot) * o.slot_bytes;
+            bad |= !bar_wait(bars + warp * o.depth + w_slot, w_parity, o.err);
+          }
+        }
+      }
+      if (!resident) next_slot();
+      T ft = T(0);
+      if (f & kOcForced) ft = fs[(k & 1) * nf + lower_bound_sm(fr, nf, r)];
+      T rn, v;
+      row_update(acc, ui, up, rc, (f & kOcForced) != 0, ft, a.int_base_prev, rn, v);
+      if (INT && (f & kOcInterface)) {
+        const int li = (int)(f >> kOcIntShift);
+        vs[li] = v;
+        if (f & kOcExportV) xput(xv, (size_t)(t0 + li), v, tag);
+        if (!a.int_base_prev) B[r] = rn;
+      } else {
+        B[r] = rn;
+        if (f & kOcExport) xput(xu, (size_t)(row0 + r), rn, tag);
+      }
+    }
+    if (INT && ni) {
+      bad |= !receive(xv, vrow, nv, vx, tag, vs + ni, tid, nt, o.err);
+      __syncthreads();
+      for (int t = warp; t < ni; t += nw) {
+        T acc = T(0);
+        for (int e = zp[t] + lane; e < zp[t + 1]; e += 32) acc += zv[e] * vs[zc[e]];
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
+        if (lane == 0) {
+          const int r = zr[t];
+          const T rn = B[r] + acc;
+          B[r] = rn;
+          if (fl[r] & kOcExport) xput(xu, (size_t)(row0 + r), rn, tag);
+        }
+      }
+    }
+    if (k + 1 < n_steps) bad |= !receive(xu, hrow, H, hx, tag, B + rpad, tid, nt, o.err);
+    if (__syncthreads_or(bad)) {
+      for (; waiting > 0; --waiting) {                  // no copy may outlive the CTA
+        if (!bar_wait(bars + warp * o.depth + w_slot, w_parity, o.err)) break;
+        if (++w_slot == o.depth) {
+          w_slot = 0;
+          w_parity ^= 1;
+        }
+      }
+      return;
+    }
+    const uint32_t x = au;
+    au = bu;
+    bu = x;
+  }
+  // the two newest states back to global memory: u_n may still be read by a
+  // CTA that is loading, u_prev only by this one
+  for (int r = tid; r < rows; r += nt) {
+    static_cast<T*>(a.u_new)[row0 + r] = sm_at<T>(sm, au + r * (uint32_t)sizeof(T));
+    const_cast<T*>(static_cast<const T*>(a.u_prev))[row0 + r] = sm_at<T>(sm, bu + r * (uint32_t)sizeof(T));
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Building the partition's device data from the sliced-ELL operator.
+
+constexpr int kRankWords = 8;     // bitmap words per stored prefix count
+
+// One CTA per part: the columns its rows read outside the part become its
+// halo (ascending rows), and every slice gets its kind and its block.
+template <typename T>
+__global__ void __launch_bounds__(1024) oc_columns(OnchipBuild b) {
+  extern __shared__ __align__(16) unsigned char smb[];
+  uint32_t* bits = reinterpret_cast<uint32_t*>(smb);
+  __shared__ int cmin, cmax, total, bytes;
+  __shared__ int scan[1024];
+  constexpr bool F32 = sizeof(T) == 4;
+  const int p = blockIdx.x, tid = threadIdx.x, nt = blockDim.x, lane = tid & 31;
+  const int s0 = b.part_slice[p], s1 = b.part_slice[p + 1];
+  const int row0 = s0 * kSlice, row1 = min(b.n, s1 * kSlice), rpad = (s1 - s0) * kSlice;
+  const int e0 = b.slice_ptr[s0], e1 = b.slice_ptr[s1];
+  if (tid == 0) { cmin = 0x7fffffff; cmax = -1; bytes = 0; }
+  __syncthreads();
+  int lo = 0x7fffffff, hi = -1;
+  for (int e = e0 + tid; e < e1; e += nt) {
+    const int c = (int)(__ldg(b.col + e) & kColMask);
+    lo = min(lo, F32 ? max(c - 2, 0) : c);
+    hi = max(hi, F32 ? min(c + 2, b.n - 1) : c);
+  }
+  for (int i = row0 + tid; i < row1; i += nt) {
+    const int base = F32 ? (int)__ldg(b.base + i) : i;
+    lo = min(lo, base);
+    hi = max(hi, min(base + 2, b.n - 1));
+  }
+  atomicMin(&cmin, lo);
+  atomicMax(&cmax, hi);
+  __syncthreads();
+  const int c0 = cmin & ~31, nwords = (cmax - c0) / 32 + 1;
+  if (nwords > b.max_words) {
+    if (tid == 0) atomicExch(b.fail, 1);
+    return;
+  }
+  int* pre = reinterpret_cast<int*>(bits + ((b.max_words + kRankWords - 1) / kRankWords) * kRankWords);
+  const int ngrp = (nwords + kRankWords - 1) / kRankWords;
+  for (int k = tid; k < ngrp * kRankWords; k += nt) bits[k] = 0;
+  __syncthreads();
+  auto mark = [&](int c) {
+    if (c < row0 || c >= row1) atomicOr(bits + ((c - c0) >> 5), 1u << ((c - c0) & 31));
+  };
+  // padding of the sliced ELL: a direct zero on the row itself
+  auto is_pad = [&](uint32_t e, T v, int i) { return (e & kDirect) && v == T(0) && (int)(e & kColMask) == min(i, b.n - 1); };
+  // the first row of the node that entry e (of DOF slot s) belongs to, if the
+  // node has rows for all of kind's DOFs; else -1
+  auto node_of = [&](uint32_t e, int kind) -> int {
+    const int c = (int)(e & kColMask), nb = c - (int)((e >> kSlotShift) & kSlotMask);
+    if (nb < 0 || nb + kind > b.n || (int)__ldg(b.base + c) != nb || (int)__ldg(b.base + nb) != nb ||
+        (int)__ldg(b.base + nb + kind - 1) != nb)
+      return -1;
+    return nb;
+  };
+  for (int s = s0 + (tid >> 5); s < s1; s += nt >> 5) {
+    const int off = b.slice_ptr[s], w = (b.slice_ptr[s + 1] - off) >> 5, i = s * kSlice + lane;
+    if (w > kSlMaxWidth) atomicExch(b.fail, 1);
+    if (!F32) {
+      for (int k = 0; k < w; ++k) mark((int)(__ldg(b.col + off + 32 * k + lane) & kColMask));
+      if (lane == 0) b.slice_word[s] = w;
+      continue;
+    }
+    // kind: which of the forms every row of the slice has
+    const int base = i < b.n ? (int)__ldg(b.base + i) : 0, pos = i - base;
+    bool k1 = true, k2 = pos < 2 || i >= b.n, k3 = pos < 3 || i >= b.n;
+    for (int k = 0; k < w; ++k) {
+      const uint32_t e = __ldg(b.col + off + 32 * k + lane);
+      if (is_pad(e, __ldg(static_cast<const T*>(b.val) + off + 32 * k + lane), i)) continue;
+      const int slot = (int)((e >> kSlotShift) & kSlotMask);
+      if (e & kDirect) { k1 = k2 = k3 = false; continue; }
+      k1 = k1 && slot == pos;
+      k2 = k2 && slot < 2 && node_of(e, 2) >= 0;
+      k3 = k3 && slot < 3 && node_of(e, 3) >= 0;
+      if (slot > 2) atomicExch(b.fail, 1);
+    }
+    k2 = k2 && (i >= b.n || (base + 2 <= b.n && (int)__ldg(b.base + base + 1) == base));
+    k3 = k3 && (i >= b.n || (base + 3 <= b.n && (int)__ldg(b.base + base + 2) == base));
+    const int kind = __all_sync(0xffffffffu, k1) ? 1 : __all_sync(0xffffffffu, k2) ? 2 : __all_sync(0xffffffffu, k3) ? 3 : 0;
+    for (int k = 0; k < w; ++k) {
+      const uint32_t e = __ldg(b.col + off + 32 * k + lane);
+      mark((int)(e & kColMask));
+      if ((e & kDirect)) continue;
+      mark(base + (int)((e >> kSlotShift) & kSlotMask));
+      if (kind >= 2)
+        for (int q = 0, nb = node_of(e, kind); q < kind; ++q) mark(nb + q);
+    }
+    if (kind >= 2 && i < b.n)
+      for (int q = 0; q < kind; ++q) mark(base + q);
+    if (lane == 0) b.slice_word[s] = w | (kind << 11);
+  }
+  __syncthreads();
+  // prefix counts over groups of words
+  int mine = 0;
+  const int per = (ngrp + nt - 1) / nt;
+  for (int g = tid * per; g < min((tid + 1) * per, ngrp); ++g)
+    for (int k = 0; k < kRankWords; ++k) mine += __popc(bits[g * kRankWords + k]);
+  scan[tid] = mine;
+  __syncthreads();
+  for (int d = 1; d < nt; d <<= 1) {
+    const int x = tid >= d ? scan[tid - d] : 0;
+    __syncthreads();
+    scan[tid] += x;
+    __syncthreads();
+  }
+  int run = scan[tid] - mine;
+  for (int g = tid * per; g < min((tid + 1) * per, ngrp); ++g) {
+    pre[g] = run;
+    for (int k = 0; k < kRankWords; ++k) run += __popc(bits[g * kRankWords + k]);
+  }
+  if (tid == nt - 1) total = scan[tid];
+  __syncthreads();
+  const int H = total;
+  // one slot of the list is kept free per other part for symmetric reading
+  if (H + b.n_parts > b.halo_cap || rpad + H > b.max_window) {
+    if (tid == 0) atomicExch(b.fail, 1);
+    return;
+  }
+  auto local = [&](int c) -> int {
+    if (c >= row0 && c < row1) return c - row0;
+    const int w = (c - c0) >> 5, g = w / kRankWords;
+    int r = pre[g];
+    for (int k = g * kRankWords; k < w; ++k) r += __popc(bits[k]);
+    return rpad + r + __popc(bits[w] & ((1u << ((c - c0) & 31)) - 1u));
+  };
+  // halo rows, their owners and export marks
+  for (int w = tid; w < nwords; w += nt) {
+    uint32_t m = bits[w];
+    while (m) {
+      const int c = c0 + 32 * w + __ffs((int)m) - 1;
+      m &= m - 1;
+      b.halo_row[(size_t)p * b.halo_cap + local(c) - rpad] = c;
+      b.exported[c] = 1;
+      int a0 = 0, a1 = b.n_parts - 1;                  // the part that owns row c
+      while (a0 < a1) {
+        const int mid = (a0 + a1 + 1) >> 1;
+        if (b.part_slice[mid] * kSlice <= c) a0 = mid; else a1 = mid - 1;
+      }
+      b.adj[(size_t)p * b.n_parts + a0] = 1;
+    }
+  }
+  if (tid == 0) b.halo_cnt[p] = H;
+  for (int s = s0 + (tid >> 5); s < s1; s += nt >> 5) {
+    const int off = b.slice_ptr[s], w = (b.slice_ptr[s + 1] - off) >> 5, i = s * kSlice + lane;
+    const T* val = static_cast<const T*>(b.val) + off + lane;
+    const uint32_t* col = b.col + off + lane;
+    unsigned char* blk = static_cast<unsigned char*>(b.blocks) + (size_t)b.block_off[s] * 16;
+    reinterpret_cast<T*>(blk)[lane] = __ldg(static_cast<const T*>(b.rowc) + min(i, b.n - 1));
+    blk += coef_bytes<T>();
+    int kind = 0, pos = 0, units = 0;
+    if (F32) {
+      kind = b.slice_word[s] >> 11;
+      const int base = i < b.n ? (int)__ldg(b.base + i) : i;
+      pos = i - base;
+      // a node block cut by the part's edge keeps the row's indices in lref;
+      // units must lie together in the window
+      unsigned used = kind >= 2 && i < b.n ? (1u << kind) - 1u : 0u;
+      bool together = true;
+      int prev = -1;
+      for (int k = 0; k < w; ++k) {
+        const uint32_t e = __ldg(col + 32 * k);
+        if (e & kDirect) continue;
+        used |= 1u << ((e >> kSlotShift) & kSlotMask);
+        if (kind >= 2) {
+          const int nb = node_of(e, kind);
+          together = together && local(nb + kind - 1) == local(nb) + kind - 1;
+          if (nb != prev) ++units;
+          prev = nb;
+        }
+      }
+      const int top = used ? 31 - __clz((int)used) : 0;
+      const bool cut = used && (base < row0 || base + top >= row1 || pos >= (int)kOcCut);
+      if (i < b.n) {
+        uint16_t x[3];
+        for (int q = 0; q < 3; ++q) x[q] = (uint16_t)((used >> q) & 1u ? local(base + q) : i - row0);
+        b.lref[i] = make_ushort4(x[0], x[1], x[2], 0);
+        b.pos[i] = (uint8_t)(cut ? kOcCut : used ? pos : 0);
+      }
+      if (kind && !__all_sync(0xffffffffu, !cut && together)) kind = 0;
+      for (int d = 16; d > 0; d >>= 1) units = max(units, __shfl_xor_sync(0xffffffffu, units, d));
+      if (kind >= 2 && block_bytes<T>(kind, units) > block_bound<T>(w)) kind = 0;
+    }
+    const int width = kind < 2 ? w : units, un = slice_units(kind, width), cu = chunk_units<T>(kind);
+    if (lane == 0) {
+      b.slice_word[s] = (F32 ? un : width) | (kind << 11);
+      atomicAdd(&bytes, block_bytes<T>(kind, un));
+      atomicMax(b.slot_bytes, chunk_bytes<T>(kind, 0, un));
+    }
+    const int own = (F32 ? 4 : 1) * (min(i, row1 - 1) - row0);       // window index of the row itself
+    if (kind < 2) {
+      for (int k = 0; k < 2 * un; ++k) {
+        uint32_t lc = (uint32_t)own | (F32 && kind == 0 ? 3u : 0u);
+        T v = T(0);
+        if (k < w) {
+          const uint32_t e = __ldg(col + 32 * k);
+          v = __ldg(val + 32 * k);
+          if (kind == 0) {
+            lc = (uint32_t)local((int)(e & kColMask));
+            if (F32) lc = lc << 2 | ((e & kDirect) ? 3u : ((e >> kSlotShift) & kSlotMask));
+          } else if (!(e & kDirect)) {
+            lc = (uint32_t)local((int)(e & kColMask)) << 2;
+          }
+        }
+        const int c = (k >> 1) / cu, q = (k >> 1) - c * cu, npc = min(cu, un - c * cu);
+        T* cv = reinterpret_cast<T*>(blk + c * units_bytes<T>(kind, cu));
+        cv[64 * q + 2 * lane + (k & 1)] = v;
+        reinterpret_cast<uint16_t*>(cv + npc * 64)[64 * q + 2 * lane + (k & 1)] = (uint16_t)lc;
+      }
+    } else if (F32) {
+      int k = 0;
+      for (int q = 0; q < un; ++q) {                   // next node of the row, zeros past its last
+        float v[3] = {0.f, 0.f, 0.f};
+        while (k < w && (__ldg(col + 32 * k) & kDirect)) ++k;
+        int nb = -1;
+        while (k < w) {
+          const uint32_t e = __ldg(col + 32 * k);
+          if (e & kDirect) { ++k; continue; }
+          const int x = node_of(e, kind);
+          if (nb < 0) nb = x;
+          if (x != nb) break;
+          v[(e >> kSlotShift) & kSlotMask] = (float)__ldg(val + 32 * k);
+          ++k;
+        }
+        // past the last node: the row's own node, so that nothing else enters
+        const uint32_t lc = nb >= 0 ? 4u * (uint32_t)local(nb) : i < b.n ? 4u * (uint32_t)(i - pos - row0) : 0u;
+        const int c = q / cu, x = q - c * cu, nc = min(cu, un - c * cu);
+        float* cv = reinterpret_cast<float*>(blk + c * units_bytes<T>(kind, cu));
+        if (kind == 2) reinterpret_cast<float2*>(cv)[32 * x + lane] = make_float2(v[0], v[1]);
+        else
+          for (int l = 0; l < 3; ++l) cv[96 * x + 32 * l + lane] = v[l];
+        uint16_t* ci = reinterpret_cast<uint16_t*>(cv + nc * kind * 32);
+        ci[64 * (x >> 1) + 2 * lane + (x & 1)] = (uint16_t)lc;
+        if ((nc & 1) && x == nc - 1) ci[64 * (x >> 1) + 2 * lane + 1] = (uint16_t)lc;
+      }
+    }
+  }
+  __syncthreads();
+  if (tid == 0) b.op_bytes[p] = bytes;
+}
+
+// Reading made symmetric: when p reads from q and q not from p, q gets the
+// first row of p as one more halo row.
+__global__ void oc_symmetric(OnchipBuild b) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= b.n_parts * b.n_parts || *b.fail) return;
+  const int p = g / b.n_parts, q = g % b.n_parts;
+  if (!b.adj[(size_t)p * b.n_parts + q] || b.adj[(size_t)q * b.n_parts + p]) return;
+  const int k = atomicAdd(b.halo_cnt + q, 1);
+  if (k >= b.halo_cap) { atomicExch(b.fail, 1); return; }
+  const int c = b.part_slice[p] * kSlice;
+  b.halo_row[(size_t)q * b.halo_cap + k] = c;
+  b.exported[c] = 1;
+}
+
+// Row flags, and each part's slices in the order of their work: slices with
+// interface rows, then slices that others read from, then the rest, the wide
+// ones of each class first. Warps take them in turn, so this also evens out
+// the warps' work (in the order of the rows a warp's turns fall on the same
+// place of every mesh column: all solid or all fluid; C1 in FP32 then took
+// 14.0 us per step).
+__global__ void __launch_bounds__(256) oc_order(OnchipBuild b) {
+  extern __shared__ int pri[];
+  if (*b.fail) return;
+  const int p = blockIdx.x, s0 = b.part_slice[p], ns = b.part_slice[p + 1] - s0;
+  const int row0 = s0 * kSlice;
+  const int t0 = lower_bound_i32(b.int_row, b.n_int, row0);
+  for (int j = threadIdx.x; j < ns; j += blockDim.x) pri[j] = 2;
+  __syncthreads();
+  for (int r = threadIdx.x; r < ns * kSlice && row0 + r < b.n; r += blockDim.x) {
+    const int i = row0 + r;
+    uint32_t f = (b.exported[i] ? kOcExport : 0u) | (b.pos ? (uint32_t)b.pos[i] << kOcPosShift : 0u);
+    if (b.n_int) {
+      const int t = lower_bound_i32(b.int_row, b.n_int, i);
+      if (t < b.n_int && b.int_row[t] == i) {
+        if (t - t0 > (int)kOcMaxInt) atomicExch(b.fail, 1);
+        f |= kOcInterface | (b.v_exported[t] ? kOcExportV : 0u) | ((uint32_t)(t - t0) << kOcIntShift);
+      }
+    }
+    b.flags[i] = (uint16_t)f;
+    if (f & kOcInterface) atomicMin(pri + r / kSlice, 0);
+    else if (f & kOcExport) atomicMin(pri + r / kSlice, 1);
+  }
+  __syncthreads();
+  for (int j = threadIdx.x; j < ns; j += blockDim.x) pri[j] = pri[j] * 4096 + 4095 - (b.slice_ptr[s0 + j + 1] - b.slice_ptr[s0 + j]) / kSlice;
+  __syncthreads();
+  for (int j = threadIdx.x; j < ns; j += blockDim.x) {
+    int rank = 0;
+    for (int i = 0; i < ns; ++i) rank += pri[i] < pri[j] || (pri[i] == pri[j] && i < j);
+    b.order[s0 + rank] = (uint16_t)j;
+  }
+}
+
+template <typename T>
+cudaError_t build_t(const OnchipBuild& b, cudaStream_t st) {
+  const size_t words = (size_t)((b.max_words + kRankWords - 1) / kRankWords) * kRankWords;
+  const size_t smem = words * 4 + words / kRankWords * 4;
+  cudaError_t e = cudaFuncSetAttribute(oc_columns<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  oc_columns<T><<<b.n_parts, 1024, smem, st>>>(b);
+  const int pairs = b.n_parts * b.n_parts;
+  oc_symmetric<<<(pairs + 255) / 256, 256, 0, st>>>(b);
+  oc_order<<<b.n_parts, 256, (size_t)b.max_part_slices * sizeof(int), st>>>(b);
+  return cudaGetLastError();
+}
+
+template <typename T, bool INT, int NT>
+cudaError_t launch_t(const OnchipArgs& o, const StepArgs& a, int64_t ti0, int64_t n_steps, int fresh,
+                     cudaStream_t st) {
+  auto* kern = march_onchip<T, INT, NT>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, o.smem);
+  if (e != cudaSuccess) return e;
+  OnchipArgs oo = o;
+  StepArgs aa = a;
+  void* args[] = {&oo, &aa, &ti0, &n_steps, &fresh};
+  return cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kern), dim3(o.n_parts), dim3(o.threads), args,
+                                     (size_t)o.smem, st);
+}
+
+}  // namespace
+
+int onchip_block_bound(int precision, int width) {
+  return precision == 0 ? block_bound<double>(width) : block_bound<float>(width);
+}
+
+cudaError_t launch_onchip_build(const OnchipBuild& b, int precision, cudaStream_t st) {
+  return precision == 0 ? build_t<double>(b, st) : build_t<float>(b, st);
+}
+
+cudaError_t launch_onchip(const OnchipArgs& o, const StepArgs& a, int precision, int64_t ti0, int64_t n_steps,
+                          int fresh, cudaStream_t st) {
+  // parts of at most 16 warps take the form with 128 registers per thread:
+  // more of a row's loads in flight
+  auto go = [&](auto zero, auto interface) {
+    using T = decltype(zero);
+    constexpr bool kInt = decltype(interface)::value;
+    return o.threads <= 512 ? launch_t<T, kInt, 512>(o, a, ti0, n_steps, fresh, st)
+                            : launch_t<T, kInt, 1024>(o, a, ti0, n_steps, fresh, st);
+  };
+  if (precision == 0) return a.n_int ? go(0.0, std::true_type()) : go(0.0, std::false_type());
+  return a.n_int ? go(0.f, std::true_type()) : go(0.f, std::false_type());
+}
+
+}  // namespace bfe

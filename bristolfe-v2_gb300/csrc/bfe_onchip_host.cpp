@@ -1,0 +1,297 @@
+// Host side of the one-source march that stays on the chip (bfe_onchip.cu):
+// cutting a plan's rows into one part per SM, the device data of the parts,
+// and what a run needs of shared memory and threads.
+#include "bfe_host.h"
+
+using namespace bfe_host;
+
+namespace {
+
+// Shared memory a CTA may use, less a margin for the kernel's static part.
+constexpr int64_t kSmemLimit = 232448 - 256;
+// Slices per part below which a part is not split further: one warp of rows
+// for each of an SM's four schedulers.
+constexpr int64_t kMinSlices = 4;
+// Largest operator, as blocks: three quarters of the 129 MB L2. Above it the
+// streamed chunks come from HBM as the step kernels' operator does: FP64
+// bricks of 202,878 DOF (163 MB) took 39 us per step against 35.5 with one
+// launch per step, coupled 961,641 DOF in FP64 (101 MB) 27.6 against 27.7,
+// while 492,579 DOF (52 MB) took 14.2 against 19.3.
+constexpr int64_t kMaxOperator = (int64_t)96 << 20;
+
+inline int64_t align2(int64_t x) { return (x + 1) & ~(int64_t)1; }
+
+// Lists of the interface correction: which interface values each part reads
+// from others (made symmetric), which are read, local columns of Z.
+struct InterfaceLists {
+  std::vector<int32_t> ptr, list;
+  std::vector<uint16_t> z_lcol;
+  std::vector<uint8_t> exported;
+  std::vector<int32_t> first;        // first interface number of each part (n_parts + 1)
+};
+
+bool interface_lists(const bfe_plan* pl, const std::vector<int32_t>& part, InterfaceLists& L) {
+  const int P = (int)part.size() - 1;
+  const int32_t ni = pl->n_int;
+  L.first.resize(P + 1);
+  for (int p = 0; p <= P; ++p)
+    L.first[p] = (int32_t)(std::lower_bound(pl->h_int_row.begin(), pl->h_int_row.end(), part[p] * bfe::kSlice) -
+                           pl->h_int_row.begin());
+  std::vector<int32_t> owner(ni);
+  for (int p = 0; p < P; ++p)
+    for (int32_t t = L.first[p]; t < L.first[p + 1]; ++t) owner[t] = p;
+  std::vector<std::vector<int32_t>> need(P);
+  std::vector<char> adj((size_t)P * P, 0);
+  for (int p = 0; p < P; ++p) {
+    for (int32_t t = L.first[p]; t < L.first[p + 1]; ++t)
+      for (int32_t e = pl->h_z_ptr[t]; e < pl->h_z_ptr[t + 1]; ++e) {
+        const int32_t c = pl->h_z_col[e];
+        if (owner[c] == p) continue;
+        need[p].push_back(c);
+        adj[(size_t)p * P + owner[c]] = 1;
+      }
+    std::sort(need[p].begin(), need[p].end());
+    need[p].erase(std::unique(need[p].begin(), need[p].end()), need[p].end());
+  }
+  std::vector<size_t> real(P);
+  for (int p = 0; p < P; ++p) real[p] = need[p].size();
+  for (int p = 0; p < P; ++p)
+    for (int q = 0; q < P; ++q)
+      if (adj[(size_t)p * P + q] && !adj[(size_t)q * P + p]) need[q].push_back(L.first[p]);
+  L.exported.assign(ni, 0);
+  L.ptr.assign(1, 0);
+  L.z_lcol.assign(pl->h_z_col.size(), 0);
+  for (int p = 0; p < P; ++p) {
+    for (int32_t c : need[p]) L.exported[c] = 1;
+    L.list.insert(L.list.end(), need[p].begin(), need[p].end());
+    L.ptr.push_back((int32_t)L.list.size());
+    const int32_t own = L.first[p + 1] - L.first[p];
+    if (own + (int64_t)need[p].size() > 65535) return false;
+    const auto b = need[p].begin(), r = b + real[p];
+    for (int32_t t = L.first[p]; t < L.first[p + 1]; ++t)
+      for (int32_t e = pl->h_z_ptr[t]; e < pl->h_z_ptr[t + 1]; ++e) {
+        const int32_t c = pl->h_z_col[e];
+        L.z_lcol[e] = (uint16_t)(owner[c] == p ? c - L.first[p] : own + (int32_t)(std::lower_bound(b, r, c) - b));
+      }
+  }
+  return true;
+}
+
+}  // namespace
+
+namespace bfe_host {
+
+int onchip_prepare(bfe_plan* pl, cudaStream_t st) {
+  Onchip& oc = *pl->onchip;
+  if (oc.state) return BFE_OK;
+  oc.state = -1;
+  const int64_t n = pl->n, S = pl->n_slices;
+  const int prec = pl->prec;
+  const int64_t es = (int64_t)elem_size(prec);
+  int coop = 0;
+  CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, pl->device));
+  const int64_t P = std::min<int64_t>(bfe::sm_count(), (S + kMinSlices - 1) / kMinSlices);
+  // 16-bit window indices; FP32 entries use two bits to name a reference value
+  const int64_t max_window = std::min<int64_t>(kSmemLimit / (2 * es), es == 8 ? 65535 : 16383);
+  if (!coop || P < 1 || n > P * max_window) return BFE_OK;
+  // contiguous parts of even cost: a slice costs its width (one load of
+  // operator and state per entry) and a fixed part for the row's update
+  const std::vector<int32_t>& sp = pl->h_slice_ptr;
+  auto cost = [&](int64_t s) { return (double)((sp[s + 1] - sp[s]) / bfe::kSlice) + 4.0; };
+  double total = 0;
+  for (int64_t s = 0; s < S; ++s) total += cost(s);
+  oc.part_slice.assign(1, 0);
+  {
+    double run = 0;
+    int64_t s = 0;
+    for (int64_t p = 0; p < P; ++p) {
+      const double target = total * (double)(p + 1) / (double)P;
+      const int64_t must = S - (P - 1 - p);          // leave a slice for every later part
+      run += cost(s++);
+      while (s < must && run + 0.5 * cost(s) <= target) run += cost(s++);
+      if (p == P - 1) {
+        s = S;
+      } else if (prec == BFE_PREC_SINGLE) {
+        // FP32 rows of a node that an edge cuts take the slow form: move the
+        // edge to a node's first row where one is near (3D: every 96 rows)
+        for (int64_t d : {0, 1, -1, 2, -2}) {
+          const int64_t x = s + d;
+          if (x <= oc.part_slice.back() || x > must || (int64_t)pl->h_base[x * bfe::kSlice] != x * bfe::kSlice) continue;
+          for (; s < x; ++s) run += cost(s);
+          for (; s > x; --s) run -= cost(s - 1);
+          break;
+        }
+      }
+      oc.part_slice.push_back((int32_t)s);
+    }
+  }
+  std::vector<int32_t> boff(S + 1, 0);
+  int64_t max_slices = 0, off = 0;
+  for (int64_t p = 0; p < P; ++p)
+    max_slices = std::max<int64_t>(max_slices, oc.part_slice[p + 1] - oc.part_slice[p]);
+  for (int64_t s = 0; s < S; ++s) {
+    boff[s] = (int32_t)(off / 16);
+    off += bfe::onchip_block_bound(prec, (sp[s + 1] - sp[s]) / bfe::kSlice);
+    if (off / 16 > INT32_MAX) return BFE_OK;
+  }
+  if (prec == BFE_PREC_DOUBLE && off > kMaxOperator) return BFE_OK;     // exact for FP64: do not build
+  if (max_slices * bfe::kSlice > max_window) return BFE_OK;
+  InterfaceLists L;
+  if (pl->n_int && !interface_lists(pl, oc.part_slice, L)) return BFE_OK;
+
+  bfe::OnchipBuild b{};
+  b.n = (int32_t)n;
+  b.n_parts = (int32_t)P;
+  b.max_part_slices = (int32_t)max_slices;
+  b.max_words = (int32_t)std::min<int64_t>((n + 31) / 32 + 1, 50000);
+  b.max_window = (int32_t)max_window;
+  b.halo_cap = (int32_t)std::min<int64_t>(max_window, n + P);
+  b.n_int = pl->n_int;
+  DevBuf<uint8_t> scratch, vexp;
+  DevBuf<uint32_t> base;
+  DevBuf<int> misfit;
+  CUDA_TRY(oc.d_part.upload(oc.part_slice));
+  CUDA_TRY(oc.d_off.upload(boff));
+  CUDA_TRY(oc.d_bytes.alloc(P));
+  CUDA_TRY(oc.d_word.alloc(S));
+  CUDA_TRY(oc.d_cnt.alloc(P));
+  CUDA_TRY(oc.d_halo.alloc((size_t)P * b.halo_cap));
+  CUDA_TRY(oc.flags.alloc(n));
+  CUDA_TRY(oc.order.alloc(S));
+  CUDA_TRY(oc.blocks.alloc(off));
+  if (prec == BFE_PREC_SINGLE) {
+    CUDA_TRY(oc.lref.alloc(n));
+    CUDA_TRY(base.upload(pl->h_base));
+  }
+  CUDA_TRY(scratch.alloc((size_t)n * 2 + (size_t)P * P));
+  CUDA_TRY(cudaMemsetAsync(scratch.p, 0, (size_t)n * 2 + (size_t)P * P, st));
+  CUDA_TRY(misfit.alloc(2));
+  CUDA_TRY(cudaMemsetAsync(misfit.p, 0, 2 * sizeof(int), st));
+  if (pl->n_int) {
+    CUDA_TRY(vexp.upload(L.exported));
+    CUDA_TRY(oc.d_vptr.upload(L.ptr));
+    CUDA_TRY(oc.d_vhalo.upload(L.list));
+    CUDA_TRY(oc.z_lcol.upload(L.z_lcol));
+    CUDA_TRY(oc.xchv.alloc((size_t)pl->n_int * 4 * es));
+    CUDA_TRY(cudaMemsetAsync(oc.xchv.p, 0, (size_t)pl->n_int * 4 * es, st));
+  }
+  CUDA_TRY(oc.xch.alloc((size_t)n * 4 * es));
+  CUDA_TRY(cudaMemsetAsync(oc.xch.p, 0, (size_t)n * 4 * es, st));
+  CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));     // the uploads, before st reads them
+  b.part_slice = oc.d_part.p;
+  b.slice_ptr = pl->slice_ptr.p;
+  b.block_off = oc.d_off.p;
+  b.col = pl->col.p;
+  b.val = pl->val.p;
+  b.rowc = pl->rowc.p;
+  b.base = base.p;
+  b.int_row = pl->int_row.p;
+  b.v_exported = vexp.p;
+  b.halo_cnt = oc.d_cnt.p;
+  b.halo_row = oc.d_halo.p;
+  b.exported = scratch.p;
+  if (prec == BFE_PREC_SINGLE) b.pos = scratch.p + n;
+  b.adj = scratch.p + 2 * n;
+  b.flags = oc.flags.p;
+  b.order = oc.order.p;
+  b.blocks = oc.blocks.p;
+  b.slice_word = oc.d_word.p;
+  b.op_bytes = oc.d_bytes.p;
+  b.lref = oc.lref.p;
+  b.fail = misfit.p;
+  b.slot_bytes = misfit.p + 1;
+  CUDA_TRY(bfe::launch_onchip_build(b, prec, st));
+  int flags[2] = {0, 0};
+  std::vector<int32_t> cnt(P), obytes(P);
+  CUDA_TRY(cudaMemcpyAsync(flags, misfit.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+  CUDA_TRY(cudaMemcpyAsync(cnt.data(), oc.d_cnt.p, P * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+  CUDA_TRY(cudaMemcpyAsync(obytes.data(), oc.d_bytes.p, P * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+  CUDA_TRY(cudaStreamSynchronize(st));
+  bool failed = flags[0] != 0;
+  int64_t max_halo = 0, op_total = 0;
+  for (int32_t x : obytes) op_total += x;
+  failed = failed || op_total > kMaxOperator;
+  oc.need.assign(P, 0);
+  for (int64_t p = 0; p < P && !failed; ++p) {
+    const int64_t ns = oc.part_slice[p + 1] - oc.part_slice[p], rp = ns * bfe::kSlice;
+    const int64_t W = (rp + cnt[p] + 5) & ~(int64_t)3;
+    int64_t need = 2 * W * es + ns * 8 + rp * 2 + 32;
+    if (pl->n_int) {
+      const int64_t own = L.first[p + 1] - L.first[p];
+      const int64_t nz = pl->h_z_ptr[L.first[p + 1]] - pl->h_z_ptr[L.first[p]];
+      need += (align2(own + L.ptr[p + 1] - L.ptr[p]) + align2(nz)) * es + (own + 1) * 4 + (align2(nz) + align2(own)) * 2;
+    }
+    oc.need[p] = need;
+    max_halo = std::max<int64_t>(max_halo, cnt[p]);
+    if (need > kSmemLimit || rp + cnt[p] > max_window) failed = true;
+  }
+  if (failed) {
+    pl->onchip.reset(new Onchip());
+    pl->onchip->state = -1;
+    return BFE_OK;
+  }
+  oc.op_bytes = obytes;
+  bfe::OnchipArgs& o = oc.args;
+  o.n_parts = (int32_t)P;
+  // a warp per slice where that is enough, else as many warps as give each the
+  // same number of slices; and enough threads to poll the halo together
+  const int64_t turns = (max_slices + 31) / 32, warps = (max_slices + turns - 1) / turns;
+  const int64_t poll = turns == 1 ? std::min<int64_t>(max_slices <= 16 ? 512 : 1024, (max_halo / 2 + 31) / 32 * 32) : 0;
+  o.threads = (int32_t)std::max<int64_t>({128, warps * 32, poll});
+  o.slot_bytes = flags[1];
+  o.part_slice = oc.d_part.p;
+  o.halo_cnt = oc.d_cnt.p;
+  o.halo_row = oc.d_halo.p;
+  o.halo_cap = b.halo_cap;
+  o.flags = oc.flags.p;
+  o.order = oc.order.p;
+  o.blocks = oc.blocks.p;
+  o.block_off = oc.d_off.p;
+  o.slice_word = oc.d_word.p;
+  o.op_bytes = oc.d_bytes.p;
+  o.lref = oc.lref.p;
+  o.vhalo_ptr = oc.d_vptr.p;
+  o.vhalo = oc.d_vhalo.p;
+  o.z_lcol = oc.z_lcol.p;
+  o.xch = oc.xch.p;
+  o.x_stride = 2 * n;
+  o.xchv = oc.xchv.p;
+  o.xv_stride = 2 * (int64_t)pl->n_int;
+  oc.next_tag = 1;
+  oc.state = 1;
+  return BFE_OK;
+}
+
+bool onchip_fit(bfe_plan* pl, const std::vector<ForceEntry>& frc, bfe::OnchipArgs& o) {
+  const Onchip& oc = *pl->onchip;
+  o = oc.args;
+  const int P = o.n_parts;
+  std::vector<int32_t> rows(frc.size());
+  for (size_t k = 0; k < frc.size(); ++k) rows[k] = frc[k].row;
+  std::sort(rows.begin(), rows.end());
+  if (std::adjacent_find(rows.begin(), rows.end()) != rows.end()) return false;
+  // slots per warp for streamed chunks: up to four as long as they take no
+  // more than half of the memory the operator has
+  const int64_t warps = o.threads / 32;
+  int64_t room = kSmemLimit;
+  std::vector<int64_t> need(P);
+  bool stream = false;
+  for (int p = 0; p < P; ++p) {
+    const int64_t nf =
+        std::lower_bound(rows.begin(), rows.end(), oc.part_slice[p + 1] * bfe::kSlice) -
+        std::lower_bound(rows.begin(), rows.end(), oc.part_slice[p] * bfe::kSlice);
+    if (nf > o.threads) return false;
+    need[p] = oc.need[p] + 2 * nf * (int64_t)elem_size(pl->prec) + 16 + nf * 4 + (warps * 4 + 1) * 8 + 16;
+    room = std::min(room, kSmemLimit - need[p]);
+    stream = stream || need[p] + oc.op_bytes[p] > kSmemLimit;
+  }
+  const int64_t ring = warps * o.slot_bytes;
+  if (room < (stream ? ring : 0)) return false;
+  o.depth = (int32_t)std::max<int64_t>(1, std::min<int64_t>(4, room / 2 / std::max<int64_t>(ring, 1)));
+  int64_t smem = 0;
+  for (int p = 0; p < P; ++p) smem = std::max(smem, std::min<int64_t>(kSmemLimit, need[p] + oc.op_bytes[p]));
+  o.smem = (int32_t)(smem & ~(int64_t)15);
+  return true;
+}
+
+}  // namespace bfe_host

@@ -781,6 +781,7 @@ int create_plan(Csr K, Csr C, Csr M, double dt, int32_t solver_mode, int32_t pre
 
   // upload
   CUDA_TRY(pl->slice_ptr.upload(sptr));
+  pl->h_slice_ptr = sptr;
   CUDA_TRY(pl->col.upload(hcol));
   if ((rc = upload_bytes(pl->val, hval))) return rc;
   std::vector<unsigned char> hrc;
@@ -795,6 +796,8 @@ int create_plan(Csr K, Csr C, Csr M, double dt, int32_t solver_mode, int32_t pre
     CUDA_TRY(pl->int_row.upload(irows));
     CUDA_TRY(pl->z_ptr.upload(zp));
     CUDA_TRY(pl->z_col.upload(zc));
+    pl->h_z_ptr = zp;
+    pl->h_z_col = zc;
     if ((rc = upload_bytes(pl->z_val, zv))) return rc;
   }
   CUDA_TRY(cudaStreamCreateWithFlags(&pl->stream, cudaStreamNonBlocking));

@@ -153,6 +153,92 @@ int prepare_run(bfe_plan* pl, std::vector<ForceEntry>& frc, const std::vector<in
   return BFE_OK;
 }
 
+namespace {
+
+// Steps below which a run is not worth the partition's setup, and steps of
+// one launch (bounds how long one kernel runs).
+constexpr int64_t kOnchipMinSteps = 96, kOnchipLaunchSteps = 8192;
+// Device memory for raw frames that an element field is reduced from.
+constexpr int64_t kRawFrameBytes = (int64_t)1 << 31;
+
+// The whole march in kernels that stay on the chip; done says whether it ran.
+// On return U[1] holds the newest state. Any reason not to run it leaves the
+// march to the step kernels.
+int march_on_chip(bfe_plan* pl, RunSpec& rs, bfe::StepArgs a, unsigned char* const U[3], bool frames,
+                  cudaStream_t st, DevBuf<double>& d_raw, bool& done) {
+  done = false;
+  const int64_t steps = rs.n_t - rs.ti_start;
+  if (pl->timing || pl->time_limit_s > 0.0 || rs.v5 || steps < kOnchipMinSteps || rs.n_t >= ((int64_t)1 << 30) ||
+      getenv("BFE_NO_GRAPH"))
+    return BFE_OK;
+  const int64_t n_frames = frames ? (rs.n_t + rs.every_n - 1) / rs.every_n : 0;
+  const bool raw = frames && rs.field;
+  if (raw && pl->n * n_frames * (int64_t)sizeof(double) > kRawFrameBytes) return BFE_OK;
+  if (onchip_prepare(pl, st) || (raw && d_raw.alloc((size_t)pl->n * n_frames) != cudaSuccess)) {
+    // no memory for the partition or the raw frames: not an error of the run
+    if (pl->onchip->state == 0) pl->onchip->state = -1;
+    cudaGetLastError();
+    g_last_error.clear();
+    return BFE_OK;
+  }
+  bfe::OnchipArgs o;
+  if (pl->onchip->state != 1 || !onchip_fit(pl, rs.frc, o)) return BFE_OK;
+  if (raw) {
+    a.fld = d_raw.p;
+    a.fld_every = rs.every_n;
+    a.fld_is_vel = rs.field_is_vel;
+    a.dt = pl->dt;
+  }
+  // step numbers of this run: none that the exchange buffers still hold
+  Onchip& oc = *pl->onchip;
+  if ((uint64_t)oc.next_tag + (uint64_t)rs.n_t + 2 > 0xffffffffull) {
+    CUDA_TRY(cudaMemsetAsync(oc.xch.p, 0, oc.xch.n, st));
+    if (oc.xchv.n) CUDA_TRY(cudaMemsetAsync(oc.xchv.p, 0, oc.xchv.n, st));
+    oc.next_tag = 1;
+  }
+  o.tag0 = oc.next_tag;
+  oc.next_tag += (uint32_t)rs.n_t + 2;
+  o.err = pl->d_flag.p + 1;
+  int prev = 2, cur = 0, next = 1;
+  for (int64_t ti = rs.ti_start; ti < rs.n_t; ti += kOnchipLaunchSteps) {
+    const int64_t k = std::min(kOnchipLaunchSteps, rs.n_t - ti);
+    a.u_prev = U[prev];
+    a.u_n = U[cur];
+    a.u_new = U[next];
+    if (bfe::launch_onchip(o, a, pl->prec, ti, k, ti == rs.ti_start, st) != cudaSuccess) {
+      cudaGetLastError();          // not launchable here
+      CUDA_TRY(cudaStreamSynchronize(st));
+      return BFE_OK;
+    }
+    pl->last.step_launches++;
+    // newest in U[next], the one before it in U[prev]
+    const int t = cur;
+    cur = next;
+    next = t;
+  }
+  int gave_up = 0;
+  CUDA_TRY(cudaMemcpyAsync(&gave_up, o.err, sizeof(int), cudaMemcpyDeviceToHost, st));
+  CUDA_TRY(cudaStreamSynchronize(st));
+  if (gave_up) {                   // CTAs were not running together: march step by step
+    pl->onchip->state = -1;
+    return BFE_OK;
+  }
+  if (cur != 1)
+    CUDA_TRY(cudaMemcpyAsync(U[1], U[cur], (size_t)pl->n * elem_size(pl->prec), cudaMemcpyDeviceToDevice, st));
+  if (raw)
+    for (int64_t k = 0; k < n_frames; ++k) {
+      if (k * rs.every_n < rs.ti_start) continue;
+      CUDA_TRY(bfe::launch_field(*rs.field, d_raw.p + (size_t)pl->n * k, nullptr, BFE_PREC_DOUBLE, 0, pl->dt,
+                                 rs.d_el + rs.field->n_el * k, st));
+      pl->last.aux_launches++;
+    }
+  if (raw) CUDA_TRY(cudaStreamSynchronize(st));
+  done = true;
+  return BFE_OK;
+}
+
+}  // namespace
+
 int execute(bfe_plan* pl, RunSpec& rs, cudaStream_t st) {
   const int64_t n = pl->n, R = rs.R;
   const int prec = pl->prec;
@@ -165,7 +251,6 @@ int execute(bfe_plan* pl, RunSpec& rs, cudaStream_t st) {
   DevBuf<unsigned char> d_u;
   const size_t state_bytes = (size_t)n * R * es;
   CUDA_TRY(d_u.alloc(3 * state_bytes));
-  CUDA_TRY(cudaMemsetAsync(d_u.p, 0, 3 * state_bytes, st));
   unsigned char* U[3] = {d_u.p, d_u.p + state_bytes, d_u.p + 2 * state_bytes};
   int iprev = 0, icur = 1, inew = 2;
   bfe_stats& stt = pl->last;
@@ -208,6 +293,7 @@ int execute(bfe_plan* pl, RunSpec& rs, cudaStream_t st) {
   int variant = 0;
   const bfe::GroupArgs* grp = pl->have_groups ? &pl->groups : nullptr;
   if (R > 1) {
+    CUDA_TRY(cudaMemsetAsync(d_u.p, 0, 3 * state_bytes, st));
     int cand[8];
     const int max_bs = grp ? bfe::group_max_bs(*grp) : 0;
     const int nc = bfe::batched_candidates(prec, (int)R, pl->have_groups, max_bs, cand);
@@ -278,6 +364,20 @@ int execute(bfe_plan* pl, RunSpec& rs, cudaStream_t st) {
   if (frames && rs.fld_time)
     for (int64_t k = 0; k * rs.every_n < rs.n_t; ++k)
       if (k * rs.every_n >= rs.ti_start) (*rs.fld_time)[k] = rs.time[k * rs.every_n];
+  if (!pl->d_flag.p) CUDA_TRY(pl->d_flag.alloc(2));
+  CUDA_TRY(cudaMemsetAsync(pl->d_flag.p, 0, 2 * sizeof(int), st));
+  // One source whose state fits on the chip: all steps in one kernel
+  // (bfe_onchip.cu), unless launches are timed one by one, a time limit wants
+  // the host between chunks, or the run is too short to pay for the setup.
+  // Element fields are reduced afterwards from raw frames kept on the device.
+  bool on_chip = false;
+  if (R == 1) {
+    DevBuf<double> d_raw;
+    const int rc1 = march_on_chip(pl, rs, a, U, frames, st, d_raw, on_chip);
+    if (rc1) return rc1;
+    if (on_chip) iprev = 0, icur = 1, inew = 2;
+    else CUDA_TRY(cudaMemsetAsync(d_u.p, 0, 3 * state_bytes, st));
+  }
   bool capturing = false;
   // One time step: step kernel, interface correction, optional frame, v5 rows.
   auto one_step = [&](int64_t ti, bool rec) -> int {
@@ -331,14 +431,14 @@ int execute(bfe_plan* pl, RunSpec& rs, cudaStream_t st) {
     inew = t;
     return BFE_OK;
   };
-  int64_t ti = rs.ti_start;
+  int64_t ti = on_chip ? rs.n_t : rs.ti_start;
   // CUDA graph replay: the launches of kGraphSteps consecutive steps (a
   // multiple of the 3-buffer state rotation and of the 2-buffer v5 velocity
   // swap) are captured once, with the time index
   // read from a device counter that the last node advances, and replayed.
   // Not used with per-launch timing, v5 frames or the legacy stream.
   const int64_t kGraphSteps = 48;
-  const bool use_graph = !timing && !(rs.v5 && frames) && st != nullptr && st != cudaStreamLegacy &&
+  const bool use_graph = !on_chip && !timing && !(rs.v5 && frames) && st != nullptr && st != cudaStreamLegacy &&
                          (rs.n_t - rs.ti_start) >= 2 * kGraphSteps && getenv("BFE_NO_GRAPH") == nullptr;
   DevBuf<int64_t> d_ti;
   cudaGraph_t graph = nullptr;
@@ -394,8 +494,6 @@ int execute(bfe_plan* pl, RunSpec& rs, cudaStream_t st) {
   // non-finite values anywhere in the march stay in the state (every row's
   // update includes its own previous value), so one check of the newest
   // state finds them
-  if (!pl->d_flag.p) CUDA_TRY(pl->d_flag.alloc(1));
-  CUDA_TRY(cudaMemsetAsync(pl->d_flag.p, 0, sizeof(int), st));
   CUDA_TRY(bfe::launch_nonfinite_check(U[icur], n * R, prec, pl->d_flag.p, st));
   stt.aux_launches++;
   CUDA_TRY(cudaStreamSynchronize(st));
