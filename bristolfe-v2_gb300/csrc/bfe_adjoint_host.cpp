@@ -120,14 +120,13 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
   RunArrays rf;
   bfe::StepArgs af;
   if ((rc = prepare_run(pl, frc, hidx, R, n_t, n_sig, d_sig.p, d_hist.p, st, rf, af))) return rc;
-  const bool use_groups = pl->have_groups && (prec == BFE_PREC_SINGLE ? (R % 64 == 0 || R == 16 || R == 32)
-                                                                       : R % 16 == 0);
-  const bfe::GroupArgs* grp = use_groups ? &pl->groups : nullptr;
+  const int64_t Rp = af.R;           // right-hand sides of the states, padding included
+  const bfe::GroupArgs* grp = pl->have_groups ? &pl->groups : nullptr;
   // the variant the forward runs chose for this R, else the default candidate
   int variant = 0;
   if (R > 1) {
     int cand[8];
-    bfe::batched_candidates(prec, (int)R, use_groups, grp ? bfe::group_max_bs(*grp) : 0, cand);
+    bfe::batched_candidates(prec, (int)Rp, pl->have_groups, grp ? bfe::group_max_bs(*grp) : 0, cand);
     variant = cand[0];
     auto it = pl->variant_of_R.find(R);
     if (it != pl->variant_of_R.end()) variant = it->second;
@@ -142,7 +141,7 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
     }
     return BFE_OK;
   };
-  const size_t sb = (size_t)n * R * es;
+  const size_t sb = (size_t)n * Rp * es;
   // With ckpt_every = 0, every forward state stays on the device when the
   // steps + 2 states and the adjoint's c + 2 segment slots fit in 3/4 of the
   // free memory: state u_t sits in slot t - ti0 + 2 of d_all (slots 0 and 1
@@ -325,13 +324,13 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
   g.ke = d_ke.p;
   g.mh = d_mh.p;
   g.ch = d_ch.p;
-  g.R = (int)R;
+  g.R = (int)Rp;
   g.dt = dt;
   g.gs = d_gs.p;
   g.gr = d_gr.p;
   g.lam = d_lam.p;
   g.u = d_seg.p;
-  g.stride = n * R;
+  g.stride = n * Rp;
   g.n = n;
   g.pw = d_pw.p;
   g.pv = d_pv.p;

@@ -35,6 +35,7 @@ __device__ __forceinline__ T forcing_sum(const StepArgs& a, int i, int r) {
 }
 
 __device__ __forceinline__ void write_history(const StepArgs& a, int i, int r, double v) {
+  if (r >= a.R_out) return;
   for (int k = lower_bound_i32(a.mon_row, a.n_mon, i); k < a.n_mon && __ldg(a.mon_row + k) == i; ++k) {
     int slot = __ldg(a.mon_slot + k);
     a.hist[(size_t)slot + (size_t)a.q * ((size_t)step_index(a) + (size_t)a.n_t * r)] = v;

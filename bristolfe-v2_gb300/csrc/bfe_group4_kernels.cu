@@ -59,8 +59,11 @@ __device__ __forceinline__ void group4_nbr(const float* nb, const float* craw, i
     cv[2 % (BS * BS)] = make_float2(cr.z, cr.z);
     cv[3 % (BS * BS)] = make_float2(cr.w, cr.w);
   } else {
-    const float cr = __ldg(craw + e);
-    cv[0] = make_float2(cr, cr);
+#pragma unroll
+    for (int t = 0; t < BS * BS; ++t) {
+      const float cr = __ldg(craw + (size_t)e * (BS * BS) + t);
+      cv[t] = make_float2(cr, cr);
+    }
   }
 #pragma unroll
   for (int l = 0; l < BS; ++l) {
@@ -139,9 +142,11 @@ __device__ __forceinline__ void group4_fluid(const StepArgs& a, const GroupArgs&
   }
 }
 
-template <int BS, int LPN>
-__device__ __forceinline__ void group4_node(const StepArgs& a, const GroupArgs& gr, int gi, int node,
-                                            int l16) {
+// The node's right-hand sides c0, c0 + stride, ... (four each); UNROLL
+// neighbours in flight.
+template <int BS, int UNROLL>
+__device__ __forceinline__ void group4_node(const StepArgs& a, const GroupArgs& gr, int gi, int node, int c0,
+                                            int stride) {
   const int4 rec = __ldg(gr.rec[gi] + node);
   const int row0 = rec.x, p0 = rec.y, p1 = rec.y + rec.z;
   const int R = a.R;
@@ -149,7 +154,7 @@ __device__ __forceinline__ void group4_node(const StepArgs& a, const GroupArgs& 
   const float* un = static_cast<const float*>(a.u_n);
   const int32_t* nrow = gr.nrow[gi];
   const float* craw = gr.coef[gi];
-  for (int c = l16 * 4; c < R; c += 4 * LPN) {
+  for (int c = c0; c < R; c += stride) {
     float4 uo[BS], up[BS], acc[BS];
 #pragma unroll
     for (int k = 0; k < BS; ++k) {
@@ -157,7 +162,7 @@ __device__ __forceinline__ void group4_node(const StepArgs& a, const GroupArgs& 
       up[k] = ld_once(static_cast<const float*>(a.u_prev) + (size_t)(row0 + k) * rs + c);
       acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-#pragma unroll (BS == 1 ? 2 : 1)
+#pragma unroll UNROLL
     for (int e = p0; e < p1; ++e)
       group4_nbr<BS>(un + (size_t)__ldg(nrow + e) * rs + c, craw, e, rs, uo, acc);
 #pragma unroll
@@ -183,8 +188,28 @@ __global__ void __launch_bounds__(128, MINB) step_f32_group4(StepArgs a, GroupAr
   }
   const int node = (b - gr.blk_begin[gi]) * (128 / LPN) + threadIdx.x / LPN;
   if (node >= gr.n_nodes[gi]) return;
-  if (gr.bs[gi] == 1) group4_node<1, LPN>(a, gr, gi, node, threadIdx.x % LPN);
-  else group4_node<2, LPN>(a, gr, gi, node, threadIdx.x % LPN);
+  if (gr.bs[gi] == 1) group4_node<1, 2>(a, gr, gi, node, threadIdx.x % LPN * 4, 4 * LPN);
+  else group4_node<2, 1>(a, gr, gi, node, threadIdx.x % LPN * 4, 4 * LPN);
+}
+
+// The same for any R that is a multiple of 4 and node blocks of up to 3 DOFs:
+// gr.lpn lanes per node, any number up to 32, so no lane is idle but the few
+// that 128 / lpn leaves over. A ragged R used to take the slice kernel, whose
+// warps put 32 lanes on a row whatever R is.
+template <int MAXBS, int MINB, int UNROLL>
+__global__ void __launch_bounds__(128, MINB) step_f32_groupn(StepArgs a, GroupArgs gr) {
+  const int b = blockIdx.x;
+  int gi = 0;
+#pragma unroll
+  for (int k = 1; k < kMaxGroups; ++k)
+    if (k < gr.n_groups && b >= gr.blk_begin[k]) gi = k;
+  const int npc = 128 / gr.lpn, ln = threadIdx.x / gr.lpn;
+  const int node = (b - gr.blk_begin[gi]) * npc + ln;
+  if (ln >= npc || node >= gr.n_nodes[gi]) return;
+  const int c0 = (threadIdx.x - ln * gr.lpn) * 4, stride = 4 * gr.lpn;
+  if (gr.bs[gi] == 1) group4_node<1, UNROLL>(a, gr, gi, node, c0, stride);
+  else if (MAXBS == 2 || gr.bs[gi] == 2) group4_node<2, UNROLL>(a, gr, gi, node, c0, stride);
+  else group4_node<MAXBS, UNROLL>(a, gr, gi, node, c0, stride);
 }
 
 // The variants of the half-warp family for lanes-per-node LPN: 20 at 12 CTAs
@@ -207,6 +232,30 @@ cudaError_t launch_group4_variant(int lpn, const StepArgs& a, const GroupArgs& g
   if (lpn == 16) launch_group4<16>(a, gr, variant, st);
   else if (lpn == 8) launch_group4<8>(a, gr, variant, st);
   else launch_group4<4>(a, gr, variant, st);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_groupn_variant(int maxbs, const StepArgs& a, const GroupArgs& gr, int variant, cudaStream_t st) {
+  GroupArgs g = gr;
+  // lanes per node: 16 bytes of every row per lane, the passes over R evened out
+  const int quads = a.R / 4, passes = (quads + 15) / 16;
+  g.lpn = (quads + passes - 1) / passes;
+  const int npc = 128 / g.lpn;
+  int blocks = 0;
+  for (int k = 0; k < g.n_groups; ++k) {
+    g.blk_begin[k] = blocks;
+    blocks += (g.n_nodes[k] + npc - 1) / npc;
+  }
+  g.blk_begin[g.n_groups] = blocks;
+  if (maxbs <= 2) {
+    if (variant == 24) step_f32_groupn<2, 12, 1><<<blocks, 128, 0, st>>>(a, g);
+    else if (variant == 25) step_f32_groupn<2, 8, 2><<<blocks, 128, 0, st>>>(a, g);
+    else step_f32_groupn<2, 5, 4><<<blocks, 128, 0, st>>>(a, g);
+  } else {
+    if (variant == 24) step_f32_groupn<3, 8, 1><<<blocks, 128, 0, st>>>(a, g);
+    else if (variant == 25) step_f32_groupn<3, 6, 1><<<blocks, 128, 0, st>>>(a, g);
+    else step_f32_groupn<3, 4, 2><<<blocks, 128, 0, st>>>(a, g);
+  }
   return cudaGetLastError();
 }
 

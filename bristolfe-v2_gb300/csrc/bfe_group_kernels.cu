@@ -98,9 +98,9 @@ __global__ void __launch_bounds__(256, MINB) step_f32_group2(StepArgs a, GroupAr
 // u_new = sum over the node's blocks (its own included) of B_block u_n
 // + D u_{n-1} + forcing, summed in column order like the one-source kernel.
 // LPN lanes per node, VEC doubles (right-hand sides) per lane and pass.
-template <int BS, int LPN, int VEC>
+template <int BS, int VEC, int UNROLL>
 __device__ __forceinline__ void group64_node(const StepArgs& a, const GroupArgs& gr, int gi, int node,
-                                             int lane) {
+                                             int c0, int stride) {
   const int4 rec = __ldg(gr.rec[gi] + node);
   const int row0 = rec.x, p0 = rec.y, p1 = rec.y + rec.z;
   const int R = a.R;
@@ -108,12 +108,13 @@ __device__ __forceinline__ void group64_node(const StepArgs& a, const GroupArgs&
   const double* un = static_cast<const double*>(a.u_n);
   const int32_t* nrow = gr.nrow[gi];
   const double* cf = gr.coef64[gi];
-  for (int c = lane * VEC; c < R; c += LPN * VEC) {
+  for (int c = c0; c < R; c += stride) {
     double acc[BS][VEC];
 #pragma unroll
     for (int k = 0; k < BS; ++k)
 #pragma unroll
       for (int v = 0; v < VEC; ++v) acc[k][v] = 0.0;
+#pragma unroll UNROLL
     for (int e = p0; e < p1; ++e) {
       const double* nb = un + (size_t)__ldg(nrow + e) * rs + c;
       double g[BS][VEC];
@@ -172,25 +173,35 @@ __device__ __forceinline__ void group64_node(const StepArgs& a, const GroupArgs&
   }
 }
 
-template <int LPN, int VEC, int MINB, int MAXBS>
+template <int LPN, int VEC, int MINB, int MAXBS, int UNROLL = 1>
 __global__ void __launch_bounds__(128, MINB) step_f64_group(StepArgs a, GroupArgs gr) {
   const int b = blockIdx.x;
   int gi = 0;
 #pragma unroll
   for (int k = 1; k < kMaxGroups; ++k)
     if (k < gr.n_groups && b >= gr.blk_begin[k]) gi = k;
-  const int node = (b - gr.blk_begin[gi]) * (128 / LPN) + threadIdx.x / LPN;
-  if (node >= gr.n_nodes[gi]) return;
-  if (gr.bs[gi] == 1) group64_node<1, LPN, VEC>(a, gr, gi, node, threadIdx.x % LPN);
-  else if (MAXBS == 2 || gr.bs[gi] == 2) group64_node<(MAXBS >= 2 ? 2 : 1), LPN, VEC>(a, gr, gi, node, threadIdx.x % LPN);
-  else group64_node<MAXBS, LPN, VEC>(a, gr, gi, node, threadIdx.x % LPN);
+  // LPN lanes per node, or gr.lpn of them (LPN = 0: any R)
+  const int lpn = LPN ? LPN : gr.lpn, npc = 128 / lpn, ln = threadIdx.x / lpn;
+  const int node = (b - gr.blk_begin[gi]) * npc + ln;
+  if (ln >= npc || node >= gr.n_nodes[gi]) return;
+  const int c0 = (threadIdx.x - ln * lpn) * VEC, stride = lpn * VEC;
+  if (gr.bs[gi] == 1) group64_node<1, VEC, UNROLL>(a, gr, gi, node, c0, stride);
+  else if (MAXBS == 2 || gr.bs[gi] == 2) group64_node<(MAXBS >= 2 ? 2 : 1), VEC, UNROLL>(a, gr, gi, node, c0, stride);
+  else group64_node<MAXBS, VEC, UNROLL>(a, gr, gi, node, c0, stride);
 }
 
 // FP64 variants: 1 = 16 lanes x 4 right-hand sides (R a multiple of 64),
-// 2 = 16 x 2 (R a multiple of 32), 3 = 8 x 2 (R a multiple of 16).
+// 2 = 16 x 2 (R a multiple of 32), 3 = 8 x 2 (R a multiple of 16), 4 and 5 =
+// any even R, two right-hand sides per lane, one or two neighbours in flight
+// (us per step, slice kernel / variant 4: coupled 241,579 DOF R = 5 154.5 /
+// 35.1, R = 21 157.5 / 111.5; the FP64 pipe bounds both). Skipping the absent
+// entries of a block (one in seven) by a branch made variant 1 slower, 359 us
+// against 272 at R = 64.
 static cudaError_t launch_group64(const StepArgs& a, const GroupArgs& gr, int variant, cudaStream_t st) {
-  const int lpn = variant == 3 ? 8 : 16;
+  const int pairs = a.R / 2, passes = (pairs + 15) / 16;
+  const int lpn = variant >= 4 ? (pairs + passes - 1) / passes : variant == 3 ? 8 : 16;
   GroupArgs g = gr;
+  g.lpn = lpn;
   int blocks = 0;
   for (int k = 0; k < g.n_groups; ++k) {
     g.blk_begin[k] = blocks;
@@ -202,11 +213,15 @@ static cudaError_t launch_group64(const StepArgs& a, const GroupArgs& gr, int va
   if (maxbs <= 2) {
     if (variant == 1) step_f64_group<16, 4, 8, 2><<<blocks, 128, 0, st>>>(a, g);
     else if (variant == 2) step_f64_group<16, 2, 10, 2><<<blocks, 128, 0, st>>>(a, g);
-    else step_f64_group<8, 2, 10, 2><<<blocks, 128, 0, st>>>(a, g);
+    else if (variant == 3) step_f64_group<8, 2, 10, 2><<<blocks, 128, 0, st>>>(a, g);
+    else if (variant == 4) step_f64_group<0, 2, 8, 2><<<blocks, 128, 0, st>>>(a, g);
+    else step_f64_group<0, 2, 6, 2, 2><<<blocks, 128, 0, st>>>(a, g);
   } else {
     if (variant == 1) step_f64_group<16, 4, 6, 3><<<blocks, 128, 0, st>>>(a, g);
     else if (variant == 2) step_f64_group<16, 2, 8, 3><<<blocks, 128, 0, st>>>(a, g);
-    else step_f64_group<8, 2, 8, 3><<<blocks, 128, 0, st>>>(a, g);
+    else if (variant == 3) step_f64_group<8, 2, 8, 3><<<blocks, 128, 0, st>>>(a, g);
+    else if (variant == 4) step_f64_group<0, 2, 6, 3><<<blocks, 128, 0, st>>>(a, g);
+    else step_f64_group<0, 2, 4, 3, 2><<<blocks, 128, 0, st>>>(a, g);
   }
   return cudaGetLastError();
 }

@@ -32,7 +32,8 @@ constexpr int64_t kMaxDof = (int64_t)kColMask;
 // Device view of everything one time step needs (passed by value).
 struct StepArgs {
   int32_t n;            // rows (DOFs)
-  int32_t R;            // right-hand sides (state is [n][R], RHS-contiguous)
+  int32_t R;            // right-hand sides of the state ([n][R], RHS-contiguous)
+  int32_t R_out;        // of them those the run asked for (the rest are padding)
   int32_t n_slices;
   const int32_t* slice_ptr;   // entry offset of each slice (n_slices + 1)
   const uint32_t* col;        // packed entries, column-major inside a slice
@@ -110,6 +111,7 @@ struct GroupArgs {
   const float* coef[kMaxGroups];     // BS*BS per neighbour block, [own k][neighbour l]
   const float2* coef2[kMaxGroups];   // the coefficients as broadcast pairs {c, c}
   const int4* rec[kMaxGroups];       // per node {first row, first neighbour block, neighbour count, 0}
+  int32_t lpn;                       // lanes per node of the any-R kernels
   const double* coef64[kMaxGroups];  // FP64 plans: B per block (own block included), [own k][l]
 };
 
@@ -118,6 +120,12 @@ cudaError_t launch_step(const StepArgs& a, int precision, cudaStream_t s);      
 // Kernel variants a batched run of (precision, R) may use, the default
 // first; writes them to out (at most 8) and returns their number.
 int batched_candidates(int precision, int R, bool have_groups, int max_bs, int* out);
+// Right-hand sides the state of an R-source run is laid out with: the group
+// kernels take R in multiples of 4 (FP32) or 2 (FP64).
+inline int padded_sources(int precision, int64_t R, bool have_groups) {
+  const int64_t q = R < 2 || !have_groups ? 1 : precision == 0 ? 2 : 4;
+  return (int)((R + q - 1) / q * q);
+}
 // Largest node block size (DOFs per node) of a group operator.
 int group_max_bs(const GroupArgs& g);
 cudaError_t launch_step_batched(const StepArgs& a, const GroupArgs* gr, int precision, int max_slice_entries,
@@ -134,6 +142,7 @@ cudaError_t launch_nonfinite_check(const void* u, int64_t count, int precision, 
 cudaError_t launch_group2_variant(int maxbs, const StepArgs& a, const GroupArgs& gr, int variant, cudaStream_t s);
 cudaError_t launch_group4_variant(int lpn, const StepArgs& a, const GroupArgs& gr, int variant, cudaStream_t s);
 cudaError_t launch_group64_variant(const StepArgs& a, const GroupArgs& gr, int variant, cudaStream_t s);
+cudaError_t launch_groupn_variant(int maxbs, const StepArgs& a, const GroupArgs& gr, int variant, cudaStream_t s);
 cudaError_t launch_frame(const StepArgs& a, int precision, double* fld, int64_t frame,
                          int field_is_vel, double dt, cudaStream_t s);
 cudaError_t launch_cast_f64_to_f32(const double* in, float* out, int64_t n, cudaStream_t s);

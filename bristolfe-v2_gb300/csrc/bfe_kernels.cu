@@ -382,15 +382,18 @@ size_t batched_smem_bytes(int precision, int max_slice_entries) {
 }
 
 // Kernel variants of batched runs (the numbers are the names BFE_VARIANT and
-// the benchmark use):
+// the benchmark use); R is the padded number of right-hand sides:
 //   0        slice-staged row kernel step_batched: every plan and R
-//   FP64 plans with the group form, R a multiple of 16:
+//   FP64 plans with the group form:
 //   1, 2, 3  FP64 group kernel with 4, 2 or 1 right-hand side pairs per lane
 //            (R % 64, R % 32, R % 16)
+//   4, 5     the same for any R, one or two pairs of neighbours in flight
 //   FP32 plans with the group form:
 //   20, 22   half-warp float4 kernel step_f32_group4 (raw coefficient
 //            loads) at 12 or 10 CTAs per SM: node blocks of at most 2 DOFs,
 //            R a multiple of 64 or R = 16, 32
+//   24 - 26  the float4 form for any R and block size, one, two or four
+//            neighbours in flight
 //   9 - 14   packed warp-per-node kernel step_f32_group2 (unroll 1, 2, 4;
 //            occupancy hints 4, 6, 8 CTAs): 3-DOF node blocks (3D), R a
 //            multiple of 64
@@ -403,17 +406,24 @@ int batched_candidates(int precision, int R, bool have_groups, int max_bs, int* 
       if (R % 64 == 0) out[k++] = 1;
       if (R % 32 == 0) out[k++] = 2;
       out[k++] = 3;
+      out[k++] = 5;
+    } else if (have_groups) {
+      out[k++] = 4;
+      out[k++] = 5;
     }
     out[k++] = 0;
     return k;
   }
   if (have_groups && max_bs <= 2 && (R % 64 == 0 || R == 16 || R == 32)) {
-    out[k++] = 20;
-    out[k++] = 22;
+    for (int v : {20, 22}) out[k++] = v;
     return k;
   }
   if (have_groups && R % 64 == 0) {
-    for (int v : {13, 9, 10, 11, 12, 14}) out[k++] = v;
+    for (int v : {24, 25, 13, 9}) out[k++] = v;
+    return k;
+  }
+  if (have_groups) {
+    for (int v : {24, 25, 26}) out[k++] = v;
     return k;
   }
   out[k++] = 0;
@@ -431,14 +441,16 @@ cudaError_t launch_step_batched(const StepArgs& a, const GroupArgs* gr, int prec
   const int threads = 256;
   const size_t smem = batched_smem_bytes(precision, max_slice_entries);
   if (precision == 0) {
-    if (variant >= 1 && variant <= 3 && gr) return launch_group64_variant(a, *gr, variant, st);
+    if (variant >= 1 && variant <= 5 && gr) return launch_group64_variant(a, *gr, variant, st);
     step_batched<double, 1><<<a.n_slices, threads, smem, st>>>(a);
     return cudaGetLastError();
   }
   const int maxbs = gr ? group_max_bs(*gr) : 0;
   const bool r64 = a.R % 64 == 0, r1632 = a.R == 16 || a.R == 32;
   const bool half_warp = variant == 20 || variant == 22;
-  if (gr && half_warp && maxbs <= 2 && (r64 || r1632)) {
+  if (gr && variant >= 24 && variant <= 26) {
+    launch_groupn_variant(maxbs, a, *gr, variant, st);
+  } else if (gr && half_warp && maxbs <= 2 && (r64 || r1632)) {
     launch_group4_variant(r64 ? 16 : a.R == 32 ? 8 : 4, a, *gr, variant, st);
   } else if (gr && r64 && ((variant >= 9 && variant <= 14) || half_warp)) {
     // 3-DOF node blocks take the warp-per-node form

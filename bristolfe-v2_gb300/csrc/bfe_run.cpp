@@ -111,7 +111,7 @@ int prepare_run(bfe_plan* pl, std::vector<ForceEntry>& frc, const std::vector<in
     CUDA_TRY(bfe::launch_cast_f64_to_f32(d_sig64, ra.sig32.p, n_t * n_sig, st));
     dsig = ra.sig32.p;
   }
-  if (pl->n_int) CUDA_TRY(ra.vint.alloc((size_t)pl->n_int * R * es));
+  if (pl->n_int) CUDA_TRY(ra.vint.alloc((size_t)pl->n_int * bfe::padded_sources(prec, R, pl->have_groups) * es));
   if (R > 1) {
     const size_t smem = bfe::batched_smem_bytes(prec, pl->max_slice_entries);
     if (smem > 227 * 1024) return fail(BFE_ERR_UNSUPPORTED, "operator rows too long for the batched kernel");
@@ -119,7 +119,8 @@ int prepare_run(bfe_plan* pl, std::vector<ForceEntry>& frc, const std::vector<in
   }
   a = bfe::StepArgs{};
   a.n = (int32_t)n;
-  a.R = (int32_t)R;
+  a.R = bfe::padded_sources(prec, R, pl->have_groups);
+  a.R_out = (int32_t)R;
   a.n_slices = pl->n_slices;
   a.slice_ptr = pl->slice_ptr.p;
   a.col = pl->col.p;
@@ -249,7 +250,7 @@ int execute(bfe_plan* pl, RunSpec& rs, cudaStream_t st) {
   int prc = prepare_run(pl, rs.frc, rs.hist_idx, R, rs.n_t, rs.n_sig, rs.d_sig64, rs.d_hist, st, ra, a);
   if (prc) return prc;
   DevBuf<unsigned char> d_u;
-  const size_t state_bytes = (size_t)n * R * es;
+  const size_t state_bytes = (size_t)n * a.R * es;
   CUDA_TRY(d_u.alloc(3 * state_bytes));
   unsigned char* U[3] = {d_u.p, d_u.p + state_bytes, d_u.p + 2 * state_bytes};
   int iprev = 0, icur = 1, inew = 2;
@@ -296,7 +297,7 @@ int execute(bfe_plan* pl, RunSpec& rs, cudaStream_t st) {
     CUDA_TRY(cudaMemsetAsync(d_u.p, 0, 3 * state_bytes, st));
     int cand[8];
     const int max_bs = grp ? bfe::group_max_bs(*grp) : 0;
-    const int nc = bfe::batched_candidates(prec, (int)R, pl->have_groups, max_bs, cand);
+    const int nc = bfe::batched_candidates(prec, a.R, pl->have_groups, max_bs, cand);
     variant = cand[0];
     const TuneKey key{pl->device, prec, max_bs, n, pl->nnz_operator, R};
     auto it = pl->variant_of_R.find(R);
@@ -494,7 +495,7 @@ int execute(bfe_plan* pl, RunSpec& rs, cudaStream_t st) {
   // non-finite values anywhere in the march stay in the state (every row's
   // update includes its own previous value), so one check of the newest
   // state finds them
-  CUDA_TRY(bfe::launch_nonfinite_check(U[icur], n * R, prec, pl->d_flag.p, st));
+  CUDA_TRY(bfe::launch_nonfinite_check(U[icur], n * a.R, prec, pl->d_flag.p, st));
   stt.aux_launches++;
   CUDA_TRY(cudaStreamSynchronize(st));
   int nonfinite = 0;
