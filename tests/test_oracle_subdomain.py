@@ -103,3 +103,24 @@ def test_oracle_subdomain_forces_reproduce_the_field(in_or_out):
     assert np.abs(U[kept]).max() > 1e-3 * scale
     assert np.abs(V[kept] - U[kept]).max() <= 1e-12 * scale
     assert np.abs(V[~kept]).max() <= 1e-12 * scale
+
+
+def test_pair_lists_of_shared_and_own_monitor_lists():
+    """The product's receiver rows per (transmitter, receiver) pair: for
+    monitor lists shared by all steps and lists of their own, repeated pairs,
+    receivers without monitored nodes and weights, against the definition
+    (ismember of the step's monitors in the receiver's nodes, in their order)."""
+    from bfe_gb300 import fmc
+    rng = np.random.default_rng(5)
+    nds = [np.array([3, 7]), np.array([9]), np.zeros(0, int), np.array([1, 2, 3, 9])]
+    for mons in ([np.arange(10)] * 3, [np.arange(10), np.array([9, 3, 7]), np.array([2])]):
+        shared = mons[0] is mons[1]
+        wts = [rng.random(np.isin(mons[0], n).sum()) for n in nds] if shared else None
+        tx, rx = rng.integers(0, 3, 40), rng.integers(0, 4, 40)
+        p, s, w = fmc._pair_lists(tx, rx, mons, nds, wts)
+        for k, (a, b) in enumerate(zip(tx, rx)):
+            sel = np.nonzero(np.isin(mons[a], nds[b]))[0]
+            assert np.array_equal(s[p[k]:p[k + 1]], sel)
+            assert np.array_equal(w[p[k]:p[k + 1]], wts[b] if shared else np.ones(sel.size))
+    p, s, w = fmc._pair_lists([], [], [np.arange(3)], nds, None)
+    assert p.tolist() == [0] and s.size == 0 and w.size == 0
