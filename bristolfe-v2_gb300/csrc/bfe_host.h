@@ -202,6 +202,14 @@ struct ForceEntry {
   double w;
 };
 
+// Host lists behind V5Args: rows and slots of the listed entries, K and C
+// rows of the slots.
+struct V5Lists {
+  std::vector<int32_t> ent_row, ent_slot, kp, kc, cp, cc, slot_row;
+  std::vector<double> kv, cv;
+  bool corrections = false;        // rows coupled by C to a prescribed DOF
+};
+
 struct RunSpec {
   int64_t R = 1, n_t = 0, ti_start = 0;
   std::vector<ForceEntry> frc;     // one per (row, rhs) after last-wins dedupe
@@ -217,6 +225,7 @@ struct RunSpec {
   const bfe::FieldArgs* field = nullptr;  // frames reduced to element values (bfe_run_field)
   double* d_el = nullptr;          // device n_el x n_frames
   const bfe::V5Args* v5 = nullptr; // prescribed-displacement rows (bfe_run_v5)
+  const V5Lists* v5_lists = nullptr;
   double* d_ud[2] = {nullptr, nullptr};
 };
 
@@ -237,7 +246,18 @@ int execute(bfe_plan* pl, RunSpec& rs, cudaStream_t st);
 // it is usable afterwards); with the run's forced rows, its shared memory and
 // thread count are set. false: this run does not fit.
 int onchip_prepare(bfe_plan* pl, cudaStream_t st);
-bool onchip_fit(bfe_plan* pl, const std::vector<ForceEntry>& frc, bfe::OnchipArgs& o);
+bool onchip_fit(bfe_plan* pl, const std::vector<ForceEntry>& frc, const std::vector<int64_t>& v5_bytes,
+                const std::vector<int32_t>& v5_count, bfe::OnchipArgs& o);
+// Device data of a run's prescribed displacements for the on-chip march, and
+// what each part needs for them; fits = false: they do not fit the form.
+struct OnchipV5 {
+  DevBuf<int32_t> ptr, ent, row, kptr;
+  DevBuf<uint16_t> kcol;
+  DevBuf<double> kval, c;
+  std::vector<int64_t> bytes;
+  std::vector<int32_t> count;
+};
+int onchip_v5(bfe_plan* pl, const V5Lists& L, OnchipV5& d, bool& fits);
 bool outputs_valid(int rc);
 int64_t first_nonzero_column(const double* frcs, int64_t rows, int64_t n_t, int64_t R);
 int check_time(bfe_plan* pl, int64_t n_t, const double* time);

@@ -174,6 +174,16 @@ struct OnchipArgs {
   int64_t xv_stride;
   uint32_t tag0;                    // step ti carries tag0 + ti
   int* err;                         // set when a wait ran out
+  // v5 prescribed displacements (nullptr: none): the entries of V5Args by
+  // part, each with its K row in window indices
+  const int32_t* v5_ptr;            // first entry of each part (n_parts + 1)
+  const int32_t* v5_ent;            // number in the force output
+  const int32_t* v5_row;            // row within the part
+  const int32_t* v5_kptr;           // K row of each entry: v5_kcol, v5_kval
+  const uint16_t* v5_kcol;
+  const double* v5_kval;
+  const double* v5_c;               // diagonal of C at the DOF
+  double* v5_ud;                    // dynamic velocity per slot, from launch to launch
 };
 // Inputs and outputs of building it.
 struct OnchipBuild {
@@ -204,8 +214,10 @@ struct OnchipBuild {
 int onchip_block_bound(int precision, int width);    // most bytes of a slice of this width
 cudaError_t launch_onchip_build(const OnchipBuild& b, int precision, cudaStream_t s);
 // n_steps steps from ti0. fresh: from rest, else from a.u_n, a.u_prev. The
-// newest state is written to a.u_new, the one before it to a.u_prev.
-cudaError_t launch_onchip(const OnchipArgs& o, const StepArgs& a, int precision, int64_t ti0, int64_t n_steps,
+// newest state is written to a.u_new, the one before it to a.u_prev. v: the
+// prescribed displacements when o.v5_ptr is set.
+struct V5Args;
+cudaError_t launch_onchip(const OnchipArgs& o, const StepArgs& a, const V5Args& v, int precision, int64_t ti0, int64_t n_steps,
                           int fresh, cudaStream_t s);
 
 // Prescribed displacements of the v5 scheme (fn_explicit_dynamic_solver_v5.m

@@ -262,7 +262,8 @@ int onchip_prepare(bfe_plan* pl, cudaStream_t st) {
   return BFE_OK;
 }
 
-bool onchip_fit(bfe_plan* pl, const std::vector<ForceEntry>& frc, bfe::OnchipArgs& o) {
+bool onchip_fit(bfe_plan* pl, const std::vector<ForceEntry>& frc, const std::vector<int64_t>& v5_bytes,
+                const std::vector<int32_t>& v5_count, bfe::OnchipArgs& o) {
   const Onchip& oc = *pl->onchip;
   o = oc.args;
   const int P = o.n_parts;
@@ -270,6 +271,12 @@ bool onchip_fit(bfe_plan* pl, const std::vector<ForceEntry>& frc, bfe::OnchipArg
   for (size_t k = 0; k < frc.size(); ++k) rows[k] = frc[k].row;
   std::sort(rows.begin(), rows.end());
   if (std::adjacent_find(rows.begin(), rows.end()) != rows.end()) return false;
+  // prescribed entries get warps of their own where there are some left
+  if (!v5_count.empty()) {
+    const int32_t most = *std::max_element(v5_count.begin(), v5_count.end());
+    o.threads = std::min(o.threads <= 512 ? 512 : 1024, o.threads + (most + 31) / 32 * 32);
+    if (most > o.threads) return false;
+  }
   // slots per warp for streamed chunks: up to four as long as they take no
   // more than half of the memory the operator has
   const int64_t warps = o.threads / 32;
@@ -281,7 +288,8 @@ bool onchip_fit(bfe_plan* pl, const std::vector<ForceEntry>& frc, bfe::OnchipArg
         std::lower_bound(rows.begin(), rows.end(), oc.part_slice[p + 1] * bfe::kSlice) -
         std::lower_bound(rows.begin(), rows.end(), oc.part_slice[p] * bfe::kSlice);
     if (nf > o.threads) return false;
-    need[p] = oc.need[p] + 2 * nf * (int64_t)elem_size(pl->prec) + 16 + nf * 4 + (warps * 4 + 1) * 8 + 16;
+    need[p] = oc.need[p] + 2 * nf * (int64_t)elem_size(pl->prec) + 16 + nf * 4 + (warps * 4 + 1) * 8 + 16 +
+              (v5_bytes.empty() ? 0 : v5_bytes[p]);
     room = std::min(room, kSmemLimit - need[p]);
     stream = stream || need[p] + oc.op_bytes[p] > kSmemLimit;
   }
@@ -292,6 +300,72 @@ bool onchip_fit(bfe_plan* pl, const std::vector<ForceEntry>& frc, bfe::OnchipArg
   for (int p = 0; p < P; ++p) smem = std::max(smem, std::min<int64_t>(kSmemLimit, need[p] + oc.op_bytes[p]));
   o.smem = (int32_t)(smem & ~(int64_t)15);
   return true;
+}
+
+// The form serves prescribed DOFs whose C row is at most its diagonal (no
+// fluid-solid coupling), without correction rows, with K rows inside the
+// part's window.
+int onchip_v5(bfe_plan* pl, const V5Lists& L, OnchipV5& d, bool& fits) {
+  fits = false;
+  if (L.corrections) return BFE_OK;
+  const Onchip& oc = *pl->onchip;
+  const int P = oc.args.n_parts;
+  const int64_t ne = (int64_t)L.ent_row.size();
+  std::vector<int32_t> ord(ne), ptr(P + 1, 0), row(ne), kptr(1, 0), cnt(P);
+  std::iota(ord.begin(), ord.end(), 0);
+  std::stable_sort(ord.begin(), ord.end(), [&](int32_t x, int32_t y) { return L.ent_row[x] < L.ent_row[y]; });
+  std::vector<uint16_t> kcol;
+  std::vector<double> kval, c(ne, 0.0);
+  CUDA_TRY(cudaMemcpy(cnt.data(), oc.d_cnt.p, P * sizeof(int32_t), cudaMemcpyDeviceToHost));
+  d.bytes.assign(P, 0);
+  d.count.assign(P, 0);
+  int64_t e = 0;
+  for (int p = 0; p < P; ++p) {
+    const int64_t r0 = (int64_t)oc.part_slice[p] * bfe::kSlice, rpad = (int64_t)oc.part_slice[p + 1] * bfe::kSlice - r0;
+    const int64_t r1 = std::min<int64_t>(pl->n, r0 + rpad);
+    std::vector<int32_t> halo;
+    std::map<int32_t, int32_t> at;             // halo row -> window index
+    const size_t k0 = kcol.size();
+    for (; e < ne && L.ent_row[ord[e]] < r1; ++e) {
+      const int32_t s = L.ent_slot[ord[e]];
+      row[e] = (int32_t)(L.ent_row[ord[e]] - r0);
+      for (int32_t x = L.cp[s]; x < L.cp[s + 1]; ++x) {
+        if (L.cc[x] != L.slot_row[s]) return BFE_OK;
+        c[e] = L.cv[x];
+      }
+      if (halo.empty() && cnt[p]) {
+        halo.resize(cnt[p]);
+        CUDA_TRY(cudaMemcpy(halo.data(), oc.d_halo.p + (size_t)p * oc.args.halo_cap, cnt[p] * sizeof(int32_t),
+                            cudaMemcpyDeviceToHost));
+        for (int32_t k = 0; k < cnt[p]; ++k) at.emplace(halo[k], (int32_t)rpad + k);
+      }
+      for (int32_t x = L.kp[s]; x < L.kp[s + 1]; ++x) {
+        const int32_t col = L.kc[x];
+        int64_t w = col - r0;
+        if (col < r0 || col >= r1) {
+          auto it = at.find(col);
+          if (it == at.end()) return BFE_OK;
+          w = it->second;
+        }
+        kcol.push_back((uint16_t)w);
+        kval.push_back(L.kv[x]);
+      }
+      kptr.push_back((int32_t)kcol.size());
+      ++d.count[p];
+    }
+    ptr[p + 1] = (int32_t)e;
+    d.bytes[p] = (int64_t)(kcol.size() - k0) * 8 + align2(kcol.size() - k0) * 2;
+  }
+  CUDA_TRY(d.ptr.upload(ptr));
+  CUDA_TRY(d.ent.upload(ord));
+  CUDA_TRY(d.row.upload(row));
+  CUDA_TRY(d.kptr.upload(kptr));
+  CUDA_TRY(d.kcol.upload(kcol));
+  CUDA_TRY(d.kval.upload(kval));
+  CUDA_TRY(d.c.upload(c));
+  CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
+  fits = true;
+  return BFE_OK;
 }
 
 }  // namespace bfe_host

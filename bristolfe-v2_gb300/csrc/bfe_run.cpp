@@ -169,7 +169,7 @@ int march_on_chip(bfe_plan* pl, RunSpec& rs, bfe::StepArgs a, unsigned char* con
                   cudaStream_t st, DevBuf<double>& d_raw, bool& done) {
   done = false;
   const int64_t steps = rs.n_t - rs.ti_start;
-  if (pl->timing || pl->time_limit_s > 0.0 || rs.v5 || steps < kOnchipMinSteps || rs.n_t >= ((int64_t)1 << 30) ||
+  if (pl->timing || pl->time_limit_s > 0.0 || (rs.v5 && !rs.v5_lists) || steps < kOnchipMinSteps || rs.n_t >= ((int64_t)1 << 30) ||
       getenv("BFE_NO_GRAPH"))
     return BFE_OK;
   const int64_t n_frames = frames ? (rs.n_t + rs.every_n - 1) / rs.every_n : 0;
@@ -183,7 +183,33 @@ int march_on_chip(bfe_plan* pl, RunSpec& rs, bfe::StepArgs a, unsigned char* con
     return BFE_OK;
   }
   bfe::OnchipArgs o;
-  if (pl->onchip->state != 1 || !onchip_fit(pl, rs.frc, o)) return BFE_OK;
+  if (pl->onchip->state != 1) return BFE_OK;
+  OnchipV5 v5;
+  if (rs.v5) {
+    bool fits = false;
+    const int rc = onchip_v5(pl, *rs.v5_lists, v5, fits);
+    if (rc) return rc;
+    if (!fits) return BFE_OK;
+  }
+  if (!onchip_fit(pl, rs.frc, v5.bytes, v5.count, o)) return BFE_OK;
+  bfe::V5Args q5{};
+  if (rs.v5) {
+    q5 = *rs.v5;
+    o.v5_ptr = v5.ptr.p;
+    o.v5_ent = v5.ent.p;
+    o.v5_row = v5.row.p;
+    o.v5_kptr = v5.kptr.p;
+    o.v5_kcol = v5.kcol.p;
+    o.v5_kval = v5.kval.p;
+    o.v5_c = v5.c.p;
+    o.v5_ud = rs.d_ud[0];
+    if (frames) {
+      a.fld = rs.d_fld;
+      a.fld_every = rs.every_n;
+      a.fld_is_vel = rs.field_is_vel;
+      a.dt = pl->dt;
+    }
+  }
   if (raw) {
     a.fld = d_raw.p;
     a.fld_every = rs.every_n;
@@ -206,7 +232,7 @@ int march_on_chip(bfe_plan* pl, RunSpec& rs, bfe::StepArgs a, unsigned char* con
     a.u_prev = U[prev];
     a.u_n = U[cur];
     a.u_new = U[next];
-    if (bfe::launch_onchip(o, a, pl->prec, ti, k, ti == rs.ti_start, st) != cudaSuccess) {
+    if (bfe::launch_onchip(o, a, q5, pl->prec, ti, k, ti == rs.ti_start, st) != cudaSuccess) {
       cudaGetLastError();          // not launchable here
       CUDA_TRY(cudaStreamSynchronize(st));
       return BFE_OK;
@@ -222,6 +248,7 @@ int march_on_chip(bfe_plan* pl, RunSpec& rs, bfe::StepArgs a, unsigned char* con
   CUDA_TRY(cudaStreamSynchronize(st));
   if (gave_up) {                   // CTAs were not running together: march step by step
     pl->onchip->state = -1;
+    if (rs.v5) CUDA_TRY(cudaMemsetAsync(rs.d_ud[0], 0, 2 * rs.v5->n_slot * sizeof(double), st));
     return BFE_OK;
   }
   if (cur != 1)
@@ -866,6 +893,7 @@ int bfe_run_v5(bfe_plan* plan, int64_t n_t, const double* time,
     rs.fld_time = &ftime;
   }
   bfe::V5Args v{};
+  const V5Lists lists{ent_row, ent_slot, kp, kc, cp, cc, slot_row, kv, cv, !crow.empty()};
   const size_t fout_n = (size_t)r * n_t;
   if (ns) {
     CUDA_TRY(d_er.upload(ent_row));
@@ -922,6 +950,7 @@ int bfe_run_v5(bfe_plan* plan, int64_t n_t, const double* time,
     v.h_slot = d_hs.p;
     v.dt = dt;
     rs.v5 = &v;
+    rs.v5_lists = &lists;
     rs.d_ud[0] = d_ud.p;
     rs.d_ud[1] = d_ud.p + ns;
   }

@@ -113,3 +113,31 @@ def test_element_fields(bfe, models, ftype, monkeypatch):
 
     on, off = _both(bfe, monkeypatch, run)
     assert np.abs(off).max() > 0 and np.array_equal(on, off)
+
+
+@pytest.mark.parametrize("prec", ["double", "single"])
+@pytest.mark.parametrize("name,cut", [("ragged", 0), ("plate", 0), ("coupled", 5)])
+def test_v5_prescribed_displacements(bfe, models, name, cut, prec, monkeypatch):
+    """Prescribed DOFs on chip: a repeated one (the last entry sets it), one
+    that is forced too, one that is monitored, rows with absorbing damping;
+    reactions and frames included."""
+    m, _ = models[name]
+    nt = 260
+    t, s = modelgen.pulse(nt, m["dt"])
+    nds = m["mod"]["nds"]
+    low = np.nonzero(nds[:, 1] < nds[:, 1].max() / 3)[0] + 1            # solid, away from the interface
+    low = low[np.linspace(cut, low.size - 1, 37).astype(int)]
+    di = modelgen.gi_of(m["gl"], low, 2)
+    di = np.concatenate([di, di[:1]])
+    D = 1e-9 * np.linspace(0.5, 1.0, di.size)[:, None] * np.roll(s, 9)[None, :]
+    fi = np.concatenate([modelgen.gi_of(m["gl"], [m["frc_nd"]], 4 if name == "coupled" else 2), di[3:4]])
+    hi = np.concatenate([di[:4], modelgen.gi_of(m["gl"], low + 1, 1)])
+
+    def run():
+        with bfe.Plan(m["K"], m["C"], m["M"], m["dt"], bfe.V5, prec, m["gl"], one_source=True) as plan:
+            h, f, frc, _ = plan.run_v5(t, fi, s, di, D, hi, 45)
+            return (h, f, frc), plan.stats()["step_launches"]
+
+    on, off = _both(bfe, monkeypatch, run)
+    for a, b in zip(on, off):
+        assert np.abs(b).max() > 0 and np.array_equal(a, b)
