@@ -144,6 +144,9 @@ struct Onchip {
 }  // namespace bfe_host
 
 struct bfe_plan {
+  bfe_plan() = default;
+  bfe_plan(const bfe_plan&) = delete;
+  ~bfe_plan() { if (stream) cudaStreamDestroy(stream); }
   int64_t n = 0;
   int32_t mode = 0, prec = 0;
   double dt = 0;

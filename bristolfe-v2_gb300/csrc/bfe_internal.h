@@ -148,6 +148,31 @@ cudaError_t launch_frame(const StepArgs& a, int precision, double* fld, int64_t 
 cudaError_t launch_cast_f64_to_f32(const double* in, float* out, int64_t n, cudaStream_t s);
 cudaError_t launch_advance(int64_t* ti_dev, int64_t k, cudaStream_t s);
 
+// Packing of a one-source plan's sliced-ELL operator from CSR arrays on the
+// device (bfe_pack.cu).
+struct PackArgs {
+  int64_t n, nnz, n_slices;
+  const int64_t* ptr;
+  const int64_t* idx;
+  const double* val;
+  const double* lscale;             // per row: factor of K, and the diagonal term of B (FP64)
+  const double* diag;
+  const int64_t* dof_node;          // FP32 with node information, else nullptr
+  const int32_t* dof_type;
+  const int32_t* blk_base;          // node block of each row
+  const int32_t* blk_len;
+  uint32_t* base;                   // out, FP32: node-block base (0: direct row)
+  uint8_t* diff;                    // out, FP32: difference form
+  int32_t* width;                   // out: entries per row of each slice
+  int64_t* totals;                  // out: stored entries, direct rows (zeroed)
+  int* irregular;                   // out (zeroed): leave the matrix to the host
+  const int32_t* slice_ptr;         // second pass
+  uint32_t* col;
+  void* out;
+};
+cudaError_t launch_pack_count(const PackArgs& p, int precision, cudaStream_t s);
+cudaError_t launch_pack_write(const PackArgs& p, int precision, cudaStream_t s);
+
 // One-source march that keeps state and operator on the chip (bfe_onchip.cu).
 // Device data of a plan's partition; the forcing, monitor and interface lists
 // are those of StepArgs.

@@ -338,7 +338,6 @@ int bfe_plan_destroy(bfe_plan* plan) {
   int dev = 0;
   cudaGetDevice(&dev);
   cudaSetDevice(plan->device);
-  if (plan->stream) cudaStreamDestroy(plan->stream);
   delete plan;
   cudaSetDevice(dev);
   return BFE_OK;
@@ -354,10 +353,102 @@ int bfe_plan_create(const bfe_sparse* Kv, const bfe_sparse* Cv, const bfe_sparse
 
 namespace {
 
+// The sliced-ELL operator of pl from K's CSR arrays, on the GPU. Called for
+// matrices in row order (checked on the device: false when they are not).
+int pack_on_device(bfe_plan* pl, const bfe_sparse& K, const std::vector<double>& lscale, const std::vector<double>& diag,
+                   const int64_t* dof_node, const int32_t* dof_type, const std::vector<int64_t>& blk_base,
+                   const std::vector<int64_t>& blk_len, int64_t& stored, int64_t& direct_rows) {
+  const int64_t n = pl->n, S = (n + bfe::kSlice - 1) / bfe::kSlice, nnz = K.nnz;
+  const bool f64 = pl->prec == BFE_PREC_DOUBLE, nodes = !f64 && dof_node;
+  // one scratch allocation, 256-byte pieces
+  size_t need = 0;
+  auto piece = [&](size_t bytes) {
+    const size_t at = need;
+    need += (bytes + 255) / 256 * 256;
+    return at;
+  };
+  const size_t o_ptr = piece((n + 1) * 8), o_idx = piece(nnz * 8), o_val = piece(nnz * 8), o_ls = piece(n * 8),
+               o_dg = piece(f64 ? n * 8 : 0), o_node = piece(nodes ? n * 8 : 0), o_type = piece(nodes ? n * 4 : 0),
+               o_bb = piece(nodes ? n * 4 : 0), o_bl = piece(nodes ? n * 4 : 0), o_base = piece(f64 ? 0 : n * 4),
+               o_diff = piece(f64 ? 0 : n), o_w = piece(S * 4), o_tot = piece(32);
+  DevBuf<unsigned char> d;
+  CUDA_TRY(d.alloc(need));
+  cudaStream_t st = pl->stream;
+  auto put = [&](size_t at, const void* h, size_t bytes) {
+    return bytes ? cudaMemcpyAsync(d.p + at, h, bytes, cudaMemcpyHostToDevice, st) : cudaSuccess;
+  };
+  std::vector<int32_t> bb, bl;
+  CUDA_TRY(put(o_ptr, K.ptr, (n + 1) * 8));
+  CUDA_TRY(put(o_idx, K.idx, nnz * 8));
+  CUDA_TRY(put(o_val, K.val, nnz * 8));
+  CUDA_TRY(put(o_ls, lscale.data(), n * 8));
+  if (f64) CUDA_TRY(put(o_dg, diag.data(), n * 8));
+  if (nodes) {
+    bb.assign(blk_base.begin(), blk_base.end());
+    bl.assign(blk_len.begin(), blk_len.end());
+    CUDA_TRY(put(o_node, dof_node, n * 8));
+    CUDA_TRY(put(o_type, dof_type, n * 4));
+    CUDA_TRY(put(o_bb, bb.data(), n * 4));
+    CUDA_TRY(put(o_bl, bl.data(), n * 4));
+  }
+  CUDA_TRY(cudaMemsetAsync(d.p + o_tot, 0, 32, st));
+  bfe::PackArgs a{};
+  a.n = n;
+  a.nnz = nnz;
+  a.n_slices = S;
+  a.ptr = reinterpret_cast<const int64_t*>(d.p + o_ptr);
+  a.idx = reinterpret_cast<const int64_t*>(d.p + o_idx);
+  a.val = reinterpret_cast<const double*>(d.p + o_val);
+  a.lscale = reinterpret_cast<const double*>(d.p + o_ls);
+  a.diag = reinterpret_cast<const double*>(d.p + o_dg);
+  if (nodes) {
+    a.dof_node = reinterpret_cast<const int64_t*>(d.p + o_node);
+    a.dof_type = reinterpret_cast<const int32_t*>(d.p + o_type);
+    a.blk_base = reinterpret_cast<const int32_t*>(d.p + o_bb);
+    a.blk_len = reinterpret_cast<const int32_t*>(d.p + o_bl);
+  }
+  a.base = reinterpret_cast<uint32_t*>(d.p + o_base);
+  a.diff = d.p + o_diff;
+  a.width = reinterpret_cast<int32_t*>(d.p + o_w);
+  a.totals = reinterpret_cast<int64_t*>(d.p + o_tot);
+  a.irregular = reinterpret_cast<int*>(d.p + o_tot + 16);
+  CUDA_TRY(bfe::launch_pack_count(a, pl->prec, st));
+  std::vector<int32_t> width(S), sptr(S + 1, 0);
+  int64_t tot[4];
+  CUDA_TRY(cudaMemcpyAsync(width.data(), a.width, S * 4, cudaMemcpyDeviceToHost, st));
+  CUDA_TRY(cudaMemcpyAsync(tot, a.totals, 32, cudaMemcpyDeviceToHost, st));
+  if (!f64) CUDA_TRY(cudaMemcpyAsync(pl->h_base.data(), a.base, n * 4, cudaMemcpyDeviceToHost, st));
+  CUDA_TRY(cudaStreamSynchronize(st));
+  if ((int)tot[2]) return fail(BFE_ERR_ARG, "K is not in row order");
+  int64_t total = 0;
+  for (int64_t s = 0; s < S; ++s) {
+    total += (int64_t)width[s] * bfe::kSlice;
+    if (total > (int64_t)INT32_MAX) return fail(BFE_ERR_UNSUPPORTED, "operator too large for 32-bit offsets");
+    sptr[s + 1] = (int32_t)total;
+    pl->max_slice_entries = std::max<int32_t>(pl->max_slice_entries, width[s] * bfe::kSlice);
+  }
+  CUDA_TRY(pl->slice_ptr.alloc(S + 1));
+  CUDA_TRY(cudaMemcpyAsync(pl->slice_ptr.p, sptr.data(), (S + 1) * 4, cudaMemcpyHostToDevice, st));
+  CUDA_TRY(pl->col.alloc(total));
+  CUDA_TRY(pl->val.alloc((size_t)total * elem_size(pl->prec)));
+  a.slice_ptr = pl->slice_ptr.p;
+  a.col = pl->col.p;
+  a.out = pl->val.p;
+  CUDA_TRY(bfe::launch_pack_write(a, pl->prec, st));
+  CUDA_TRY(cudaStreamSynchronize(st));
+  pl->h_slice_ptr.swap(sptr);
+  stored = tot[0];
+  direct_rows = tot[1];
+  return BFE_OK;
+}
+
 // Plan creation from owned CSR matrices (bfe_plan_create_ex converts its
-// views; bfe_plan_create_multi hands over the joined operator).
+// views; bfe_plan_create_multi hands over the joined operator). With Kv (a
+// one-source plan), K is only its sizes and the operator is packed from the
+// view on the GPU.
 int create_plan(Csr K, Csr C, Csr M, double dt, int32_t solver_mode, int32_t precision,
-                const int64_t* dof_node, const int32_t* dof_type, uint32_t flags, bfe_plan** out) {
+                const int64_t* dof_node, const int32_t* dof_type, uint32_t flags, bfe_plan** out,
+                const bfe_sparse* Kv = nullptr) {
   if (flags & ~(uint32_t)BFE_PLAN_ONE_SOURCE) return fail(BFE_ERR_ARG, "unknown plan flags 0x%x", flags);
   // the group block-sparse form serves only runs with many right-hand
   // sides; a one-source plan skips building it
@@ -386,6 +477,7 @@ int create_plan(Csr K, Csr C, Csr M, double dt, int32_t solver_mode, int32_t pre
   pl->prec = precision;
   pl->dt = dt;
   CUDA_TRY(cudaGetDevice(&pl->device));
+  CUDA_TRY(cudaStreamCreateWithFlags(&pl->stream, cudaStreamNonBlocking));
 
   // lumped mass: sum(M).' = column sums (v6.m:122-123)
   std::vector<double> m(n, 0.0);
@@ -465,9 +557,18 @@ int create_plan(Csr K, Csr C, Csr M, double dt, int32_t solver_mode, int32_t pre
     int64_t stored = 0, direct = 0;
   };
   pl->h_base.assign(n, 0);
-  const int n_pack = plan_threads(n_slices, 1024);
+  int64_t stored = 0, direct_rows = 0, total = 0;
+  if (Kv) {
+    std::vector<double> diag(f64_ops ? n : 0);
+    for (int64_t i = 0; i < (int64_t)diag.size(); ++i) diag[i] = diag_term(i);
+    if ((rc = pack_on_device(pl.get(), *Kv, lscale, diag, have_nodes ? dof_node : nullptr, dof_type, blk_base, blk_len,
+                             stored, direct_rows)))
+      return rc;
+    total = pl->h_slice_ptr.back();
+  }
+  const int n_pack = Kv ? 1 : plan_threads(n_slices, 1024);
   std::vector<Piece> pieces(n_pack);
-  const bool packed = parallel_chunks(n_slices, n_pack, [&](int t, int64_t s0, int64_t s1) {
+  const bool packed = Kv || parallel_chunks(n_slices, n_pack, [&](int t, int64_t s0, int64_t s1) {
     Piece& pc = pieces[t];
     std::vector<std::pair<uint32_t, double>> rows[bfe::kSlice];
     for (int64_t s = s0; s < s1; ++s) {
@@ -553,9 +654,8 @@ int create_plan(Csr K, Csr C, Csr M, double dt, int32_t solver_mode, int32_t pre
     }
   });
   if (!packed) return fail(BFE_ERR_OOM, "host allocation failed while packing the operator");
-  std::vector<int32_t> sptr(n_slices + 1, 0);
-  int64_t stored = 0, direct_rows = 0, total = 0;
-  {
+  std::vector<int32_t> sptr(Kv ? 0 : n_slices + 1, 0);
+  if (!Kv) {
     int64_t s = 0;
     for (const Piece& pc : pieces) {
       for (int64_t w : pc.width) {
@@ -569,9 +669,9 @@ int create_plan(Csr K, Csr C, Csr M, double dt, int32_t solver_mode, int32_t pre
     }
   }
   const size_t es_ops = f64_ops ? sizeof(double) : sizeof(float);
-  std::vector<uint32_t> hcol((size_t)total);
-  std::vector<unsigned char> hval((size_t)total * es_ops);
-  {
+  std::vector<uint32_t> hcol(Kv ? 0 : (size_t)total);
+  std::vector<unsigned char> hval(hcol.size() * es_ops);
+  if (!Kv) {
     size_t o = 0;
     for (Piece& pc : pieces) {
       const size_t k = pc.col.size();
@@ -765,7 +865,7 @@ int create_plan(Csr K, Csr C, Csr M, double dt, int32_t solver_mode, int32_t pre
     }
   }
   pl->nnz_operator = stored;
-  pl->nnz_padded = (int64_t)hcol.size();
+  pl->nnz_padded = total;
   pl->n_direct_rows = direct_rows;
   pl->h_acoef = acoef;
 
@@ -780,15 +880,13 @@ int create_plan(Csr K, Csr C, Csr M, double dt, int32_t solver_mode, int32_t pre
   pl->h_int_row = irows;
 
   // upload
-  CUDA_TRY(pl->slice_ptr.upload(sptr));
-  pl->h_slice_ptr = sptr;
-  CUDA_TRY(pl->col.upload(hcol));
-  if ((rc = upload_bytes(pl->val, hval))) return rc;
-  std::vector<unsigned char> hrc;
-  for (int64_t i = 0; i < n; ++i) {
-    if (precision == BFE_PREC_DOUBLE) push_val<double>(hrc, rowc[i]); else push_val<float>(hrc, rowc[i]);
+  if (!Kv) {
+    CUDA_TRY(pl->slice_ptr.upload(sptr));
+    pl->h_slice_ptr = sptr;
+    CUDA_TRY(pl->col.upload(hcol));
+    if ((rc = upload_bytes(pl->val, hval))) return rc;
   }
-  if ((rc = upload_bytes(pl->rowc, hrc))) return rc;
+  if ((rc = upload_bytes(pl->rowc, cast_bytes(precision, rowc.data(), n)))) return rc;
   if (pl->n_int) {
     std::vector<int32_t> zp(Z.ptr.begin(), Z.ptr.end()), zc(Z.idx.begin(), Z.idx.end());
     std::vector<unsigned char> zv;
@@ -800,7 +898,6 @@ int create_plan(Csr K, Csr C, Csr M, double dt, int32_t solver_mode, int32_t pre
     pl->h_z_col = zc;
     if ((rc = upload_bytes(pl->z_val, zv))) return rc;
   }
-  CUDA_TRY(cudaStreamCreateWithFlags(&pl->stream, cudaStreamNonBlocking));
   if (solver_mode == BFE_MODE_V5) {
     pl->hK = std::move(K);
     pl->hC = std::move(C);
@@ -822,6 +919,21 @@ int bfe_plan_create_ex(const bfe_sparse* Kv, const bfe_sparse* Cv, const bfe_spa
   *out = nullptr;
   Csr K, C, M;
   int rc;
+  // A one-source plan packs K on the GPU (a v5 plan keeps K on the host).
+  // Whatever that path does not take or cannot do is left to the path below,
+  // which reports errors in its own order.
+  if ((flags & BFE_PLAN_ONE_SOURCE) && solver_mode != BFE_MODE_V5 && Kv && Kv->format == BFE_CSR && Kv->n_rows > 0 &&
+      Kv->n_rows == Kv->n_cols && Kv->n_rows <= bfe::kMaxDof && Kv->nnz >= 0 && Kv->ptr && (Kv->nnz == 0 || (Kv->idx && Kv->val)) &&
+      Kv->ptr[0] == 0 && Kv->ptr[Kv->n_rows] == Kv->nnz && to_csr(Cv, "C", C) == BFE_OK && to_csr(Mv, "M", M) == BFE_OK) {
+    K.n = K.m = Kv->n_rows;
+    if (create_plan(std::move(K), std::move(C), std::move(M), dt, solver_mode, precision, dof_node, dof_type, flags, out,
+                    Kv) == BFE_OK)
+      return BFE_OK;
+    cudaGetLastError();
+    *out = nullptr;
+    K = Csr();
+  }
+  g_last_error.clear();
   if ((rc = to_csr(Kv, "K", K))) return rc;
   if ((rc = to_csr(Cv, "C", C))) return rc;
   if ((rc = to_csr(Mv, "M", M))) return rc;
