@@ -131,7 +131,9 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
     auto it = pl->variant_of_R.find(R);
     if (it != pl->variant_of_R.end()) variant = it->second;
   }
+  int64_t launches = 0;
   auto step = [&](bfe::StepArgs& a) -> int {
+    ++launches;
     cudaError_t e = R == 1 ? bfe::launch_step(a, prec, st)
                            : bfe::launch_step_batched(a, grp, prec, pl->max_slice_entries, variant, st);
     if (e != cudaSuccess) return fail(BFE_ERR_CUDA, "step kernel launch failed: %s", cudaGetErrorString(e));
@@ -142,6 +144,66 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
     return BFE_OK;
   };
   const size_t sb = (size_t)n * Rp * es;
+  // Marches that fit on the chip run there (bfe_onchip_multi.cu), writing
+  // every state to its slot: one launch for the forward march and one per
+  // segment instead of one per step.
+  if (!pl->d_flag.p) CUDA_TRY(pl->d_flag.alloc(2));
+  CUDA_TRY(cudaMemsetAsync(pl->d_flag.p, 0, 2 * sizeof(int), st));
+  auto rows_of = [](const std::vector<ForceEntry>& f) {
+    std::vector<int32_t> r;
+    for (auto& x : f) r.push_back(x.row);
+    std::sort(r.begin(), r.end());
+    return r;
+  };
+  // steps t, t + dir, ... (count of them) from the states un, up (fresh: from
+  // rest), each new state to out + k * dir * sb; false: not launched
+  auto chip_march = [&](const bfe::OnchipArgs& oa, bfe::StepArgs a, int64_t t, int64_t dir, int64_t count, bool fresh,
+                        unsigned char* un, unsigned char* up, unsigned char* out) -> bool {
+    constexpr int64_t kSteps = 8192;                // per launch: bounds how long one kernel runs
+    for (int64_t k = 0; k < count; k += kSteps) {
+      const int64_t m_steps = std::min(kSteps, count - k);
+      bfe::OnchipArgs o = oa;
+      if (onchip_tags(pl, m_steps, st, o.tag0)) return false;
+      o.err = pl->d_flag.p + 1;
+      a.u_n = un;
+      a.u_prev = up;
+      a.u_new = nullptr;
+      bfe::OnchipMulti m{};
+      m.ti0 = t + dir * k;
+      m.ti_step = dir;
+      m.out = out + dir * k * (int64_t)sb;
+      m.out_stride = dir * n * Rp;
+      if (bfe::launch_onchip_multi(o, a, m, prec, m_steps, fresh && k == 0, st) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+      }
+      ++launches;
+      un = static_cast<unsigned char*>(m.out) + dir * (m_steps - 1) * (int64_t)sb;
+      up = un - dir * (int64_t)sb;
+    }
+    return true;
+  };
+  auto gave_up = [&](bool& yes) -> int {            // after a synchronisation point
+    int e = 0;
+    CUDA_TRY(cudaMemcpy(&e, pl->d_flag.p + 1, sizeof(int), cudaMemcpyDeviceToHost));
+    yes = e != 0;
+    if (yes) {
+      pl->onchip->state = -1;
+      CUDA_TRY(cudaMemsetAsync(pl->d_flag.p, 0, 2 * sizeof(int), st));
+    }
+    return BFE_OK;
+  };
+  bfe::OnchipArgs of, oa;
+  bool chip = onchip_multi_may_fit(pl, Rp) && Rp <= 16 && c >= 8 && !pl->timing && !getenv("BFE_NO_GRAPH") && n_t < ((int64_t)1 << 30);
+  if (chip && onchip_prepare(pl, st)) {
+    if (pl->onchip->state == 0) pl->onchip->state = -1;
+    cudaGetLastError();
+    g_last_error.clear();
+  }
+  chip = chip && pl->onchip->state == 1;
+  std::vector<int32_t> mrows(hidx.begin(), hidx.end());
+  std::sort(mrows.begin(), mrows.end());
+  chip = chip && onchip_multi_fit(pl, af, rows_of(frc), mrows, false, st, of);
   // With ckpt_every = 0, every forward state stays on the device when the
   // steps + 2 states and the adjoint's c + 2 segment slots fit in 3/4 of the
   // free memory: state u_t sits in slot t - ti0 + 2 of d_all (slots 0 and 1
@@ -165,18 +227,22 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
   stt.variant = variant;
   stt.adjoint_segments = n_seg;
   stt.adjoint_kept = keep_all ? 1 : 0;
-  stt.step_launches = (keep_all ? 2 : 3) * steps;
   DevBuf<unsigned char> d_u, d_ck, d_all;
-  if (keep_all) {
-    CUDA_TRY(d_all.alloc((size_t)(steps + 2) * sb));
-    CUDA_TRY(cudaMemsetAsync(d_all.p, 0, 2 * sb, st));
+  auto forward_steps = [&]() -> int {
     for (int64_t t = ti0; t < n_t; ++t) {
       af.ti = t;
       af.u_prev = d_all.p + (size_t)(t - ti0) * sb;
       af.u_n = d_all.p + (size_t)(t - ti0 + 1) * sb;
       af.u_new = d_all.p + (size_t)(t - ti0 + 2) * sb;
-      if ((rc = step(af))) return rc;
+      if (int r = step(af)) return r;
     }
+    return BFE_OK;
+  };
+  if (keep_all) {
+    CUDA_TRY(d_all.alloc((size_t)(steps + 2) * sb));
+    CUDA_TRY(cudaMemsetAsync(d_all.p, 0, 2 * sb, st));
+    chip = chip && chip_march(of, af, ti0, 1, steps, true, nullptr, nullptr, d_all.p + 2 * sb);
+    if (!chip && (rc = forward_steps())) return rc;
   } else {
     CUDA_TRY(d_u.alloc(3 * sb));
     CUDA_TRY(cudaMemsetAsync(d_u.p, 0, 3 * sb, st));
@@ -273,6 +339,16 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
   std::vector<double> hist(hist_n);
   CUDA_TRY(cudaMemcpyAsync(hist.data(), d_hist.p, hist_n * sizeof(double), cudaMemcpyDeviceToHost, st));
   CUDA_TRY(cudaStreamSynchronize(st));
+  if (chip && keep_all) {
+    bool yes = false;
+    if ((rc = gave_up(yes))) return rc;
+    if (yes) {
+      chip = false;
+      if ((rc = forward_steps())) return rc;
+      CUDA_TRY(cudaMemcpyAsync(hist.data(), d_hist.p, hist_n * sizeof(double), cudaMemcpyDeviceToHost, st));
+      CUDA_TRY(cudaStreamSynchronize(st));
+    }
+  }
   if (hist_out) std::memcpy(hist_out, hist.data(), hist_n * sizeof(double));
   const int64_t n_rsig = q * R;
   std::vector<double> res((size_t)n_t * n_rsig, 0.0);
@@ -304,16 +380,11 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
   DevBuf<double> d_gs, d_gr;
   if (!keep_all) CUDA_TRY(d_seg.alloc((size_t)(c + 2) * sb));
   CUDA_TRY(d_lam.alloc((size_t)(c + 2) * sb));
-  CUDA_TRY(cudaMemsetAsync(d_lam.p, 0, (size_t)(c + 2) * sb, st));
   CUDA_TRY(d_gs.alloc(n_el));
   CUDA_TRY(d_gr.alloc(n_el));
-  CUDA_TRY(cudaMemsetAsync(d_gs.p, 0, n_el * sizeof(double), st));
-  CUDA_TRY(cudaMemsetAsync(d_gr.p, 0, n_el * sizeof(double), st));
   DevBuf<double> d_pw, d_pv;
   CUDA_TRY(d_pw.alloc(n));
   CUDA_TRY(d_pv.alloc(n));
-  CUDA_TRY(cudaMemsetAsync(d_pw.p, 0, n * sizeof(double), st));
-  CUDA_TRY(cudaMemsetAsync(d_pv.p, 0, n * sizeof(double), st));
   auto S = [&](int64_t k) { return d_seg.p + (size_t)k * sb; };
   auto Lm = [&](int64_t k) { return d_lam.p + (size_t)k * sb; };
   af.n_mon = 0;                      // the recompute does not rewrite the history
@@ -339,41 +410,66 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
     g.el_dof_w = d_dof_w.p;
     g.el_out = d_out.p;
   }
-  for (int64_t j = n_seg - 1; j >= 0; --j) {
-    const int64_t ts = ti0 + j * c, te = std::min(ts + c, n_t);
-    if (keep_all) {
-      g.u = d_all.p + (size_t)(ts - ti0) * sb;        // slot k: u_{ts + k - 2}
-    } else {
-      CUDA_TRY(cudaMemcpyAsync(S(0), d_ck.p + 2 * sb * j, 2 * sb, cudaMemcpyDeviceToDevice, st));
-      for (int64_t t = ts; t < te; ++t) {
-        af.ti = t;
-        af.u_prev = S(t - ts);
-        af.u_n = S(t - ts + 1);
-        af.u_new = S(t - ts + 2);
-        if ((rc = step(af))) return rc;
+  constexpr int kNotLaunched = -1;
+  auto sweep = [&](bool use_chip) -> int {
+    CUDA_TRY(cudaMemsetAsync(d_lam.p, 0, (size_t)(c + 2) * sb, st));
+    CUDA_TRY(cudaMemsetAsync(d_gs.p, 0, n_el * sizeof(double), st));
+    CUDA_TRY(cudaMemsetAsync(d_gr.p, 0, n_el * sizeof(double), st));
+    CUDA_TRY(cudaMemsetAsync(d_pw.p, 0, n * sizeof(double), st));
+    CUDA_TRY(cudaMemsetAsync(d_pv.p, 0, n * sizeof(double), st));
+    for (int64_t j = n_seg - 1; j >= 0; --j) {
+      const int64_t ts = ti0 + j * c, te = std::min(ts + c, n_t);
+      if (keep_all) {
+        g.u = d_all.p + (size_t)(ts - ti0) * sb;        // slot k: u_{ts + k - 2}
+      } else {
+        CUDA_TRY(cudaMemcpyAsync(S(0), d_ck.p + 2 * sb * j, 2 * sb, cudaMemcpyDeviceToDevice, st));
+        if (use_chip) {
+          if (!chip_march(of, af, ts, 1, te - ts, false, S(1), S(0), S(2))) return kNotLaunched;
+        } else for (int64_t t = ts; t < te; ++t) {
+          af.ti = t;
+          af.u_prev = S(t - ts);
+          af.u_n = S(t - ts + 1);
+          af.u_new = S(t - ts + 2);
+          if (int r = step(af)) return r;
+        }
+      }
+      if (use_chip) {
+        if (!chip_march(oa, aa, te - 1, -1, te - ts, false, Lm(te - ts), Lm(te - ts + 1), Lm(te - 1 - ts)))
+          return kNotLaunched;
+      } else for (int64_t t = te - 1; t >= ts; --t) {
+        aa.ti = t;
+        aa.u_prev = Lm(t - ts + 2);
+        aa.u_n = Lm(t - ts + 1);
+        aa.u_new = Lm(t - ts);
+        if (int r = step(aa)) return r;
+      }
+      g.n_steps = (int)(te - ts);
+      const cudaError_t e = bfe::launch_grad(g, prec, st);
+      if (e != cudaSuccess) return fail(BFE_ERR_CUDA, "gradient kernel launch failed: %s", cudaGetErrorString(e));
+      if (j > 0) {
+        // lam_ts, lam_{ts+1} start the previous segment (slots c, c + 1);
+        // slot 1 moves first so that c = 1 never overwrites an unread slot
+        CUDA_TRY(cudaMemcpyAsync(Lm(c + 1), Lm(1), sb, cudaMemcpyDeviceToDevice, st));
+        CUDA_TRY(cudaMemcpyAsync(Lm(c), Lm(0), sb, cudaMemcpyDeviceToDevice, st));
       }
     }
-    for (int64_t t = te - 1; t >= ts; --t) {
-      aa.ti = t;
-      aa.u_prev = Lm(t - ts + 2);
-      aa.u_n = Lm(t - ts + 1);
-      aa.u_new = Lm(t - ts);
-      if ((rc = step(aa))) return rc;
+    {
+      const cudaError_t e = bfe::launch_grad_rho(g, prec, st);
+      if (e != cudaSuccess) return fail(BFE_ERR_CUDA, "gradient kernel launch failed: %s", cudaGetErrorString(e));
     }
-    g.n_steps = (int)(te - ts);
-    const cudaError_t e = bfe::launch_grad(g, prec, st);
-    if (e != cudaSuccess) return fail(BFE_ERR_CUDA, "gradient kernel launch failed: %s", cudaGetErrorString(e));
-    if (j > 0) {
-      // lam_ts, lam_{ts+1} start the previous segment (slots c, c + 1);
-      // slot 1 moves first so that c = 1 never overwrites an unread slot
-      CUDA_TRY(cudaMemcpyAsync(Lm(c + 1), Lm(1), sb, cudaMemcpyDeviceToDevice, st));
-      CUDA_TRY(cudaMemcpyAsync(Lm(c), Lm(0), sb, cudaMemcpyDeviceToDevice, st));
-    }
+    return BFE_OK;
+  };
+  chip = chip && onchip_multi_fit(pl, aa, rows_of(afrc), {}, false, st, oa);
+  rc = sweep(chip);
+  if (rc == kNotLaunched) rc = sweep(chip = false);
+  if (rc) return rc;
+  if (chip) {
+    CUDA_TRY(cudaStreamSynchronize(st));
+    bool yes = false;
+    if ((rc = gave_up(yes))) return rc;
+    if (yes && (rc = sweep(false))) return rc;
   }
-  {
-    const cudaError_t e = bfe::launch_grad_rho(g, prec, st);
-    if (e != cudaSuccess) return fail(BFE_ERR_CUDA, "gradient kernel launch failed: %s", cudaGetErrorString(e));
-  }
+  stt.step_launches = launches;
   CUDA_TRY(cudaMemcpyAsync(g_stiff, d_gs.p, n_el * sizeof(double), cudaMemcpyDeviceToHost, st));
   CUDA_TRY(cudaMemcpyAsync(g_rho, d_gr.p, n_el * sizeof(double), cudaMemcpyDeviceToHost, st));
   CUDA_TRY(cudaStreamSynchronize(st));

@@ -138,6 +138,8 @@ struct Onchip {
   DevBuf<int32_t> d_part, d_off, d_word, d_bytes, d_cnt, d_halo, d_vptr, d_vhalo;
   DevBuf<uint16_t> flags, order, z_lcol;
   DevBuf<unsigned char> blocks, xch, xchv;
+  DevBuf<uint4> xchm;               // exchange words of marches with several sources
+  std::vector<int32_t> halo_cnt;
   DevBuf<ushort4> lref;
 };
 
@@ -251,6 +253,15 @@ int execute(bfe_plan* pl, RunSpec& rs, cudaStream_t st);
 int onchip_prepare(bfe_plan* pl, cudaStream_t st);
 bool onchip_fit(bfe_plan* pl, const std::vector<ForceEntry>& frc, const std::vector<int64_t>& v5_bytes,
                 const std::vector<int32_t>& v5_count, bfe::OnchipArgs& o);
+// Shared memory, threads and exchange buffer of a march with several sources
+// (a: its forcing, monitors and padded R). false: it does not fit, or the step
+// kernels (against_graph: replayed from a graph) are faster.
+bool onchip_multi_fit(bfe_plan* pl, const bfe::StepArgs& a, const std::vector<int32_t>& frc_rows,
+                      const std::vector<int32_t>& mon_rows, bool against_graph, cudaStream_t st, bfe::OnchipArgs& o);
+// Whether that is worth building the partition for.
+bool onchip_multi_may_fit(const bfe_plan* pl, int64_t R);
+// Step numbers for n steps that the exchange buffers do not hold yet.
+int onchip_tags(bfe_plan* pl, int64_t n, cudaStream_t st, uint32_t& tag0);
 // Device data of a run's prescribed displacements for the on-chip march, and
 // what each part needs for them; fits = false: they do not fit the form.
 struct OnchipV5 {

@@ -245,6 +245,21 @@ struct V5Args;
 cudaError_t launch_onchip(const OnchipArgs& o, const StepArgs& a, const V5Args& v, int precision, int64_t ti0, int64_t n_steps,
                           int fresh, cudaStream_t s);
 
+// March of several sources on the chip (bfe_onchip_multi.cu): the states of
+// a.R right-hand sides and the whole operator in shared memory. o.xch holds
+// 16-byte words here, o.x_stride of them per buffer.
+struct OnchipMulti {
+  int64_t ti0;                      // time index of the first step, and from step to step (+1, -1)
+  int64_t ti_step;
+  void* out;                        // every new state: out + k out_stride values (nullptr: none)
+  int64_t out_stride;
+  uint32_t wpr_magic;               // set by the launcher
+};
+int onchip_multi_rv(int precision); // right-hand sides per thread; a.R is a multiple of it
+// As launch_onchip; with a.u_new == nullptr the states are not written back.
+cudaError_t launch_onchip_multi(const OnchipArgs& o, const StepArgs& a, const OnchipMulti& m, int precision,
+                                int64_t n_steps, int fresh, cudaStream_t s);
+
 // Prescribed displacements of the v5 scheme (fn_explicit_dynamic_solver_v5.m
 // :142-188). The main step kernel advances every row with the velocity
 // u_n - u_{n-1}; the v5 kernel then handles the rows that differ from that:

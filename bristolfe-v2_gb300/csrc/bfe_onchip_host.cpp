@@ -231,6 +231,7 @@ int onchip_prepare(bfe_plan* pl, cudaStream_t st) {
     return BFE_OK;
   }
   oc.op_bytes = obytes;
+  oc.halo_cnt = cnt;
   bfe::OnchipArgs& o = oc.args;
   o.n_parts = (int32_t)P;
   // a warp per slice where that is enough, else as many warps as give each the
@@ -365,6 +366,78 @@ int onchip_v5(bfe_plan* pl, const V5Lists& L, OnchipV5& d, bool& fits) {
   CUDA_TRY(d.c.upload(c));
   CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
   fits = true;
+  return BFE_OK;
+}
+
+bool onchip_multi_may_fit(const bfe_plan* pl, int64_t R) {
+  if (pl->n_int || R < 2 || R > 64 || R % bfe::onchip_multi_rv(pl->prec)) return false;
+  // the states alone must fit in the SMs' shared memory
+  return 2 * (double)pl->n * (double)R * (double)elem_size(pl->prec) <= (double)kSmemLimit * bfe::sm_count();
+}
+
+bool onchip_multi_fit(bfe_plan* pl, const bfe::StepArgs& a, const std::vector<int32_t>& frc_rows,
+                      const std::vector<int32_t>& mon_rows, bool against_graph, cudaStream_t st, bfe::OnchipArgs& o) {
+  Onchip& oc = *pl->onchip;
+  o = oc.args;
+  const int P = o.n_parts;
+  const int64_t R = a.R, es = (int64_t)elem_size(pl->prec), rv = bfe::onchip_multi_rv(pl->prec);
+  if (!onchip_multi_may_fit(pl, R)) return false;
+  int64_t smem = 0, tasks = 0, words = 0;
+  const int64_t wpr = pl->prec == BFE_PREC_DOUBLE ? R : R / 2;
+  auto in_part = [&](const std::vector<int32_t>& v, int p) {
+    return std::lower_bound(v.begin(), v.end(), oc.part_slice[p + 1] * bfe::kSlice) -
+           std::lower_bound(v.begin(), v.end(), oc.part_slice[p] * bfe::kSlice);
+  };
+  for (int p = 0; p < P; ++p) {
+    const int64_t ns = oc.part_slice[p + 1] - oc.part_slice[p], rp = ns * bfe::kSlice, H = oc.halo_cnt[p];
+    const int64_t nf = in_part(frc_rows, p), nm = in_part(mon_rows, p);
+    const int64_t W = (rp + H + 2) | 1;
+    const int64_t need = 2 * R * W * es + 3 * align2(nf) * es + ns * 8 + (2 * nf + 2 * nm + H) * 4 + rp * 2 + 16 +
+                         oc.op_bytes[p];
+    if (need > kSmemLimit || nf > 1024) return false;
+    smem = std::max(smem, need);
+    tasks = std::max(tasks, ns * (R / rv));
+    words = std::max(words, H * wpr);
+  }
+  // Against step kernels replayed from a graph (about 8 us per step for small
+  // models) the exchange decides, about 2 us per 1,000 words of a part. us per
+  // step on chip / graph: plate of 40,602 DOF FP32 R = 4 3.3 / 8.1 (808
+  // words), R = 16 9.3 / 9.1 (3,232), R = 32 14.1 / 9.9; 10,302 DOF R = 16 5.3
+  // / 8.8, R = 32 8.0 / 9.1 (3,264); bricks of 46,128 DOF R = 4 8.0 / 11.7. In
+  // FP64 the multiply-adds weigh as much: 40,602 DOF R = 4 6.6 / 10.0, R = 8
+  // 12.2 / 13.9; 1,722 DOF R = 16 9.6 / 8.2. One launch per step, which the
+  // adjoint would make, is slower wherever this fits up to R = 16 (17 us per
+  // step of 90,902 DOF, R = 16, against 13).
+  if (against_graph ? !(R <= (es == 8 ? 4 : 8) || (words <= 3300 && R <= (es == 8 ? 8 : 64))) : R > 16) return false;
+  const int64_t turns = (tasks + 31) / 32, warps = (tasks + turns - 1) / turns;
+  o.threads = (int32_t)std::max<int64_t>({128, warps * 32, std::min<int64_t>(1024, (words / 4 + 31) / 32 * 32)});
+  for (int p = 0; p < P; ++p)
+    if (in_part(frc_rows, p) > o.threads) o.threads = 1024;
+  o.smem = (int32_t)((smem + 15) & ~(int64_t)15);
+  const size_t need_words = (size_t)pl->n * wpr * 2;
+  if (oc.xchm.n < need_words) {
+    if (oc.xchm.alloc(need_words) != cudaSuccess ||
+        cudaMemsetAsync(oc.xchm.p, 0, need_words * sizeof(uint4), st) != cudaSuccess) {
+      cudaGetLastError();
+      oc.xchm.alloc(0);
+      return false;
+    }
+  }
+  o.xch = oc.xchm.p;
+  o.x_stride = (int64_t)pl->n * wpr;
+  return true;
+}
+
+int onchip_tags(bfe_plan* pl, int64_t n, cudaStream_t st, uint32_t& tag0) {
+  Onchip& oc = *pl->onchip;
+  if ((uint64_t)oc.next_tag + (uint64_t)n + 2 > 0xffffffffull) {
+    CUDA_TRY(cudaMemsetAsync(oc.xch.p, 0, oc.xch.n, st));
+    if (oc.xchv.n) CUDA_TRY(cudaMemsetAsync(oc.xchv.p, 0, oc.xchv.n, st));
+    if (oc.xchm.n) CUDA_TRY(cudaMemsetAsync(oc.xchm.p, 0, oc.xchm.n * sizeof(uint4), st));
+    oc.next_tag = 1;
+  }
+  tag0 = oc.next_tag;
+  oc.next_tag += (uint32_t)n + 2;
   return BFE_OK;
 }
 

@@ -162,6 +162,63 @@ constexpr int64_t kOnchipMinSteps = 96, kOnchipLaunchSteps = 8192;
 // Device memory for raw frames that an element field is reduced from.
 constexpr int64_t kRawFrameBytes = (int64_t)1 << 31;
 
+// The same for several sources (bfe_onchip_multi.cu).
+int march_on_chip_multi(bfe_plan* pl, RunSpec& rs, bfe::StepArgs a, unsigned char* const U[3], cudaStream_t st,
+                        bool& done) {
+  done = false;
+  const int64_t steps = rs.n_t - rs.ti_start;
+  if (pl->timing || pl->time_limit_s > 0.0 || steps < kOnchipMinSteps || rs.n_t >= ((int64_t)1 << 30) || pl->n_int ||
+      getenv("BFE_NO_GRAPH") || getenv("BFE_VARIANT"))
+    return BFE_OK;
+  if (!onchip_multi_may_fit(pl, a.R)) return BFE_OK;
+  if (onchip_prepare(pl, st)) {
+    if (pl->onchip->state == 0) pl->onchip->state = -1;
+    cudaGetLastError();
+    g_last_error.clear();
+    return BFE_OK;
+  }
+  if (pl->onchip->state != 1) return BFE_OK;
+  std::vector<int32_t> frows, mrows;
+  for (auto& f : rs.frc) frows.push_back(f.row);
+  for (int64_t h : rs.hist_idx)
+    if (h >= 0) mrows.push_back((int32_t)h);
+  std::sort(frows.begin(), frows.end());
+  std::sort(mrows.begin(), mrows.end());
+  bfe::OnchipArgs o;
+  if (!onchip_multi_fit(pl, a, frows, mrows, true, st, o)) return BFE_OK;
+  o.err = pl->d_flag.p + 1;
+  int prev = 2, cur = 0, next = 1;
+  for (int64_t ti = rs.ti_start; ti < rs.n_t; ti += kOnchipLaunchSteps) {
+    const int64_t k = std::min(kOnchipLaunchSteps, rs.n_t - ti);
+    int rc;
+    if ((rc = onchip_tags(pl, k, st, o.tag0))) return rc;
+    a.u_prev = U[prev];
+    a.u_n = U[cur];
+    a.u_new = U[next];
+    bfe::OnchipMulti m{};
+    m.ti0 = ti;
+    m.ti_step = 1;
+    if (bfe::launch_onchip_multi(o, a, m, pl->prec, k, ti == rs.ti_start, st) != cudaSuccess) {
+      cudaGetLastError();
+      CUDA_TRY(cudaStreamSynchronize(st));
+      return BFE_OK;
+    }
+    pl->last.step_launches++;
+    std::swap(cur, next);
+  }
+  int gave_up = 0;
+  CUDA_TRY(cudaMemcpyAsync(&gave_up, o.err, sizeof(int), cudaMemcpyDeviceToHost, st));
+  CUDA_TRY(cudaStreamSynchronize(st));
+  if (gave_up) {
+    pl->onchip->state = -1;
+    return BFE_OK;
+  }
+  if (cur != 1)
+    CUDA_TRY(cudaMemcpyAsync(U[1], U[cur], (size_t)pl->n * a.R * elem_size(pl->prec), cudaMemcpyDeviceToDevice, st));
+  done = true;
+  return BFE_OK;
+}
+
 // The whole march in kernels that stay on the chip; done says whether it ran.
 // On return U[1] holds the newest state. Any reason not to run it leaves the
 // march to the step kernels.
@@ -216,15 +273,8 @@ int march_on_chip(bfe_plan* pl, RunSpec& rs, bfe::StepArgs a, unsigned char* con
     a.fld_is_vel = rs.field_is_vel;
     a.dt = pl->dt;
   }
-  // step numbers of this run: none that the exchange buffers still hold
-  Onchip& oc = *pl->onchip;
-  if ((uint64_t)oc.next_tag + (uint64_t)rs.n_t + 2 > 0xffffffffull) {
-    CUDA_TRY(cudaMemsetAsync(oc.xch.p, 0, oc.xch.n, st));
-    if (oc.xchv.n) CUDA_TRY(cudaMemsetAsync(oc.xchv.p, 0, oc.xchv.n, st));
-    oc.next_tag = 1;
-  }
-  o.tag0 = oc.next_tag;
-  oc.next_tag += (uint32_t)rs.n_t + 2;
+  int rct;
+  if ((rct = onchip_tags(pl, rs.n_t, st, o.tag0))) return rct;
   o.err = pl->d_flag.p + 1;
   int prev = 2, cur = 0, next = 1;
   for (int64_t ti = rs.ti_start; ti < rs.n_t; ti += kOnchipLaunchSteps) {
@@ -318,9 +368,17 @@ int execute(bfe_plan* pl, RunSpec& rs, cudaStream_t st) {
   auto launch_batched = [&](const bfe::GroupArgs* grpp, int v) -> cudaError_t {
     return bfe::launch_step_batched(a, grpp, prec, pl->max_slice_entries, v, st);
   };
+  if (!pl->d_flag.p) CUDA_TRY(pl->d_flag.alloc(2));
+  CUDA_TRY(cudaMemsetAsync(pl->d_flag.p, 0, 2 * sizeof(int), st));
+  bool on_chip = false;
+  if (R > 1) {
+    const int rc1 = march_on_chip_multi(pl, rs, a, U, st, on_chip);
+    if (rc1) return rc1;
+    if (!on_chip) CUDA_TRY(cudaMemsetAsync(pl->d_flag.p, 0, 2 * sizeof(int), st));
+  }
   int variant = 0;
   const bfe::GroupArgs* grp = pl->have_groups ? &pl->groups : nullptr;
-  if (R > 1) {
+  if (R > 1 && !on_chip) {
     CUDA_TRY(cudaMemsetAsync(d_u.p, 0, 3 * state_bytes, st));
     int cand[8];
     const int max_bs = grp ? bfe::group_max_bs(*grp) : 0;
@@ -392,13 +450,10 @@ int execute(bfe_plan* pl, RunSpec& rs, cudaStream_t st) {
   if (frames && rs.fld_time)
     for (int64_t k = 0; k * rs.every_n < rs.n_t; ++k)
       if (k * rs.every_n >= rs.ti_start) (*rs.fld_time)[k] = rs.time[k * rs.every_n];
-  if (!pl->d_flag.p) CUDA_TRY(pl->d_flag.alloc(2));
-  CUDA_TRY(cudaMemsetAsync(pl->d_flag.p, 0, 2 * sizeof(int), st));
   // One source whose state fits on the chip: all steps in one kernel
   // (bfe_onchip.cu), unless launches are timed one by one, a time limit wants
   // the host between chunks, or the run is too short to pay for the setup.
   // Element fields are reduced afterwards from raw frames kept on the device.
-  bool on_chip = false;
   if (R == 1) {
     DevBuf<double> d_raw;
     const int rc1 = march_on_chip(pl, rs, a, U, frames, st, d_raw, on_chip);

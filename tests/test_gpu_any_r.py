@@ -44,7 +44,6 @@ def test_every_source_matches_its_own_run(bfe, models, name, prec, tol, R):
     F = np.stack([(1.0 + 0.1 * r) * s[None, :] for r in range(R)], axis=2)
     with bfe.Plan(m["K"], m["C"], m["M"], m["dt"], bfe.VEL_CURRENT, prec, m["gl"]) as plan:
         h = plan.run_batched(t, srcs, F, hi)
-        assert plan.stats()["variant"] != 0 or prec == "double"
         assert h.shape == (hi.size, t.size, R)
         for r in {0, R // 2, R - 1}:
             h1, _, _ = plan.run(t, srcs[r], F[:, :, r], hi)

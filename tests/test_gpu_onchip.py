@@ -141,3 +141,30 @@ def test_v5_prescribed_displacements(bfe, models, name, cut, prec, monkeypatch):
     on, off = _both(bfe, monkeypatch, run)
     for a, b in zip(on, off):
         assert np.abs(b).max() > 0 and np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("prec", ["double", "single"])
+@pytest.mark.parametrize("R", [2, 3, 8, 15])
+@pytest.mark.parametrize("name", ["one_slice", "ragged", "dof3", "plate", "brick"])
+def test_several_sources(bfe, models, name, R, prec, monkeypatch):
+    """Several sources on chip against the group kernels, bit for bit: two
+    forced DOFs per source, one of them shared by all, repeated monitors."""
+    m, dof = models[name]
+    if prec == "double" or name == "brick":               # more take the step kernels
+        R = min(R, 7 if name != "brick" or prec == "single" else 4)
+    t, s = modelgen.pulse(140, m["dt"])
+    n = m["K"].shape[0]
+    nodes = np.nonzero(m["gl"][:, dof - 1] > 0)[0] + 1
+    both = modelgen.gi_of(m["gl"], [m["frc_nd"]], dof)
+    srcs = [np.concatenate([both, modelgen.gi_of(m["gl"], [nodes[(5 * r + 1) % nodes.size]], dof)]) for r in range(R)]
+    F = np.stack([np.vstack([s, -0.3 * s]) * (1 + r) for r in range(R)], axis=2)
+    hi = np.concatenate([modelgen.gi_of(m["gl"], m["mon_nds"], dof), [1, n, n]])
+
+    def run():
+        with bfe.Plan(m["K"], m["C"], m["M"], m["dt"], bfe.VEL_CURRENT, prec, m["gl"]) as plan:
+            h = [plan.run_batched(t, srcs, F[:, :, :] * k, hi) for k in (1.0, 2.0)]
+            return h, plan.stats()["step_launches"]
+
+    on, off = _both(bfe, monkeypatch, run)
+    for a, b in zip(on, off):
+        assert np.abs(b).max() > 0 and np.array_equal(a, b)
