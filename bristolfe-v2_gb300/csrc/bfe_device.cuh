@@ -49,6 +49,42 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
   e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
 }
 
+// Asks L2 for [p, p + bytes), cut to 16-byte boundaries and to the end of the
+// array: one bulk instruction of one thread.
+__device__ __forceinline__ void prefetch_l2(const void* p, size_t bytes, const void* end) {
+  const uintptr_t b = reinterpret_cast<uintptr_t>(p) & ~uintptr_t(15);
+  const uintptr_t lim = reinterpret_cast<uintptr_t>(end);
+  uintptr_t e = reinterpret_cast<uintptr_t>(p) + bytes;
+  e = (e < lim ? e : lim) & ~uintptr_t(15);
+  if (e > b) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(b), "r"((uint32_t)(e - b)) : "memory");
+}
+
+// One thread of a group kernel's CTA, whose first node is `node` of npc:
+// requests to L2 for what the CTA will read last (its rows of u_{n-1}) and for
+// what the CTA gr.ahead further on will read first (its rows of u_n, its
+// neighbour lists and blocks). A node's loads are a chain, record -> neighbour
+// row -> state, in which each DRAM miss costs about a microsecond; with the
+// requests made early they are L2 hits. Rows and blocks of a group follow the
+// order of its nodes, so the place of the later CTA's is estimated from this
+// one's: a request that misses its aim only costs its bytes.
+__device__ __forceinline__ void prefetch_group(const StepArgs& a, const GroupArgs& gr, int gi, int node, int npc) {
+  const int4 rec = __ldg(gr.rec[gi] + node);
+  const int bs = gr.bs[gi], dn = gr.ahead * npc;
+  const size_t R = (size_t)a.R, state = (size_t)a.n * R, bytes = (size_t)(npc * bs) * R * sizeof(float);
+  const float* up = static_cast<const float*>(a.u_prev);
+  const float* un = static_cast<const float*>(a.u_n);
+  prefetch_l2(up + (size_t)rec.x * R, bytes, up + state);
+  const int64_t row = (int64_t)rec.x + (int64_t)dn * bs;
+  if (row < a.n) prefetch_l2(un + (size_t)row * R, bytes, un + state);
+  if (node + dn >= gr.n_nodes[gi]) return;
+  const size_t e = (size_t)rec.y + (size_t)rec.z * dn, n_blk = (size_t)__ldg(gr.nptr[gi] + gr.n_nodes[gi]);
+  if (e >= n_blk) return;
+  const size_t cnt = (size_t)rec.z * npc, bb = (size_t)(bs * bs);
+  prefetch_l2(gr.coef[gi] + e * bb, cnt * bb * sizeof(float), gr.coef[gi] + n_blk * bb);
+  prefetch_l2(gr.nrow[gi] + e, cnt * sizeof(int32_t), gr.nrow[gi] + n_blk);
+  prefetch_l2(gr.rec[gi] + node + dn, npc * sizeof(int4), gr.rec[gi] + gr.n_nodes[gi]);
+}
+
 // Packed FP32x2 forms (__ffma2_rn / __fadd2_rn: IEEE round-to-nearest per
 // component, the same results as two scalar operations).
 __device__ __forceinline__ float2 f2sub(float2 a, float2 b) {        // a - b, exact rounding

@@ -4,6 +4,7 @@
 // batched variant.
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <type_traits>
 
 #include "bfe_device.cuh"
 #include "bfe_internal.h"
@@ -170,10 +171,12 @@ __device__ __forceinline__ void group4_node(const StepArgs& a, const GroupArgs& 
   }
 }
 
+// AHEAD: with the L2 requests of prefetch_group (a form of its own: as a test
+// at run time they cost 0.5 % of a march that does not use them).
 // 128 threads = 128 / LPN nodes of LPN lanes each (LPN = 16 for R a
 // multiple of 64, 8 for R = 32, 4 for R = 16); gr.blk_begin must hold the
 // CTA ranges for 128 / LPN nodes per CTA.
-template <int MINB, int LPN = 16>
+template <int MINB, int LPN, bool AHEAD>
 __global__ void __launch_bounds__(128, MINB) step_f32_group4(StepArgs a, GroupArgs gr) {
   const int b = blockIdx.x;
   int gi = 0;
@@ -183,11 +186,13 @@ __global__ void __launch_bounds__(128, MINB) step_f32_group4(StepArgs a, GroupAr
   if (LPN == 16 && gr.bs[gi] == 1) {                    // one-DOF nodes: 8 lanes, 16 nodes per CTA
     const int node = (b - gr.blk_begin[gi]) * 16 + (threadIdx.x >> 3);
     if (node >= gr.n_nodes[gi]) return;
+    if (AHEAD && threadIdx.x == 0) prefetch_group(a, gr, gi, node, 16);
     group4_fluid(a, gr, gi, node, threadIdx.x & 7);
     return;
   }
   const int node = (b - gr.blk_begin[gi]) * (128 / LPN) + threadIdx.x / LPN;
   if (node >= gr.n_nodes[gi]) return;
+  if (AHEAD && threadIdx.x == 0) prefetch_group(a, gr, gi, node, 128 / LPN);
   if (gr.bs[gi] == 1) group4_node<1, 2>(a, gr, gi, node, threadIdx.x % LPN * 4, 4 * LPN);
   else group4_node<2, 1>(a, gr, gi, node, threadIdx.x % LPN * 4, 4 * LPN);
 }
@@ -196,7 +201,7 @@ __global__ void __launch_bounds__(128, MINB) step_f32_group4(StepArgs a, GroupAr
 // gr.lpn lanes per node, any number up to 32, so no lane is idle but the few
 // that 128 / lpn leaves over. A ragged R used to take the slice kernel, whose
 // warps put 32 lanes on a row whatever R is.
-template <int MAXBS, int MINB, int UNROLL>
+template <int MAXBS, int MINB, int UNROLL, bool AHEAD>
 __global__ void __launch_bounds__(128, MINB) step_f32_groupn(StepArgs a, GroupArgs gr) {
   const int b = blockIdx.x;
   int gi = 0;
@@ -206,6 +211,7 @@ __global__ void __launch_bounds__(128, MINB) step_f32_groupn(StepArgs a, GroupAr
   const int npc = 128 / gr.lpn, ln = threadIdx.x / gr.lpn;
   const int node = (b - gr.blk_begin[gi]) * npc + ln;
   if (ln >= npc || node >= gr.n_nodes[gi]) return;
+  if (AHEAD && threadIdx.x == 0) prefetch_group(a, gr, gi, node, npc);
   const int c0 = (threadIdx.x - ln * gr.lpn) * 4, stride = 4 * gr.lpn;
   if (gr.bs[gi] == 1) group4_node<1, UNROLL>(a, gr, gi, node, c0, stride);
   else if (MAXBS == 2 || gr.bs[gi] == 2) group4_node<2, UNROLL>(a, gr, gi, node, c0, stride);
@@ -224,8 +230,14 @@ static void launch_group4(const StepArgs& a, const GroupArgs& gr, int variant, c
     blocks += (g.n_nodes[k] + npc - 1) / npc;
   }
   g.blk_begin[g.n_groups] = blocks;
-  if (variant == 22) step_f32_group4<10, LPN><<<blocks, 128, 0, st>>>(a, g);
-  else step_f32_group4<12, LPN><<<blocks, 128, 0, st>>>(a, g);
+  g.ahead = group_ahead(a, g);
+  auto go = [&](auto ahead) {
+    constexpr bool A = decltype(ahead)::value;
+    if (variant == 22) step_f32_group4<10, LPN, A><<<blocks, 128, 0, st>>>(a, g);
+    else step_f32_group4<12, LPN, A><<<blocks, 128, 0, st>>>(a, g);
+  };
+  if (g.ahead) go(std::true_type());
+  else go(std::false_type());
 }
 
 cudaError_t launch_group4_variant(int lpn, const StepArgs& a, const GroupArgs& gr, int variant, cudaStream_t st) {
@@ -247,15 +259,21 @@ cudaError_t launch_groupn_variant(int maxbs, const StepArgs& a, const GroupArgs&
     blocks += (g.n_nodes[k] + npc - 1) / npc;
   }
   g.blk_begin[g.n_groups] = blocks;
-  if (maxbs <= 2) {
-    if (variant == 24) step_f32_groupn<2, 12, 1><<<blocks, 128, 0, st>>>(a, g);
-    else if (variant == 25) step_f32_groupn<2, 8, 2><<<blocks, 128, 0, st>>>(a, g);
-    else step_f32_groupn<2, 5, 4><<<blocks, 128, 0, st>>>(a, g);
-  } else {
-    if (variant == 24) step_f32_groupn<3, 8, 1><<<blocks, 128, 0, st>>>(a, g);
-    else if (variant == 25) step_f32_groupn<3, 6, 1><<<blocks, 128, 0, st>>>(a, g);
-    else step_f32_groupn<3, 4, 2><<<blocks, 128, 0, st>>>(a, g);
-  }
+  g.ahead = group_ahead(a, g);
+  auto go = [&](auto ahead) {
+    constexpr bool A = decltype(ahead)::value;
+    if (maxbs <= 2) {
+      if (variant == 24) step_f32_groupn<2, 12, 1, A><<<blocks, 128, 0, st>>>(a, g);
+      else if (variant == 25) step_f32_groupn<2, 8, 2, A><<<blocks, 128, 0, st>>>(a, g);
+      else step_f32_groupn<2, 5, 4, A><<<blocks, 128, 0, st>>>(a, g);
+    } else {
+      if (variant == 24) step_f32_groupn<3, 8, 1, A><<<blocks, 128, 0, st>>>(a, g);
+      else if (variant == 25) step_f32_groupn<3, 6, 1, A><<<blocks, 128, 0, st>>>(a, g);
+      else step_f32_groupn<3, 4, 2, A><<<blocks, 128, 0, st>>>(a, g);
+    }
+  };
+  if (g.ahead) go(std::true_type());
+  else go(std::false_type());
   return cudaGetLastError();
 }
 

@@ -112,6 +112,7 @@ struct GroupArgs {
   const float2* coef2[kMaxGroups];   // the coefficients as broadcast pairs {c, c}
   const int4* rec[kMaxGroups];       // per node {first row, first neighbour block, neighbour count, 0}
   int32_t lpn;                       // lanes per node of the any-R kernels
+  int32_t ahead;                     // CTAs whose data a CTA asks L2 for (0 = none)
   const double* coef64[kMaxGroups];  // FP64 plans: B per block (own block included), [own k][l]
 };
 
@@ -126,6 +127,8 @@ inline int padded_sources(int precision, int64_t R, bool have_groups) {
   const int64_t q = R < 2 || !have_groups ? 1 : precision == 0 ? 2 : 4;
   return (int)((R + q - 1) / q * q);
 }
+// CTAs ahead of an FP32 group kernel's own for which it prefetches (0 = none).
+int group_ahead(const StepArgs& a, const GroupArgs& g);
 // Largest node block size (DOFs per node) of a group operator.
 int group_max_bs(const GroupArgs& g);
 cudaError_t launch_step_batched(const StepArgs& a, const GroupArgs* gr, int precision, int max_slice_entries,

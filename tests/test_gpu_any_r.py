@@ -81,3 +81,31 @@ def test_adjoint_of_three_sources_is_the_sum_over_sources(bfe):
     for g, k in ((gs, 1), (gr, 2)):
         ref = sum(o[k] for o in one)
         assert np.abs(g - ref).max() <= 1e-10 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("name,R", [("coupled", 48), ("coupled", 61), ("coupled", 128), ("brick", 61), ("brick", 52)])
+def test_states_beyond_l2(bfe, name, R):
+    """States that exceed L2: the group kernels prefetch the rows and blocks of
+    later CTAs, up to the ends of the arrays. Every source against its own run,
+    to the FP32 bound of the other parity tests."""
+    import torch
+    from bfe_gb300 import model
+    if name == "coupled":
+        m = model.coupled_water_steel(60e-3, 20e-3, 10e-3, 0.1e-3, abs_wavelengths=3.0)
+        dof = 4
+    else:
+        m = model.steel_block_3d(10e-3, 10e-3, 5.6e-3, 0.2e-3, n_mon=4)
+        dof = 3
+    t, s = modelgen.pulse(40, m["dt"])
+    rows = np.nonzero(m["gl"][:, dof - 1] > 0)[0] + 1
+    pick = np.r_[rows[0], rows[-1], rows[np.linspace(1, rows.size - 2, R - 2).astype(int)]]
+    srcs = [modelgen.gi_of(m["gl"], [x], dof) for x in pick]
+    hi = modelgen.gi_of(m["gl"], pick[:4], dof)
+    with bfe.Plan(m["K"], m["C"], m["M"], m["dt"], bfe.VEL_CURRENT, "single", m["gl"]) as plan:
+        assert 12 * plan.n * R > torch.cuda.get_device_properties(0).L2_cache_size
+        h = plan.run_batched(t, srcs, s, hi)
+        for r in (0, 1, 2, R - 1):
+            h1, _, _ = plan.run(t, srcs[r], s, hi)
+            if r < 3:
+                assert np.abs(h1).max() > 0
+            assert np.abs(h[:, :, r] - h1).max() <= 1e-4 * np.abs(h1).max(), r
