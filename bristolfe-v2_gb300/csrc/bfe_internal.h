@@ -258,7 +258,11 @@ struct OnchipMulti {
   int64_t out_stride;
   uint32_t wpr_magic;               // set by the launcher
 };
-int onchip_multi_rv(int precision); // right-hand sides per thread; a.R is a multiple of it
+// Right-hand sides per thread; a.R is a multiple of it.
+int onchip_multi_rv(int precision);
+// Elements of a state plane of a window of so many rows: planes start on 16
+// bytes, and those of one row fall on different banks.
+__host__ __device__ inline int onchip_multi_window(int rows) { return rows + 2 + (-rows & 3); }
 // As launch_onchip; with a.u_new == nullptr the states are not written back.
 cudaError_t launch_onchip_multi(const OnchipArgs& o, const StepArgs& a, const OnchipMulti& m, int precision,
                                 int64_t n_steps, int fresh, cudaStream_t s);

@@ -391,7 +391,7 @@ bool onchip_multi_fit(bfe_plan* pl, const bfe::StepArgs& a, const std::vector<in
   for (int p = 0; p < P; ++p) {
     const int64_t ns = oc.part_slice[p + 1] - oc.part_slice[p], rp = ns * bfe::kSlice, H = oc.halo_cnt[p];
     const int64_t nf = in_part(frc_rows, p), nm = in_part(mon_rows, p);
-    const int64_t W = (rp + H + 2) | 1;
+    const int64_t W = bfe::onchip_multi_window((int)(rp + H));
     const int64_t need = 2 * R * W * es + 3 * align2(nf) * es + ns * 8 + (2 * nf + 2 * nm + H) * 4 + rp * 2 + 16 +
                          oc.op_bytes[p];
     if (need > kSmemLimit || nf > 1024) return false;

@@ -30,6 +30,7 @@ template <typename T> struct Elem;
 template <> struct Elem<float> { using E = float2; static constexpr int kPer = 2; };
 template <> struct Elem<double> { using E = double; static constexpr int kPer = 1; };
 constexpr int kRe = 2;                                  // elements per thread
+constexpr int kSlPaired = kSlResident;                  // (all slices are resident here)
 
 __device__ __forceinline__ float2 e_sub(float2 a, float2 b) { return f2sub(a, b); }
 __device__ __forceinline__ float2 e_fma(float c, float2 x, float2 acc) {
@@ -110,6 +111,38 @@ __device__ __forceinline__ void row_sums(double (&acc)[kRe], const unsigned char
     }
   }
 }
+// Slices whose nodes all start at an even place of the window: both DOFs of a
+// neighbour (kind 2) come with one 16-byte load. Shared-memory reads bound the
+// rows (two lanes of a node read the same words, so 16 distinct ones per load
+// either way): 6.5 instead of 10.5 wavefronts a neighbour, 90,902 DOF R = 16
+// 16,000 -> 13,700 clocks of rows per step. Eight right-hand sides per lane in
+// place of four: no faster at R = 16 (12.3 us per step both), slower at R = 8
+// (6.7 / 5.7).
+__device__ __forceinline__ void row_sums_paired(float2 (&acc)[kRe], const unsigned char* blk, int lane, int u,
+                                                const unsigned char* sm, uint32_t au, uint32_t ws,
+                                                const float2 (&ref)[3][kRe]) {
+  const float2* v = reinterpret_cast<const float2*>(blk) + lane;
+  const uint32_t* c = reinterpret_cast<const uint32_t*>(blk + u * 256) + lane;
+#pragma unroll 4
+  for (int k = 0; k < u; ++k) {
+    const uint32_t cc = c[32 * (k >> 1)], c0 = au + 2 * (k & 1 ? cc >> 16 : cc & 0xffffu);
+    const float2 x = v[32 * k];
+#pragma unroll
+    for (int r = 0; r < kRe; ++r) {
+      const float4 n = sm_at<float4>(sm, c0 + r * ws);
+      acc[r] = e_fma(x.x, e_sub(make_float2(n.x, n.y), ref[0][r]), acc[r]);
+      acc[r] = e_fma(x.y, e_sub(make_float2(n.z, n.w), ref[1][r]), acc[r]);
+    }
+  }
+}
+__device__ __forceinline__ void row_sums_paired(double (&)[kRe], const unsigned char*, int, int, const unsigned char*,
+                                                uint32_t, uint32_t, const double (&)[3][kRe]) {}
+__device__ __forceinline__ void split4(const float4& n, float2& lo, float2& hi) {
+  lo = make_float2(n.x, n.y);
+  hi = make_float2(n.z, n.w);
+}
+__device__ __forceinline__ void split4(const float4&, double&, double&) {}
+
 __device__ __forceinline__ void row_sums(float2 (&acc)[kRe], const unsigned char* blk, int lane, int kind, int u,
                                          const unsigned char* sm, uint32_t au, uint32_t ws, const float2 (&ref)[3][kRe]) {
   auto add = [&](float x, uint32_t at, const float2 (&rf)[kRe]) {
@@ -173,7 +206,7 @@ __global__ void __launch_bounds__(1024, 1) march_onchip_multi(OnchipArgs o, Step
   const int rows = min(a.n - row0, rpad);
   const int R = a.R, nc = R / RV, wpr = R / PER;        // chunks and exchange words of a row
   const int H = o.halo_cnt[p];
-  const int W = (rpad + H + 2) | 1;
+  const int W = onchip_multi_window(rpad + H);
   const uint32_t ws = (uint32_t)(W * sizeof(E));        // bytes of a plane (of PER right-hand sides)
   const int f0 = lower_bound_i32(a.frc_row, a.n_frc, row0);
   const int nf = lower_bound_i32(a.frc_row, a.n_frc, row0 + rows) - f0;
@@ -218,7 +251,21 @@ __global__ void __launch_bounds__(1024, 1) march_onchip_multi(OnchipArgs o, Step
         const int4* src = reinterpret_cast<const int4*>(static_cast<const unsigned char*>(o.blocks) + (size_t)d.x * 16);
         for (int k = lane; k < bytes / 16; k += 32) reinterpret_cast<int4*>(cache + off)[k] = __ldg(src + k);
         __syncwarp();
-        if (lane == 0) sd[j].x = off;
+        bool paired = sizeof(T) == 4 && sl_kind(d.y) == 2;
+        if (paired) {
+          const int r = (d.y >> kSlLocalShift) * kSlice + lane, un = sl_units<T>(d.y), cu = chunk_units<T>(2);
+          uint32_t odd = (uint32_t)(r - ((fl[r] >> kOcPosShift) & 7)) << 2;
+          for (int k = 0; k < un; k += cu) {
+            const int u = min(cu, un - k);
+            const uint32_t* c = reinterpret_cast<const uint32_t*>(cache + off + coef_bytes<T>() + k / cu * units_bytes<T>(2, cu) + u * 256);
+            for (int h = 0; 2 * h < u; ++h) odd |= c[32 * h + lane] | c[32 * h + lane] >> 16;
+          }
+          paired = __all_sync(0xffffffffu, !(odd & 4u));
+        }
+        if (lane == 0) {
+          sd[j].x = off;
+          if (paired) sd[j].y = d.y | kSlPaired;
+        }
       }
       off += bytes;
     }
@@ -249,6 +296,7 @@ __global__ void __launch_bounds__(1024, 1) march_onchip_multi(OnchipArgs o, Step
   T* out = static_cast<T*>(m.out);
   __syncthreads();
 
+  const uint32_t nc_magic = nc == 1 ? 0u : (uint32_t)((0x100000000ull + nc - 1) / nc);
   uint32_t au = 0, bu = (uint32_t)wpr * ws;             // byte offsets of u_n and of u_{n-1} / u_{n+1}
   bool bad = false;
   for (int64_t k = 0; k <= n_steps; ++k) {
@@ -267,7 +315,7 @@ __global__ void __launch_bounds__(1024, 1) march_onchip_multi(OnchipArgs o, Step
     }
     uint4* xw = k & 1 ? x1 : x0;
     for (int t = warp; t < ns * nc; t += nw) {
-      const int j = t / nc, c = t - j * nc, r0 = c * RV;
+      const int j = nc == 1 ? t : (int)__umulhi((uint32_t)t, nc_magic), c = t - j * nc, r0 = c * RV;
       const int2 d = sd[j];
       const int kind = sizeof(T) == 8 ? 0 : sl_kind(d.y), r = (d.y >> kSlLocalShift) * kSlice + lane;
       const uint32_t ap = au + r0 / PER * ws, at = ap + r * (uint32_t)sizeof(E), bt = at - au + bu;
@@ -279,7 +327,12 @@ __global__ void __launch_bounds__(1024, 1) march_onchip_multi(OnchipArgs o, Step
         ref[0][v] = ui[v];
         e_zero(acc[v]);
       }
-      if (sizeof(T) == 4 && kind != 1) {
+      const bool paired = sizeof(T) == 4 && (d.y & kSlPaired);
+      if (paired) {
+        const uint32_t own = at - 8 * ((f >> kOcPosShift) & 7);
+#pragma unroll
+        for (int v = 0; v < kRe; ++v) split4(sm_at<float4>(sm, own + v * ws), ref[0][v], ref[1][v]);
+      } else if (sizeof(T) == 4 && kind != 1) {
         const int pos = (int)(f >> kOcPosShift) & 7;
         int q0 = r - pos, q1 = q0 + 1, q2 = q0 + 2;
         if (kind == 0 && pos == (int)kOcCut) {
@@ -298,8 +351,12 @@ __global__ void __launch_bounds__(1024, 1) march_onchip_multi(OnchipArgs o, Step
       const T rc = reinterpret_cast<const T*>(blk)[lane];
       blk += coef_bytes<T>();
       const int cu = chunk_units<T>(kind), full = sizeof(T) == 8 ? 2 * cu : cu, step = units_bytes<T>(kind, cu);
-      for (int left = sl_width(d.y); left > 0; left -= full, blk += step)
-        row_sums(acc, blk, lane, kind, min(left, full), sm, ap, ws, ref);
+      if (paired)
+        for (int left = sl_width(d.y); left > 0; left -= full, blk += step)
+          row_sums_paired(acc, blk, lane, min(left, full), sm, ap, ws, ref);
+      else
+        for (int left = sl_width(d.y); left > 0; left -= full, blk += step)
+          row_sums(acc, blk, lane, kind, min(left, full), sm, ap, ws, ref);
       E ft[kRe];
 #pragma unroll
       for (int v = 0; v < kRe; ++v) e_zero(ft[v]);
