@@ -149,12 +149,7 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
   // segment instead of one per step.
   if (!pl->d_flag.p) CUDA_TRY(pl->d_flag.alloc(2));
   CUDA_TRY(cudaMemsetAsync(pl->d_flag.p, 0, 2 * sizeof(int), st));
-  auto rows_of = [](const std::vector<ForceEntry>& f) {
-    std::vector<int32_t> r;
-    for (auto& x : f) r.push_back(x.row);
-    std::sort(r.begin(), r.end());
-    return r;
-  };
+  Onchip* oc = nullptr;
   // steps t, t + dir, ... (count of them) from the states un, up (fresh: from
   // rest), each new state to out + k * dir * sb; false: not launched
   auto chip_march = [&](const bfe::OnchipArgs& oa, bfe::StepArgs a, int64_t t, int64_t dir, int64_t count, bool fresh,
@@ -163,7 +158,7 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
     for (int64_t k = 0; k < count; k += kSteps) {
       const int64_t m_steps = std::min(kSteps, count - k);
       bfe::OnchipArgs o = oa;
-      if (onchip_tags(pl, m_steps, st, o.tag0)) return false;
+      if (onchip_tags(*oc, m_steps, st, o.tag0)) return false;
       o.err = pl->d_flag.p + 1;
       a.u_n = un;
       a.u_prev = up;
@@ -188,22 +183,20 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
     CUDA_TRY(cudaMemcpy(&e, pl->d_flag.p + 1, sizeof(int), cudaMemcpyDeviceToHost));
     yes = e != 0;
     if (yes) {
-      pl->onchip->state = -1;
+      oc->state = -1;
       CUDA_TRY(cudaMemsetAsync(pl->d_flag.p, 0, 2 * sizeof(int), st));
     }
     return BFE_OK;
   };
   bfe::OnchipArgs of, oa;
-  bool chip = onchip_multi_may_fit(pl, Rp) && Rp <= 16 && c >= 8 && !pl->timing && !getenv("BFE_NO_GRAPH") && n_t < ((int64_t)1 << 30);
-  if (chip && onchip_prepare(pl, st)) {
-    if (pl->onchip->state == 0) pl->onchip->state = -1;
-    cudaGetLastError();
-    g_last_error.clear();
-  }
-  chip = chip && pl->onchip->state == 1;
-  std::vector<int32_t> mrows(hidx.begin(), hidx.end());
-  std::sort(mrows.begin(), mrows.end());
-  chip = chip && onchip_multi_fit(pl, af, rows_of(frc), mrows, false, st, of);
+  bool chip = onchip_multi_may_fit(pl, Rp, false) && c >= 8 && !pl->timing && !getenv("BFE_NO_GRAPH") && n_t < ((int64_t)1 << 30);
+  oc = chip ? onchip_for_several(pl, st) : nullptr;
+  chip = oc != nullptr;
+  MultiLists lf, la;
+  bfe::StepArgs afc = af;                           // the forward inputs as the chip's parts have them
+  if (chip) onchip_multi_rows(*oc, frc, hidx, lf);
+  chip = chip && onchip_multi_fit(pl, *oc, af, lf.frows, lf.mrows, false, st, of);
+  if (chip && (rc = onchip_multi_lists(pl, *oc, frc, lf, afc))) return rc;
   // With ckpt_every = 0, every forward state stays on the device when the
   // steps + 2 states and the adjoint's c + 2 segment slots fit in 3/4 of the
   // free memory: state u_t sits in slot t - ti0 + 2 of d_all (slots 0 and 1
@@ -241,7 +234,7 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
   if (keep_all) {
     CUDA_TRY(d_all.alloc((size_t)(steps + 2) * sb));
     CUDA_TRY(cudaMemsetAsync(d_all.p, 0, 2 * sb, st));
-    chip = chip && chip_march(of, af, ti0, 1, steps, true, nullptr, nullptr, d_all.p + 2 * sb);
+    chip = chip && chip_march(of, afc, ti0, 1, steps, true, nullptr, nullptr, d_all.p + 2 * sb);
     if (!chip && (rc = forward_steps())) return rc;
   } else {
     CUDA_TRY(d_u.alloc(3 * sb));
@@ -388,6 +381,7 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
   auto S = [&](int64_t k) { return d_seg.p + (size_t)k * sb; };
   auto Lm = [&](int64_t k) { return d_lam.p + (size_t)k * sb; };
   af.n_mon = 0;                      // the recompute does not rewrite the history
+  afc.n_mon = 0;
   bfe::GradArgs g{};
   g.n_el = n_el;
   g.ndf = ndf;
@@ -411,6 +405,10 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
     g.el_out = d_out.p;
   }
   constexpr int kNotLaunched = -1;
+  bfe::StepArgs aac = aa;
+  if (chip) onchip_multi_rows(*oc, afrc, no_mon, la);
+  chip = chip && onchip_multi_fit(pl, *oc, aa, la.frows, la.mrows, false, st, oa);
+  if (chip && (rc = onchip_multi_lists(pl, *oc, afrc, la, aac))) return rc;
   auto sweep = [&](bool use_chip) -> int {
     CUDA_TRY(cudaMemsetAsync(d_lam.p, 0, (size_t)(c + 2) * sb, st));
     CUDA_TRY(cudaMemsetAsync(d_gs.p, 0, n_el * sizeof(double), st));
@@ -424,7 +422,7 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
       } else {
         CUDA_TRY(cudaMemcpyAsync(S(0), d_ck.p + 2 * sb * j, 2 * sb, cudaMemcpyDeviceToDevice, st));
         if (use_chip) {
-          if (!chip_march(of, af, ts, 1, te - ts, false, S(1), S(0), S(2))) return kNotLaunched;
+          if (!chip_march(of, afc, ts, 1, te - ts, false, S(1), S(0), S(2))) return kNotLaunched;
         } else for (int64_t t = ts; t < te; ++t) {
           af.ti = t;
           af.u_prev = S(t - ts);
@@ -434,7 +432,7 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
         }
       }
       if (use_chip) {
-        if (!chip_march(oa, aa, te - 1, -1, te - ts, false, Lm(te - ts), Lm(te - ts + 1), Lm(te - 1 - ts)))
+        if (!chip_march(oa, aac, te - 1, -1, te - ts, false, Lm(te - ts), Lm(te - ts + 1), Lm(te - 1 - ts)))
           return kNotLaunched;
       } else for (int64_t t = te - 1; t >= ts; --t) {
         aa.ti = t;
@@ -459,7 +457,6 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
     }
     return BFE_OK;
   };
-  chip = chip && onchip_multi_fit(pl, aa, rows_of(afrc), {}, false, st, oa);
   rc = sweep(chip);
   if (rc == kNotLaunched) rc = sweep(chip = false);
   if (rc) return rc;

@@ -138,6 +138,8 @@ struct Onchip {
   DevBuf<int32_t> d_part, d_off, d_word, d_bytes, d_cnt, d_halo, d_vptr, d_vhalo;
   DevBuf<uint16_t> flags, order, z_lcol;
   DevBuf<unsigned char> blocks, xch, xchv;
+  DevBuf<int32_t> row_of;           // tiled parts: the plan's row of each row here, and its inverse
+  std::vector<int32_t> place;
   DevBuf<uint4> xchm;               // exchange words of marches with several sources
   std::vector<int32_t> halo_cnt;
   DevBuf<ushort4> lref;
@@ -163,6 +165,7 @@ struct bfe_plan {
   bfe_host::DevBuf<unsigned char> rowc;       // double or float
   std::vector<int32_t> h_slice_ptr;
   std::unique_ptr<bfe_host::Onchip> onchip{new bfe_host::Onchip()};
+  std::unique_ptr<bfe_host::Onchip> tiled{new bfe_host::Onchip()};   // several sources, 2D: parts cut as tiles
   std::vector<uint32_t> h_base;     // node-block base per row
   std::vector<double> h_acoef;      // forcing coefficient per row (diagonal of A)
   // interface correction
@@ -256,12 +259,26 @@ bool onchip_fit(bfe_plan* pl, const std::vector<ForceEntry>& frc, const std::vec
 // Shared memory, threads and exchange buffer of a march with several sources
 // (a: its forcing, monitors and padded R). false: it does not fit, or the step
 // kernels (against_graph: replayed from a graph) are faster.
-bool onchip_multi_fit(bfe_plan* pl, const bfe::StepArgs& a, const std::vector<int32_t>& frc_rows,
+bool onchip_multi_fit(bfe_plan* pl, Onchip& oc, const bfe::StepArgs& a, const std::vector<int32_t>& frc_rows,
                       const std::vector<int32_t>& mon_rows, bool against_graph, cudaStream_t st, bfe::OnchipArgs& o);
+// The partition a march with several sources uses, built at its first use:
+// tiles where the model has them, else the one-source partition; nullptr: none.
+Onchip* onchip_for_several(bfe_plan* pl, cudaStream_t st);
+// The forced and monitored rows of such a march in its partition's order, and
+// (tiles) as a's device lists.
+struct MultiLists {
+  DevBuf<int32_t> ints;
+  DevBuf<unsigned char> coef;
+  std::vector<int32_t> forced, frows, mrows, mslots;
+};
+void onchip_multi_rows(const Onchip& oc, const std::vector<ForceEntry>& frc, const std::vector<int64_t>& hist_idx,
+                       MultiLists& L);
+int onchip_multi_lists(const bfe_plan* pl, const Onchip& oc, const std::vector<ForceEntry>& frc, MultiLists& L,
+                       bfe::StepArgs& a);
 // Whether that is worth building the partition for.
-bool onchip_multi_may_fit(const bfe_plan* pl, int64_t R);
+bool onchip_multi_may_fit(const bfe_plan* pl, int64_t R, bool against_graph);
 // Step numbers for n steps that the exchange buffers do not hold yet.
-int onchip_tags(bfe_plan* pl, int64_t n, cudaStream_t st, uint32_t& tag0);
+int onchip_tags(Onchip& oc, int64_t n, cudaStream_t st, uint32_t& tag0);
 // Device data of a run's prescribed displacements for the on-chip march, and
 // what each part needs for them; fits = false: they do not fit the form.
 struct OnchipV5 {

@@ -192,6 +192,7 @@ struct OnchipArgs {
   const int32_t* slice_word;        // its width and kind
   const int32_t* op_bytes;          // bytes of each part's blocks
   int32_t depth, slot_bytes;        // slots per warp for streamed chunks
+  const int32_t* row_of;            // several sources: the state row of each row (nullptr: itself)
   const ushort4* lref;              // FP32: window indices of a cut block's reference values
   const int32_t* vhalo_ptr;         // interface values each part reads (n_parts + 1)
   const int32_t* vhalo;             // their interface numbers
@@ -239,6 +240,23 @@ struct OnchipBuild {
   int* slot_bytes;                  // of the largest chunk, zeroed
   int* fail;                        // set when the operator does not fit the form
 };
+// The sliced-ELL operator with its rows in another order: row i is row
+// row_of[i] of the given one, place its inverse; a row keeps the order of its
+// entries. slice_ptr is the new one, wide enough for every row.
+struct OnchipReorder {
+  int32_t n, n_slices;
+  const int32_t* row_of;
+  const int32_t* place;
+  const int32_t* old_ptr;
+  const uint32_t* old_col;
+  const void* old_val;
+  const void* old_rowc;
+  const int32_t* slice_ptr;
+  uint32_t* col;
+  void* val;
+  void* rowc;
+};
+cudaError_t launch_onchip_reorder(const OnchipReorder& r, int precision, cudaStream_t s);
 int onchip_block_bound(int precision, int width);    // most bytes of a slice of this width
 cudaError_t launch_onchip_build(const OnchipBuild& b, int precision, cudaStream_t s);
 // n_steps steps from ti0. fresh: from rest, else from a.u_n, a.u_prev. The

@@ -750,6 +750,32 @@ __global__ void __launch_bounds__(256) oc_order(OnchipBuild b) {
   }
 }
 
+// One warp per slice of the new order, lane = row.
+template <typename T>
+__global__ void __launch_bounds__(256) oc_reorder(OnchipReorder r) {
+  const int s = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (s >= r.n_slices) return;
+  const int i = s * kSlice + lane, off = __ldg(r.slice_ptr + s), w = (__ldg(r.slice_ptr + s + 1) - off) >> 5;
+  int from = 0, wf = 0;
+  if (i < r.n) {
+    const int o = __ldg(r.row_of + i), so = o >> 5;
+    from = __ldg(r.old_ptr + so) + (o & 31);
+    wf = (__ldg(r.old_ptr + so + 1) - __ldg(r.old_ptr + so)) >> 5;
+    static_cast<T*>(r.rowc)[i] = __ldg(static_cast<const T*>(r.old_rowc) + o);
+  }
+  for (int k = 0; k < w; ++k) {
+    uint32_t e = (uint32_t)min(i, r.n - 1) | (sizeof(T) == 8 ? 0u : kDirect);
+    T v = T(0);
+    if (k < wf) {
+      e = __ldg(r.old_col + from + 32 * k);
+      e = (e & ~kColMask) | (uint32_t)__ldg(r.place + (e & kColMask));
+      v = __ldg(static_cast<const T*>(r.old_val) + from + 32 * k);
+    }
+    r.col[off + 32 * k + lane] = e;
+    static_cast<T*>(r.val)[off + 32 * k + lane] = v;
+  }
+}
+
 template <typename T>
 cudaError_t build_t(const OnchipBuild& b, cudaStream_t st) {
   const size_t words = (size_t)((b.max_words + kRankWords - 1) / kRankWords) * kRankWords;
@@ -781,6 +807,13 @@ cudaError_t launch_t(const OnchipArgs& o, const StepArgs& a, const V5Args& v, in
 
 int onchip_block_bound(int precision, int width) {
   return precision == 0 ? block_bound<double>(width) : block_bound<float>(width);
+}
+
+cudaError_t launch_onchip_reorder(const OnchipReorder& r, int precision, cudaStream_t st) {
+  const int blocks = (r.n_slices * 32 + 255) / 256;
+  if (precision == 0) oc_reorder<double><<<blocks, 256, 0, st>>>(r);
+  else oc_reorder<float><<<blocks, 256, 0, st>>>(r);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_onchip_build(const OnchipBuild& b, int precision, cudaStream_t st) {

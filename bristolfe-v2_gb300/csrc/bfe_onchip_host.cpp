@@ -79,29 +79,128 @@ bool interface_lists(const bfe_plan* pl, const std::vector<int32_t>& part, Inter
 
 }  // namespace
 
+namespace {
+
+// The operator the parts are cut from: the plan's, or the same in tile order.
+struct PartView {
+  const std::vector<int32_t>* sp;    // slice offsets, here and on the device
+  const int32_t* slice_ptr;
+  const uint32_t* col;
+  const void *val, *rowc;
+};
+
+// Tiles for a 2D model. Contiguous ranges of the caller's node order (column
+// by column) are strips of a mesh column or two when a part is small, and then
+// all of their rows are read by other parts. Here the nodes are put in an
+// order whose contiguous ranges are tiles: the columns are the runs of
+// consecutive nodes that are neighbours; a node's height is its place in its
+// run, levelled to the run on its left by one neighbour there; the columns are
+// cut into px strips, and a strip's nodes sorted by height and cut into py
+// parts. Any order is correct; models that are not so numbered only gain less.
+// perm: row of the plan of each row in tile order. False: not worth it.
+bool tile_order(const bfe_plan* pl, int64_t P, std::vector<int32_t>& perm, std::vector<int32_t>& parts) {
+  const int64_t bs = pl->groups.bs[0], N = pl->groups.n_nodes[0], S = pl->n_slices;
+  if (!pl->have_groups || pl->groups.n_groups != 1 || bs > 2 || N * bs != pl->n) return false;
+  std::vector<int32_t> nptr(N + 1);
+  if (cudaMemcpy(nptr.data(), pl->g_nptr[0].p, nptr.size() * 4, cudaMemcpyDeviceToHost) != cudaSuccess) return false;
+  std::vector<int32_t> nrow(nptr[N]);
+  if (cudaMemcpy(nrow.data(), pl->g_nrow[0].p, nrow.size() * 4, cudaMemcpyDeviceToHost) != cudaSuccess) return false;
+  std::vector<int32_t> start, run(N), level;
+  for (int64_t q = 0; q < N; ++q) {
+    const auto b = nrow.begin() + nptr[q], e = nrow.begin() + nptr[q + 1];
+    if (q == 0 || !std::binary_search(b, e, (int32_t)((q - 1) * bs))) start.push_back((int32_t)q);
+    run[q] = (int32_t)start.size() - 1;
+  }
+  const int64_t M = (int64_t)start.size();
+  level.assign(M, 0);
+  for (int64_t r = 1; r < M; ++r) {
+    const int64_t q0 = start[r], q1 = r + 1 < M ? start[r + 1] : N;
+    for (int64_t d = 0; d < q1 - q0; ++d) {
+      // a node near the middle of the run with neighbours on both sides of its left one
+      const int64_t q = q0 + ((q1 - q0) / 2 + d) % (q1 - q0);
+      int64_t hi = -1, lo = 0;
+      for (int32_t e = nptr[q]; e < nptr[q + 1] && nrow[e] / bs < q0; ++e) {
+        const int64_t j = nrow[e] / bs;
+        if (hi < 0 || run[j] != run[hi]) lo = j;
+        hi = j;
+      }
+      if (hi - lo != 2) continue;
+      level[r] = (int32_t)(level[run[hi]] + (lo + 1 - start[run[hi]]) - (q - q0));
+      break;
+    }
+  }
+  // px strips of py parts: a row costs about twice what a halo row does
+  const double len = (double)N / (double)M;
+  auto cost = [&](int64_t px, int64_t py) {
+    const double w = (double)M / (double)px, h = len / (double)py;
+    const double halo = (px > 1 ? 2 * h : 0) + (py > 1 ? 2 * w : 0) + 4;
+    return (double)((S + px * py - 1) / (px * py) * bfe::kSlice) + 0.5 * halo * (double)bs;
+  };
+  int64_t px = P, py = 1;
+  for (int64_t x = 1; x <= std::min(P, M); ++x)
+    for (int64_t y = 1; x * y <= P && y <= (int64_t)len; ++y)
+      if (cost(x, y) < cost(px, py)) px = x, py = y;
+  if (py == 1 || cost(px, py) > 0.9 * cost(P, 1)) return false;
+  perm.resize(pl->n);
+  parts.assign(1, 0);
+  std::vector<int32_t> first, node;
+  for (int64_t x = 0; x < px; ++x) {
+    const int64_t s0 = S * x / px, s1 = S * (x + 1) / px;
+    const int64_t a = s0 * bfe::kSlice / bs, b = std::min<int64_t>(N, s1 * bfe::kSlice / bs);
+    auto height = [&](int64_t q) { return (int64_t)q - start[run[q]] + level[run[q]]; };
+    int64_t lo = INT64_MAX, hi = INT64_MIN;
+    for (int64_t q = a; q < b; ++q) lo = std::min(lo, height(q)), hi = std::max(hi, height(q));
+    if (hi - lo > 8 * N) return false;
+    first.assign(hi - lo + 2, 0);
+    for (int64_t q = a; q < b; ++q) ++first[height(q) - lo + 1];
+    std::partial_sum(first.begin(), first.end(), first.begin());
+    node.resize(b - a);
+    for (int64_t q = a; q < b; ++q) node[first[height(q) - lo]++] = (int32_t)q;
+    for (int64_t k = 0; k < b - a; ++k)
+      for (int64_t l = 0; l < bs; ++l) perm[(a + k) * bs + l] = (int32_t)(node[k] * bs + l);
+    for (int64_t y = 0; y < py; ++y) parts.push_back((int32_t)(s0 + (s1 - s0) * (y + 1) / py));
+  }
+  return true;
+}
+
+}  // namespace
+
 namespace bfe_host {
 
-int onchip_prepare(bfe_plan* pl, cudaStream_t st) {
-  Onchip& oc = *pl->onchip;
-  if (oc.state) return BFE_OK;
-  oc.state = -1;
+// Sources up to which a march on the chip is the faster one (onchip_multi_fit);
+// FP64 multiply-adds weigh as much as a launch: 1,722 DOF R = 16 9.6 us per
+// step on chip against 8.2.
+static int64_t most_sources(int prec, bool against_graph) {
+  return !against_graph ? 16 : prec == BFE_PREC_DOUBLE ? 8 : 64;
+}
+
+static int64_t max_parts(int64_t slices) {
+  return std::min<int64_t>(bfe::sm_count(), (slices + kMinSlices - 1) / kMinSlices);
+}
+
+
+// Builds the partition of holder; parts already in part_slice are kept.
+static int build_parts(bfe_plan* pl, std::unique_ptr<Onchip>& holder, const PartView& view,
+                       const std::vector<uint32_t>& h_base, cudaStream_t st) {
+  Onchip& oc = *holder;
   const int64_t n = pl->n, S = pl->n_slices;
   const int prec = pl->prec;
   const int64_t es = (int64_t)elem_size(prec);
   int coop = 0;
   CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, pl->device));
-  const int64_t P = std::min<int64_t>(bfe::sm_count(), (S + kMinSlices - 1) / kMinSlices);
+  const bool given = !oc.part_slice.empty();
+  const int64_t P = given ? (int64_t)oc.part_slice.size() - 1 : max_parts(S);
   // 16-bit window indices; FP32 entries use two bits to name a reference value
   const int64_t max_window = std::min<int64_t>(kSmemLimit / (2 * es), es == 8 ? 65535 : 16383);
   if (!coop || P < 1 || n > P * max_window) return BFE_OK;
   // contiguous parts of even cost: a slice costs its width (one load of
   // operator and state per entry) and a fixed part for the row's update
-  const std::vector<int32_t>& sp = pl->h_slice_ptr;
+  const std::vector<int32_t>& sp = *view.sp;
   auto cost = [&](int64_t s) { return (double)((sp[s + 1] - sp[s]) / bfe::kSlice) + 4.0; };
   double total = 0;
   for (int64_t s = 0; s < S; ++s) total += cost(s);
-  oc.part_slice.assign(1, 0);
-  {
+  if (!given) {
+    oc.part_slice.assign(1, 0);
     double run = 0;
     int64_t s = 0;
     for (int64_t p = 0; p < P; ++p) {
@@ -116,7 +215,7 @@ int onchip_prepare(bfe_plan* pl, cudaStream_t st) {
         // edge to a node's first row where one is near (3D: every 96 rows)
         for (int64_t d : {0, 1, -1, 2, -2}) {
           const int64_t x = s + d;
-          if (x <= oc.part_slice.back() || x > must || (int64_t)pl->h_base[x * bfe::kSlice] != x * bfe::kSlice) continue;
+          if (x <= oc.part_slice.back() || x > must || (int64_t)h_base[x * bfe::kSlice] != x * bfe::kSlice) continue;
           for (; s < x; ++s) run += cost(s);
           for (; s > x; --s) run -= cost(s - 1);
           break;
@@ -161,7 +260,7 @@ int onchip_prepare(bfe_plan* pl, cudaStream_t st) {
   CUDA_TRY(oc.blocks.alloc(off));
   if (prec == BFE_PREC_SINGLE) {
     CUDA_TRY(oc.lref.alloc(n));
-    CUDA_TRY(base.upload(pl->h_base));
+    CUDA_TRY(base.upload(h_base));
   }
   CUDA_TRY(scratch.alloc((size_t)n * 2 + (size_t)P * P));
   CUDA_TRY(cudaMemsetAsync(scratch.p, 0, (size_t)n * 2 + (size_t)P * P, st));
@@ -175,15 +274,17 @@ int onchip_prepare(bfe_plan* pl, cudaStream_t st) {
     CUDA_TRY(oc.xchv.alloc((size_t)pl->n_int * 4 * es));
     CUDA_TRY(cudaMemsetAsync(oc.xchv.p, 0, (size_t)pl->n_int * 4 * es, st));
   }
-  CUDA_TRY(oc.xch.alloc((size_t)n * 4 * es));
-  CUDA_TRY(cudaMemsetAsync(oc.xch.p, 0, (size_t)n * 4 * es, st));
+  if (!given) {
+    CUDA_TRY(oc.xch.alloc((size_t)n * 4 * es));
+    CUDA_TRY(cudaMemsetAsync(oc.xch.p, 0, (size_t)n * 4 * es, st));
+  }
   CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));     // the uploads, before st reads them
   b.part_slice = oc.d_part.p;
-  b.slice_ptr = pl->slice_ptr.p;
+  b.slice_ptr = view.slice_ptr;
   b.block_off = oc.d_off.p;
-  b.col = pl->col.p;
-  b.val = pl->val.p;
-  b.rowc = pl->rowc.p;
+  b.col = view.col;
+  b.val = view.val;
+  b.rowc = view.rowc;
   b.base = base.p;
   b.int_row = pl->int_row.p;
   b.v_exported = vexp.p;
@@ -226,8 +327,8 @@ int onchip_prepare(bfe_plan* pl, cudaStream_t st) {
     if (need > kSmemLimit || rp + cnt[p] > max_window) failed = true;
   }
   if (failed) {
-    pl->onchip.reset(new Onchip());
-    pl->onchip->state = -1;
+    holder.reset(new Onchip());
+    holder->state = -1;
     return BFE_OK;
   }
   oc.op_bytes = obytes;
@@ -250,6 +351,7 @@ int onchip_prepare(bfe_plan* pl, cudaStream_t st) {
   o.block_off = oc.d_off.p;
   o.slice_word = oc.d_word.p;
   o.op_bytes = oc.d_bytes.p;
+  o.row_of = oc.row_of.p;
   o.lref = oc.lref.p;
   o.vhalo_ptr = oc.d_vptr.p;
   o.vhalo = oc.d_vhalo.p;
@@ -261,6 +363,69 @@ int onchip_prepare(bfe_plan* pl, cudaStream_t st) {
   oc.next_tag = 1;
   oc.state = 1;
   return BFE_OK;
+}
+
+int onchip_prepare(bfe_plan* pl, cudaStream_t st) {
+  if (pl->onchip->state) return BFE_OK;
+  pl->onchip->state = -1;
+  const PartView view{&pl->h_slice_ptr, pl->slice_ptr.p, pl->col.p, pl->val.p, pl->rowc.p};
+  return build_parts(pl, pl->onchip, view, pl->h_base, st);
+}
+
+// The tiled partition, if the model has one.
+static int prepare_tiled(bfe_plan* pl, cudaStream_t st) {
+  if (pl->tiled->state) return BFE_OK;
+  pl->tiled->state = -1;
+  Onchip& oc = *pl->tiled;
+  const int64_t n = pl->n, S = pl->n_slices;
+  std::vector<int32_t> perm;
+  if (!tile_order(pl, max_parts(S), perm, oc.part_slice)) return BFE_OK;
+  oc.place.resize(n);
+  for (int64_t i = 0; i < n; ++i) oc.place[perm[i]] = (int32_t)i;
+  std::vector<uint32_t> base;
+  if (pl->prec == BFE_PREC_SINGLE) {
+    base.resize(n);
+    for (int64_t i = 0; i < n; ++i) base[i] = (uint32_t)oc.place[pl->h_base[perm[i]]];
+  }
+  std::vector<int32_t> sp(S + 1, 0);
+  for (int64_t s = 0; s < S; ++s) {
+    int32_t w = 0;
+    for (int64_t i = s * bfe::kSlice; i < std::min<int64_t>(n, (s + 1) * bfe::kSlice); ++i) {
+      const int32_t o = perm[i] / bfe::kSlice;
+      w = std::max(w, pl->h_slice_ptr[o + 1] - pl->h_slice_ptr[o]);
+    }
+    if ((int64_t)sp[s] + w > INT32_MAX) return BFE_OK;
+    sp[s + 1] = sp[s] + w;
+  }
+  const int64_t es = (int64_t)elem_size(pl->prec);
+  DevBuf<int32_t> place, slice_ptr;
+  DevBuf<uint32_t> col;
+  DevBuf<unsigned char> val, rowc;
+  CUDA_TRY(oc.row_of.upload(perm));
+  CUDA_TRY(place.upload(oc.place));
+  CUDA_TRY(slice_ptr.upload(sp));
+  CUDA_TRY(col.alloc(sp[S]));
+  CUDA_TRY(val.alloc((size_t)sp[S] * es));
+  CUDA_TRY(rowc.alloc((size_t)n * es));
+  CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));     // the uploads, before st reads them
+  bfe::OnchipReorder r{(int32_t)n, (int32_t)S, oc.row_of.p, place.p, pl->slice_ptr.p, pl->col.p, pl->val.p, pl->rowc.p,
+                       slice_ptr.p, col.p, val.p, rowc.p};
+  CUDA_TRY(bfe::launch_onchip_reorder(r, pl->prec, st));
+  const PartView view{&sp, slice_ptr.p, col.p, val.p, rowc.p};
+  return build_parts(pl, pl->tiled, view, base, st);     // synchronises before it returns
+}
+
+Onchip* onchip_for_several(bfe_plan* pl, cudaStream_t st) {
+  for (auto* oc : {&pl->tiled, &pl->onchip}) {
+    if ((oc == &pl->tiled ? prepare_tiled(pl, st) : onchip_prepare(pl, st)) != BFE_OK) {
+      if ((*oc)->state == 0) (*oc)->state = -1;
+      cudaStreamSynchronize(st);
+      cudaGetLastError();
+      g_last_error.clear();
+    }
+    if ((*oc)->state == 1) return oc->get();
+  }
+  return nullptr;
 }
 
 bool onchip_fit(bfe_plan* pl, const std::vector<ForceEntry>& frc, const std::vector<int64_t>& v5_bytes,
@@ -369,19 +534,62 @@ int onchip_v5(bfe_plan* pl, const V5Lists& L, OnchipV5& d, bool& fits) {
   return BFE_OK;
 }
 
-bool onchip_multi_may_fit(const bfe_plan* pl, int64_t R) {
-  if (pl->n_int || R < 2 || R > 64 || R % bfe::onchip_multi_rv(pl->prec)) return false;
+bool onchip_multi_may_fit(const bfe_plan* pl, int64_t R, bool against_graph) {
+  if (pl->n_int || R < 2 || R > most_sources(pl->prec, against_graph) || R % bfe::onchip_multi_rv(pl->prec)) return false;
   // the states alone must fit in the SMs' shared memory
   return 2 * (double)pl->n * (double)R * (double)elem_size(pl->prec) <= (double)kSmemLimit * bfe::sm_count();
 }
 
-bool onchip_multi_fit(bfe_plan* pl, const bfe::StepArgs& a, const std::vector<int32_t>& frc_rows,
+void onchip_multi_rows(const Onchip& oc, const std::vector<ForceEntry>& frc, const std::vector<int64_t>& hist_idx,
+                       MultiLists& L) {
+  auto at = [&](int64_t row) { return oc.place.empty() ? (int32_t)row : oc.place[row]; };
+  L.forced.resize(frc.size());
+  std::iota(L.forced.begin(), L.forced.end(), 0);
+  std::stable_sort(L.forced.begin(), L.forced.end(),
+                   [&](int32_t x, int32_t y) { return at(frc[x].row) < at(frc[y].row); });
+  std::vector<std::pair<int32_t, int32_t>> mons;
+  for (size_t k = 0; k < hist_idx.size(); ++k)
+    if (hist_idx[k] >= 0) mons.emplace_back(at(hist_idx[k]), (int32_t)k);
+  std::sort(mons.begin(), mons.end());
+  for (int32_t k : L.forced) L.frows.push_back(at(frc[k].row));
+  for (auto& x : mons) {
+    L.mrows.push_back(x.first);
+    L.mslots.push_back(x.second);
+  }
+}
+
+int onchip_multi_lists(const bfe_plan* pl, const Onchip& oc, const std::vector<ForceEntry>& frc, MultiLists& L,
+                       bfe::StepArgs& a) {
+  if (oc.place.empty()) return BFE_OK;             // the run's own lists serve
+  std::vector<int32_t> ints(L.frows);
+  for (int32_t k : L.forced) ints.push_back(frc[k].rhs);
+  for (int32_t k : L.forced) ints.push_back(frc[k].sig);
+  ints.insert(ints.end(), L.mrows.begin(), L.mrows.end());
+  ints.insert(ints.end(), L.mslots.begin(), L.mslots.end());
+  std::vector<unsigned char> coef;
+  for (int32_t k : L.forced) {
+    const double c = pl->h_acoef[frc[k].row] * frc[k].w;
+    if (pl->prec == BFE_PREC_DOUBLE) push_val<double>(coef, c); else push_val<float>(coef, c);
+  }
+  CUDA_TRY(L.ints.upload(ints));
+  CUDA_TRY(L.coef.upload(coef));
+  CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));     // before the run's stream reads them
+  const size_t nf = L.frows.size(), nm = L.mrows.size();
+  a.frc_row = L.ints.p;
+  a.frc_rhs = L.ints.p + nf;
+  a.frc_sig = L.ints.p + 2 * nf;
+  a.frc_coef = L.coef.p;
+  a.mon_row = L.ints.p + 3 * nf;
+  a.mon_slot = L.ints.p + 3 * nf + nm;
+  return BFE_OK;
+}
+
+bool onchip_multi_fit(bfe_plan* pl, Onchip& oc, const bfe::StepArgs& a, const std::vector<int32_t>& frc_rows,
                       const std::vector<int32_t>& mon_rows, bool against_graph, cudaStream_t st, bfe::OnchipArgs& o) {
-  Onchip& oc = *pl->onchip;
   o = oc.args;
   const int P = o.n_parts;
   const int64_t R = a.R, es = (int64_t)elem_size(pl->prec), rv = bfe::onchip_multi_rv(pl->prec);
-  if (!onchip_multi_may_fit(pl, R)) return false;
+  if (!onchip_multi_may_fit(pl, R, against_graph)) return false;
   int64_t smem = 0, tasks = 0, words = 0;
   const int64_t wpr = pl->prec == BFE_PREC_DOUBLE ? R : R / 2;
   auto in_part = [&](const std::vector<int32_t>& v, int p) {
@@ -392,23 +600,24 @@ bool onchip_multi_fit(bfe_plan* pl, const bfe::StepArgs& a, const std::vector<in
     const int64_t ns = oc.part_slice[p + 1] - oc.part_slice[p], rp = ns * bfe::kSlice, H = oc.halo_cnt[p];
     const int64_t nf = in_part(frc_rows, p), nm = in_part(mon_rows, p);
     const int64_t W = bfe::onchip_multi_window((int)(rp + H));
-    const int64_t need = 2 * R * W * es + 3 * align2(nf) * es + ns * 8 + (2 * nf + 2 * nm + H) * 4 + rp * 2 + 16 +
+    const int64_t need = 2 * R * W * es + 3 * align2(nf) * es + ns * 8 + (2 * nf + 2 * nm + H + rp) * 4 + rp * 2 + 16 +
                          oc.op_bytes[p];
     if (need > kSmemLimit || nf > 1024) return false;
     smem = std::max(smem, need);
     tasks = std::max(tasks, ns * (R / rv));
     words = std::max(words, H * wpr);
   }
-  // Against step kernels replayed from a graph (about 8 us per step for small
-  // models) the exchange decides, about 2 us per 1,000 words of a part. us per
-  // step on chip / graph: plate of 40,602 DOF FP32 R = 4 3.3 / 8.1 (808
-  // words), R = 16 9.3 / 9.1 (3,232), R = 32 14.1 / 9.9; 10,302 DOF R = 16 5.3
-  // / 8.8, R = 32 8.0 / 9.1 (3,264); bricks of 46,128 DOF R = 4 8.0 / 11.7. In
-  // FP64 the multiply-adds weigh as much: 40,602 DOF R = 4 6.6 / 10.0, R = 8
-  // 12.2 / 13.9; 1,722 DOF R = 16 9.6 / 8.2. One launch per step, which the
-  // adjoint would make, is slower wherever this fits up to R = 16 (17 us per
-  // step of 90,902 DOF, R = 16, against 13).
-  if (against_graph ? !(R <= (es == 8 ? 4 : 8) || (words <= 3300 && R <= (es == 8 ? 8 : 64))) : R > 16) return false;
+  // Against step kernels replayed from a graph (8 to 12 us per step for models
+  // that fit) the exchange decides, about 2 us per 1,000 words of a part. Us
+  // per step on chip / graph, in tiles: plate of 40,602 DOF FP32 R = 4 2.8 /
+  // 8.1, R = 16 4.7 / 9.1, R = 32 7.2 / 10.2, R = 48 10.3 / 12.2; 90,902 DOF
+  // R = 16 7.1 / 10.6, R = 24 9.8 / 13.0; 1,722 DOF R = 64 7.6 / 9.7; FP64
+  // 40,602 DOF R = 8 10.1 / 13.9. In strips (a model without tiles): bricks of
+  // 14,553 DOF R = 8 8.6 / 9.9, of 46,128 R = 4 8.0 / 12.0; a plate in strips
+  // 40,602 DOF R = 16 9.3 / 9.1 (3,232 words), R = 32 14.1 / 9.9. One launch
+  // per step, which the adjoint would make, is slower wherever this fits up to
+  // R = 16 (17 us per step of 90,902 DOF, R = 16, against 7.5).
+  if (against_graph && words > 3300 && R > (es == 8 ? 4 : 8)) return false;
   const int64_t turns = (tasks + 31) / 32, warps = (tasks + turns - 1) / turns;
   o.threads = (int32_t)std::max<int64_t>({128, warps * 32, std::min<int64_t>(1024, (words / 4 + 31) / 32 * 32)});
   for (int p = 0; p < P; ++p)
@@ -428,10 +637,9 @@ bool onchip_multi_fit(bfe_plan* pl, const bfe::StepArgs& a, const std::vector<in
   return true;
 }
 
-int onchip_tags(bfe_plan* pl, int64_t n, cudaStream_t st, uint32_t& tag0) {
-  Onchip& oc = *pl->onchip;
+int onchip_tags(Onchip& oc, int64_t n, cudaStream_t st, uint32_t& tag0) {
   if ((uint64_t)oc.next_tag + (uint64_t)n + 2 > 0xffffffffull) {
-    CUDA_TRY(cudaMemsetAsync(oc.xch.p, 0, oc.xch.n, st));
+    if (oc.xch.n) CUDA_TRY(cudaMemsetAsync(oc.xch.p, 0, oc.xch.n, st));
     if (oc.xchv.n) CUDA_TRY(cudaMemsetAsync(oc.xchv.p, 0, oc.xchv.n, st));
     if (oc.xchm.n) CUDA_TRY(cudaMemsetAsync(oc.xchm.p, 0, oc.xchm.n * sizeof(uint4), st));
     oc.next_tag = 1;

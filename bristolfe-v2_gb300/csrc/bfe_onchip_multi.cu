@@ -10,7 +10,12 @@
 // RV right-hand sides, so an entry's value and index are loaded once for RV
 // multiply-adds; states are planes [R][window], so lanes of a gather fall on
 // neighbouring words. Exchange words hold two FP32 values or one FP64 value,
-// each 4 bytes beside their step number. With m.out every new state is also
+// each 4 bytes beside their step number. Its volume, R words a halo row, bounds
+// the march for many sources, so 2D models are cut into tiles (o.row_of,
+// bfe_onchip_host.cpp) where contiguous rows would be strips of a mesh column
+// or two, all read by other parts: 90,902 DOF, R = 16 12.0 us per step in
+// strips (604 halo rows a part), 7.1 in tiles (about 150); 40,602 DOF R = 16
+// 8.8 / 4.7, R = 4 3.3 / 2.8. With m.out every new state is also
 // written to global memory, [n][R] at m.out + k m.out_stride.
 //
 // Arithmetic and order are those of the group kernels (step_f32_groupn,
@@ -221,10 +226,14 @@ __global__ void __launch_bounds__(1024, 1) march_onchip_multi(OnchipArgs o, Step
   int32_t* mrow = frr + nf;
   int32_t* mslot = mrow + nm;
   int32_t* hr = mslot + nm;                             // halo rows
-  uint16_t* fl = reinterpret_cast<uint16_t*>(hr + H);
+  int32_t* orow = hr + H;                               // the rows' places in the caller's states
+  uint16_t* fl = reinterpret_cast<uint16_t*>(orow + rpad);
   unsigned char* cache = sm + ((reinterpret_cast<unsigned char*>(fl + rpad) - sm + 15) & ~15);
 
-  for (int r = tid; r < rpad; r += nt) fl[r] = r < rows ? __ldg(o.flags + row0 + r) : 0;
+  for (int r = tid; r < rpad; r += nt) {
+    fl[r] = r < rows ? __ldg(o.flags + row0 + r) : 0;
+    orow[r] = r < rows && o.row_of ? __ldg(o.row_of + row0 + r) : row0 + r;
+  }
   for (int k = tid; k < nf; k += nt) {
     frw[k] = __ldg(a.frc_row + f0 + k) - row0;
     frr[k] = __ldg(a.frc_rhs + f0 + k);
@@ -273,7 +282,8 @@ __global__ void __launch_bounds__(1024, 1) march_onchip_multi(OnchipArgs o, Step
   for (int k = tid; k < R * W; k += nt) {
     const int r = k / W, x = k - r * W;
     T un = T(0), up = T(0);
-    const int g = x < rpad ? (x < rows ? row0 + x : -1) : (x < rpad + H ? hr[x - rpad] : -1);
+    int g = x < rpad ? (x < rows ? orow[x] : -1) : (x < rpad + H ? hr[x - rpad] : -1);
+    if (x >= rpad && g >= 0 && o.row_of) g = __ldg(o.row_of + g);
     if (!fresh && g >= 0) {
       un = static_cast<const T*>(a.u_n)[(size_t)g * R + r];
       if (x < rpad) up = static_cast<const T*>(a.u_prev)[(size_t)g * R + r];
@@ -380,7 +390,7 @@ __global__ void __launch_bounds__(1024, 1) march_onchip_multi(OnchipArgs o, Step
 #pragma unroll
         for (int v = 0; v < kRe; ++v) wput(w + v, pk.e[v], tag);
       }
-      if (out && r < rows) *reinterpret_cast<Pack*>(out + (size_t)(row0 + r) * R + r0) = pk;
+      if (out && r < rows) *reinterpret_cast<Pack*>(out + (size_t)orow[r] * R + r0) = pk;
     }
     out = out ? out + m.out_stride : out;
     if (k + 1 < n_steps) {
@@ -418,8 +428,8 @@ __global__ void __launch_bounds__(1024, 1) march_onchip_multi(OnchipArgs o, Step
   for (int k = tid; k < rows * R; k += nt) {
     const int x = k / R, r = k - x * R;
     const uint32_t at = r / PER * ws + x * (uint32_t)sizeof(E) + r % PER * (uint32_t)sizeof(T);
-    static_cast<T*>(a.u_new)[(size_t)(row0 + x) * R + r] = sm_at<T>(sm, au + at);
-    const_cast<T*>(static_cast<const T*>(a.u_prev))[(size_t)(row0 + x) * R + r] = sm_at<T>(sm, bu + at);
+    static_cast<T*>(a.u_new)[(size_t)orow[x] * R + r] = sm_at<T>(sm, au + at);
+    const_cast<T*>(static_cast<const T*>(a.u_prev))[(size_t)orow[x] * R + r] = sm_at<T>(sm, bu + at);
   }
 }
 

@@ -170,28 +170,20 @@ int march_on_chip_multi(bfe_plan* pl, RunSpec& rs, bfe::StepArgs a, unsigned cha
   if (pl->timing || pl->time_limit_s > 0.0 || steps < kOnchipMinSteps || rs.n_t >= ((int64_t)1 << 30) || pl->n_int ||
       getenv("BFE_NO_GRAPH") || getenv("BFE_VARIANT"))
     return BFE_OK;
-  if (!onchip_multi_may_fit(pl, a.R)) return BFE_OK;
-  if (onchip_prepare(pl, st)) {
-    if (pl->onchip->state == 0) pl->onchip->state = -1;
-    cudaGetLastError();
-    g_last_error.clear();
-    return BFE_OK;
-  }
-  if (pl->onchip->state != 1) return BFE_OK;
-  std::vector<int32_t> frows, mrows;
-  for (auto& f : rs.frc) frows.push_back(f.row);
-  for (int64_t h : rs.hist_idx)
-    if (h >= 0) mrows.push_back((int32_t)h);
-  std::sort(frows.begin(), frows.end());
-  std::sort(mrows.begin(), mrows.end());
+  if (!onchip_multi_may_fit(pl, a.R, true)) return BFE_OK;
+  Onchip* oc = onchip_for_several(pl, st);
+  if (!oc) return BFE_OK;
+  MultiLists L;
   bfe::OnchipArgs o;
-  if (!onchip_multi_fit(pl, a, frows, mrows, true, st, o)) return BFE_OK;
+  onchip_multi_rows(*oc, rs.frc, rs.hist_idx, L);
+  if (!onchip_multi_fit(pl, *oc, a, L.frows, L.mrows, true, st, o)) return BFE_OK;
+  if (const int rc = onchip_multi_lists(pl, *oc, rs.frc, L, a)) return rc;
   o.err = pl->d_flag.p + 1;
   int prev = 2, cur = 0, next = 1;
   for (int64_t ti = rs.ti_start; ti < rs.n_t; ti += kOnchipLaunchSteps) {
     const int64_t k = std::min(kOnchipLaunchSteps, rs.n_t - ti);
     int rc;
-    if ((rc = onchip_tags(pl, k, st, o.tag0))) return rc;
+    if ((rc = onchip_tags(*oc, k, st, o.tag0))) return rc;
     a.u_prev = U[prev];
     a.u_n = U[cur];
     a.u_new = U[next];
@@ -210,7 +202,7 @@ int march_on_chip_multi(bfe_plan* pl, RunSpec& rs, bfe::StepArgs a, unsigned cha
   CUDA_TRY(cudaMemcpyAsync(&gave_up, o.err, sizeof(int), cudaMemcpyDeviceToHost, st));
   CUDA_TRY(cudaStreamSynchronize(st));
   if (gave_up) {
-    pl->onchip->state = -1;
+    oc->state = -1;
     return BFE_OK;
   }
   if (cur != 1)
@@ -274,7 +266,7 @@ int march_on_chip(bfe_plan* pl, RunSpec& rs, bfe::StepArgs a, unsigned char* con
     a.dt = pl->dt;
   }
   int rct;
-  if ((rct = onchip_tags(pl, rs.n_t, st, o.tag0))) return rct;
+  if ((rct = onchip_tags(*pl->onchip, rs.n_t, st, o.tag0))) return rct;
   o.err = pl->d_flag.p + 1;
   int prev = 2, cur = 0, next = 1;
   for (int64_t ti = rs.ti_start; ti < rs.n_t; ti += kOnchipLaunchSteps) {

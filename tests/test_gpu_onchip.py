@@ -168,3 +168,38 @@ def test_several_sources(bfe, models, name, R, prec, monkeypatch):
     on, off = _both(bfe, monkeypatch, run)
     for a, b in zip(on, off):
         assert np.abs(b).max() > 0 and np.array_equal(a, b)
+
+
+def _tile_models():
+    from bfe_gb300 import model
+    p = modelgen.solid_plate(W=9e-3, H=4.7e-3, h=0.1e-3)
+    yield "wide", p["K"], p["C"], p["M"], p["gl"], p["dt"], 2
+    p = modelgen.solid_plate(W=3.1e-3, H=12e-3, h=0.1e-3)
+    yield "tall", p["K"], p["C"], p["M"], p["gl"], p["dt"], 2
+    p = modelgen.solid_plate(W=9e-3, H=4.7e-3, h=0.1e-3, dof_to_use=(3,))
+    yield "one_dof", p["K"], p["C"], p["M"], p["gl"], p["dt"], 3
+    p = model.steel_subdomain(6e-3, 0.1e-3, seed=3, n_src=4, n_mon=4)      # a void: columns in two pieces
+    yield "void", p["K"], p["C"], p["M"], p["gl"], p["dt"], 2
+
+
+@pytest.mark.parametrize("prec", ["double", "single"])
+@pytest.mark.parametrize("name", ["wide", "tall", "one_dof", "void"])
+def test_tiles(bfe, name, prec, monkeypatch):
+    """Parts cut as tiles against the step kernels, bit for bit: sources and
+    monitors all over the model, each in its own order."""
+    K, C, M, gl, dt, dof = {x[0]: x[1:] for x in _tile_models()}[name]
+    n = K.shape[0]
+    rng = np.random.default_rng(5)
+    t, s = modelgen.pulse(130, dt)
+    nodes = rng.permutation(np.nonzero(gl[:, dof - 1] > 0)[0] + 1)
+    srcs = [modelgen.gi_of(gl, nodes[[r, r + 8]], dof) for r in range(8)]
+    hi = np.concatenate([rng.permutation(np.arange(1, n + 1))[:700], [1, n, n]])
+
+    def run():
+        with bfe.Plan(K, C, M, dt, bfe.VEL_CURRENT, prec, gl) as plan:
+            h = [plan.run_batched(t, srcs, s * k, hi) for k in (1.0, 2.0)]
+            return h, plan.stats()["step_launches"]
+
+    on, off = _both(bfe, monkeypatch, run)
+    for a, b in zip(on, off):
+        assert np.abs(b).max() > 0 and np.array_equal(a, b)
