@@ -240,8 +240,15 @@ __global__ void __launch_bounds__(256) grad_stiff_w(int64_t n_el, const int32_t*
 // DOF that is unused (-1) reads row 0 unmasked: its row of W_e is zero (the
 // host zeroes the unused rows and columns of K_e before factoring), so it
 // adds nothing while every load of a step issues unconditionally.
+// Bound by the latency of a step's 2 NDF gathered loads: for 6 DOFs, five
+// blocks of 128 threads per SM leave 92 registers, with which a step's loads
+// are all in flight (90,902 DOF, 16 sources, 1,000 steps: 4.2 ms against 6.2
+// with 256 threads at 76 registers; six blocks 5.5, eight 5.8, the next step's
+// loads ahead in registers 4.6 at best).
+template <int NDF> constexpr int kWfThreads = NDF == 6 ? 128 : 256;
+template <int NDF> constexpr int kWfBlocks = NDF == 6 ? 5 : 1;
 template <int NDF, int RK>
-__global__ void __launch_bounds__(256) grad_stiff_wf(int64_t n_el, const int32_t* __restrict__ el_dof,
+__global__ void __launch_bounds__(kWfThreads<NDF>, kWfBlocks<NDF>) grad_stiff_wf(int64_t n_el, const int32_t* __restrict__ el_dof,
                                                      const float* __restrict__ w,
                                                      const int32_t* __restrict__ el_out,
                                                      const float* __restrict__ lam, const float* __restrict__ u,
@@ -406,7 +413,7 @@ template <typename T, int NDF, int RK>
 cudaError_t launch_stiff_w(const GradArgs& g, cudaStream_t st) {
   if (sizeof(T) == 4 && g.R % 4 == 0 && g.n * g.R < (int64_t)INT32_MAX) {
     const int tpe = lanes_for(g.R, 4);
-    const int threads = 256;
+    const int threads = kWfThreads<NDF>;
     const int64_t blocks = (g.n_el * tpe + threads - 1) / threads;
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
     const float* w = static_cast<const float*>(g.w);
