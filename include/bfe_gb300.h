@@ -379,7 +379,8 @@ int bfe_run_device(bfe_plan* plan, int64_t R, int64_t n_t, int64_t ti_start,
  * segment into the gradients in one pass. With ckpt_every = 0 the forward
  * march keeps every state on the device when (steps + c + 4) n R state
  * values fit in 3/4 of the free device memory, and the sweep contracts
- * straight from them. Otherwise (or with ckpt_every > 0) it stores
+ * straight from them (in segments four times as long where these fit as
+ * well). Otherwise (or with ckpt_every > 0) it stores
  * (u_{t-2}, u_{t-1}) every c steps and recomputes each segment from its
  * checkpoint: about 2 n R (steps / c + c) state values of device memory.
  * Both give the same gradient. Only 'vel at curent time step' plans with a
