@@ -15,9 +15,10 @@ constexpr int64_t kMinSlices = 4;
 // Largest operator, as blocks: three quarters of the 129 MB L2. Above it the
 // streamed chunks come from HBM as the step kernels' operator does: FP64
 // bricks of 202,878 DOF (163 MB) took 39 us per step against 35.5 with one
-// launch per step, coupled 961,641 DOF in FP64 (101 MB) 27.6 against 27.7,
-// while 492,579 DOF (52 MB) took 14.2 against 19.3.
-constexpr int64_t kMaxOperator = (int64_t)96 << 20;
+// launch per step. FP64, whose blocks are known before they are built, stops
+// a little lower: coupled 961,641 DOF (96 MB) took 27.6 us against 25.6, while
+// 492,579 DOF (52 MB) took 14.2 against 19.3.
+constexpr int64_t kMaxOperator = (int64_t)96 << 20, kMaxOperator64 = (int64_t)88 << 20;
 
 inline int64_t align2(int64_t x) { return (x + 1) & ~(int64_t)1; }
 
@@ -233,7 +234,7 @@ static int build_parts(bfe_plan* pl, std::unique_ptr<Onchip>& holder, const Part
     off += bfe::onchip_block_bound(prec, (sp[s + 1] - sp[s]) / bfe::kSlice);
     if (off / 16 > INT32_MAX) return BFE_OK;
   }
-  if (prec == BFE_PREC_DOUBLE && off > kMaxOperator) return BFE_OK;     // exact for FP64: do not build
+  if (prec == BFE_PREC_DOUBLE && off > kMaxOperator64) return BFE_OK;   // exact for FP64: do not build
   if (max_slices * bfe::kSlice > max_window) return BFE_OK;
   InterfaceLists L;
   if (pl->n_int && !interface_lists(pl, oc.part_slice, L)) return BFE_OK;
