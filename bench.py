@@ -773,7 +773,7 @@ def adjoint_section(torch, bfe_gb300, model, n_fd=20, n_t=4000):
         obs = p.run_batched(t, srcs, sig, rec)
     K0, C0, M0 = model.assemble_from_elements(ke, mh, ch, dof, n, None, rho_e)
     res = {"n_dof": n, "elements": int(len(dof)), "sources": len(srcs), "receivers": int(rec.size),
-           "samples": n_t, "segment_steps": int(np.ceil(np.sqrt(n_t)))}
+           "samples": n_t}
     grads = {}
     for prec in ("single", "double"):
         with bfe_gb300.Plan(K0, C0, M0, dt, bfe_gb300.VEL_CURRENT, prec, m["gl"]) as p:
@@ -783,6 +783,7 @@ def adjoint_section(torch, bfe_gb300, model, n_fd=20, n_t=4000):
             J, gs, gr = p.adjoint_gradient((ke, mh, ch, dof), t, srcs, sig, rec, obs)
             el = time.perf_counter() - t0
             kept = p.stats()["adjoint_kept"]
+            res["segment_steps"] = int(np.ceil(n_t / p.stats()["adjoint_segments"]))
         grads[prec] = (J, gs, gr)
         res["fp32" if prec == "single" else "fp64"] = {
             "gradient_s": el, "misfit": J,

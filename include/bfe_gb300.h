@@ -404,7 +404,8 @@ int bfe_adjoint_gradient(bfe_plan* plan, int64_t n_el, int32_t ndf, const int64_
 /* Counters of a plan's last run (no reference counterpart; used by the
  * benchmark for its roofline and launch-count figures). */
 typedef struct bfe_stats {
-  int64_t step_launches;     /* time-step kernel launches in the last run */
+  int64_t step_launches;     /* time-step kernel launches in the last run (a march that stays on
+                                the chip is one launch for up to 8,192 steps) */
   int64_t aux_launches;      /* interface / frame / conversion launches */
   double step_ms;            /* summed device time of the step kernels (timing on) */
   double aux_ms;             /* summed device time of the other launches (timing on) */
