@@ -419,8 +419,15 @@ int batched_candidates(int precision, int R, bool have_groups, int max_bs, int* 
       out[k++] = 3;
       out[k++] = 5;
     } else if (have_groups) {
+      // a slice kernel's warp with 28 or more of its 32 lanes busy loses less
+      // than the blocks' zeros cost on all-solid models, so it is the default
+      // there and the group form has to be clearly faster (us per step, slice /
+      // group: five sub-domains of 108,752 DOF R = 60 178.9 / 181.9, R = 28 91.3
+      // / 83.6; coupled 60,891 DOF R = 60 105.7 / 87.2, R = 29 59.2 / 51.5)
+      if (R % 32 >= 28) out[k++] = 0;
       out[k++] = 4;
       out[k++] = 5;
+      if (R % 32 >= 28) return k;
     }
     out[k++] = 0;
     return k;
