@@ -36,40 +36,49 @@ def _pair_lists(tx, rx, mon_nds_of_step, trans_nds, trans_wts):
     The rows of receiver b depend on the step only through its monitor list,
     which the steps of a capture share: they are looked up once per distinct
     list and receiver (64 instead of 4,096 look-ups for a 64-element capture,
-    which took 45 of the 52 ms of its time data) and gathered per pair."""
-    tx, rx = np.asarray(tx), np.asarray(rx)
-    for x in (tx, rx):
-        if x.ndim != 1 or (x.size and x.dtype.kind not in "iub"):
-            raise TypeError("tx and rx must be lists of integers")
-    m = min(tx.size, rx.size)
-    tx, rx = tx[:m].astype(np.int64), rx[:m].astype(np.int64)
-    lists, of_step = {}, {}
-    for a in np.unique(tx).tolist():
-        mon = np.asarray(mon_nds_of_step[a]).ravel()
-        of_step[a] = lists.setdefault((mon.dtype.str, mon.tobytes()), (len(lists), mon))[0]
-    which = np.asarray([of_step[a] for a in tx.tolist()], np.int64)
-    lo = int(rx.min()) if m else 0
-    n_rx = int(rx.max()) - lo + 1 if m else 1
-    key = which * n_rx + rx - lo
-    used, inverse = np.unique(key, return_inverse=True)
-    mons = [mon for _, mon in lists.values()]
-    sels, wts = [], []
-    for k in used.tolist():
-        b = k % n_rx + lo
-        sel = np.nonzero(np.isin(mons[k // n_rx], np.asarray(trans_nds[b]).ravel()))[0]
+    which took 45 of the 52 ms of its time data) and gathered per pair.
+    Integer lists go that way; anything else that names steps and receivers
+    (other keys of a dictionary, object arrays) is looked up pair by pair."""
+    def rows(mon, b):
+        sel = np.nonzero(np.isin(mon, np.asarray(trans_nds[b]).ravel()))[0]
         wt = np.ones(sel.size) if trans_wts is None or trans_wts[b] is None else \
             np.asarray(trans_wts[b], float).ravel()
         if wt.size != sel.size:
-            raise SolverError("receiver %d has %d weights for %d monitored nodes" % (b, wt.size, sel.size))
-        sels.append(sel)
-        wts.append(wt)
-    size = np.asarray([x.size for x in sels], np.int64)
+            raise SolverError("receiver %s has %d weights for %d monitored nodes" % (b, wt.size, sel.size))
+        return sel, wt
+
+    def integers(x):
+        try:
+            x = np.asarray(x)
+        except ValueError:                                # names of different lengths
+            return False
+        return x.ndim == 1 and (x.size == 0 or x.dtype.kind in "iu")
+
+    if not (integers(tx) and integers(rx)):
+        pairs = [rows(np.asarray(mon_nds_of_step[a]).ravel(), b) for a, b in zip(tx, rx)]
+        ptr_ = np.concatenate([[0], np.cumsum([sel.size for sel, _ in pairs])]).astype(np.int64)
+        return (ptr_, np.concatenate([sel for sel, _ in pairs] or [[]]).astype(np.int64),
+                np.concatenate([wt for _, wt in pairs] or [[]]).astype(float))
+    tx, rx = np.asarray(tx), np.asarray(rx)
+    m = min(tx.size, rx.size)
+    lists, of_step = {}, {}
+    steps, step = np.unique(tx[:m], return_inverse=True)
+    for a in steps.tolist():
+        mon = np.asarray(mon_nds_of_step[a]).ravel()
+        of_step[a] = lists.setdefault((mon.dtype.str, mon.tobytes()), (len(lists), mon))[0]
+    which = np.asarray([of_step[a] for a in steps.tolist()], np.int64)[step]
+    receivers, receiver = np.unique(rx[:m], return_inverse=True)
+    used, inverse = np.unique(which * receivers.size + receiver, return_inverse=True)
+    mons = [mon for _, mon in lists.values()]
+    names = receivers.tolist()
+    found = [rows(mons[k // len(names)], names[k % len(names)]) for k in used.tolist()]
+    size = np.asarray([sel.size for sel, _ in found], np.int64)
     start = np.cumsum(size) - size
     count = size[inverse]
     ptr_ = np.concatenate([[0], np.cumsum(count)]).astype(np.int64)
     at = np.repeat(start[inverse] - ptr_[:-1], count) + np.arange(ptr_[-1])
-    slot = np.concatenate(sels).astype(np.int64)[at] if sels else np.zeros(0, np.int64)
-    w = np.concatenate(wts).astype(float)[at] if wts else np.zeros(0)
+    slot = np.concatenate([sel for sel, _ in found]).astype(np.int64)[at] if found else np.zeros(0, np.int64)
+    w = np.concatenate([wt for _, wt in found]).astype(float)[at] if found else np.zeros(0)
     return ptr_, np.ascontiguousarray(slot), np.ascontiguousarray(w)
 
 
