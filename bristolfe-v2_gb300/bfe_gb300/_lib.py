@@ -37,6 +37,8 @@ BFE_FIELD_CURL = 3
 BFE_PREC_DOUBLE = 0
 BFE_PREC_SINGLE = 1
 BFE_PLAN_ONE_SOURCE = 1
+BFE_MARCH_FAULT_NONE = 0
+BFE_MARCH_FAULT_LAUNCH = 1
 
 I64 = ctypes.c_int64
 I32 = ctypes.c_int32
@@ -121,6 +123,7 @@ SIGNATURES = {
     "bfe_run_f64_noalloc": (I32, [I64, VP, VP, VP, VP, I64, I64, I64, VP, VP, VP, I64, VP, VP, VP]),
     "bfe_plan_set_timing": (I32, [VP, I32]),
     "bfe_plan_set_time_limit": (I32, [VP, ctypes.c_double]),
+    "bfe_plan_set_march_fault": (I32, [VP, I32]),
     "bfe_plan_stats": (I32, [VP, ctypes.POINTER(BfeStats)]),
     "bfe_last_error": (ctypes.c_char_p, []),
     "bfe_version": (I32, [PI32, PI32, PI32]),

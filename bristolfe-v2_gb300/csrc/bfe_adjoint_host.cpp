@@ -167,7 +167,8 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
       m.ti_step = dir;
       m.out = out + dir * k * (int64_t)sb;
       m.out_stride = dir * n * Rp;
-      if (bfe::launch_onchip_multi(o, a, m, prec, m_steps, fresh && k == 0, st) != cudaSuccess) {
+      if (refuse_piece(pl, k > 0) ||
+          bfe::launch_onchip_multi(o, a, m, prec, m_steps, fresh && k == 0, st) != cudaSuccess) {
         cudaGetLastError();
         return false;
       }

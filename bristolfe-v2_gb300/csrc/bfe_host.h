@@ -181,6 +181,7 @@ struct bfe_plan {
   int64_t n_direct_rows = 0;
   bool timing = false;
   double time_limit_s = 0.0;        // wall-clock limit of a run (0 = none)
+  int32_t march_fault = 0;          // BFE_MARCH_FAULT_*, for tests
   bfe_host::DevBuf<int> d_flag;     // non-finite flag of the last run, and a march's wait-ran-out flag
   bfe_stats last{};
   // autotuned batched-kernel variant per R (chosen on the first run with that R)
@@ -217,6 +218,10 @@ struct V5Lists {
   std::vector<double> kv, cv;
   bool corrections = false;        // rows coupled by C to a prescribed DOF
 };
+
+// Whether the launch of a later piece of an on-chip march is to be refused
+// (bfe_plan_set_march_fault).
+inline bool refuse_piece(const bfe_plan* pl, bool later) { return later && pl->march_fault == BFE_MARCH_FAULT_LAUNCH; }
 
 struct RunSpec {
   int64_t R = 1, n_t = 0, ti_start = 0;

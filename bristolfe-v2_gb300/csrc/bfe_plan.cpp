@@ -321,6 +321,13 @@ int bfe_plan_set_time_limit(bfe_plan* plan, double seconds) {
   return BFE_OK;
 }
 
+int bfe_plan_set_march_fault(bfe_plan* plan, int32_t fault) {
+  if (!plan) return fail(BFE_ERR_ARG, "plan is NULL");
+  if (fault < BFE_MARCH_FAULT_NONE || fault > BFE_MARCH_FAULT_LAUNCH) return fail(BFE_ERR_ARG, "unknown fault %d", fault);
+  plan->march_fault = fault;
+  return BFE_OK;
+}
+
 int bfe_plan_stats(const bfe_plan* plan, bfe_stats* out) {
   if (!plan || !out) return fail(BFE_ERR_ARG, "NULL argument");
   *out = plan->last;

@@ -190,7 +190,8 @@ int march_on_chip_multi(bfe_plan* pl, RunSpec& rs, bfe::StepArgs a, unsigned cha
     bfe::OnchipMulti m{};
     m.ti0 = ti;
     m.ti_step = 1;
-    if (bfe::launch_onchip_multi(o, a, m, pl->prec, k, ti == rs.ti_start, st) != cudaSuccess) {
+    if (refuse_piece(pl, ti > rs.ti_start) ||
+        bfe::launch_onchip_multi(o, a, m, pl->prec, k, ti == rs.ti_start, st) != cudaSuccess) {
       cudaGetLastError();
       CUDA_TRY(cudaStreamSynchronize(st));
       return BFE_OK;
@@ -274,7 +275,8 @@ int march_on_chip(bfe_plan* pl, RunSpec& rs, bfe::StepArgs a, unsigned char* con
     a.u_prev = U[prev];
     a.u_n = U[cur];
     a.u_new = U[next];
-    if (bfe::launch_onchip(o, a, q5, pl->prec, ti, k, ti == rs.ti_start, st) != cudaSuccess) {
+    if (refuse_piece(pl, ti > rs.ti_start) ||
+        bfe::launch_onchip(o, a, q5, pl->prec, ti, k, ti == rs.ti_start, st) != cudaSuccess) {
       cudaGetLastError();          // not launchable here
       CUDA_TRY(cudaStreamSynchronize(st));
       return BFE_OK;
@@ -290,7 +292,6 @@ int march_on_chip(bfe_plan* pl, RunSpec& rs, bfe::StepArgs a, unsigned char* con
   CUDA_TRY(cudaStreamSynchronize(st));
   if (gave_up) {                   // CTAs were not running together: march step by step
     pl->onchip->state = -1;
-    if (rs.v5) CUDA_TRY(cudaMemsetAsync(rs.d_ud[0], 0, 2 * rs.v5->n_slot * sizeof(double), st));
     return BFE_OK;
   }
   if (cur != 1)
@@ -450,8 +451,12 @@ int execute(bfe_plan* pl, RunSpec& rs, cudaStream_t st) {
     DevBuf<double> d_raw;
     const int rc1 = march_on_chip(pl, rs, a, U, frames, st, d_raw, on_chip);
     if (rc1) return rc1;
-    if (on_chip) iprev = 0, icur = 1, inew = 2;
-    else CUDA_TRY(cudaMemsetAsync(d_u.p, 0, 3 * state_bytes, st));
+    if (on_chip) {
+      iprev = 0, icur = 1, inew = 2;
+    } else {                       // from rest, whatever an abandoned march left
+      CUDA_TRY(cudaMemsetAsync(d_u.p, 0, 3 * state_bytes, st));
+      if (rs.v5) CUDA_TRY(cudaMemsetAsync(rs.d_ud[0], 0, 2 * rs.v5->n_slot * sizeof(double), st));
+    }
   }
   bool capturing = false;
   // One time step: step kernel, interface correction, optional frame, v5 rows.

@@ -436,6 +436,18 @@ int bfe_plan_set_timing(bfe_plan* plan, int32_t enable);
  */
 int bfe_plan_set_time_limit(bfe_plan* plan, double seconds);
 
+/*
+ * Fault injection on the host, for tests of what a run does when a march that
+ * stays on the chip cannot be finished there (no reference counterpart). Later
+ * runs on this plan meet the fault until it is set to BFE_MARCH_FAULT_NONE;
+ * they fall back to one launch per step and give the same results.
+ */
+enum {
+  BFE_MARCH_FAULT_NONE = 0,
+  BFE_MARCH_FAULT_LAUNCH = 1   /* the launch of a march's second piece of 8,192 steps is refused */
+};
+int bfe_plan_set_march_fault(bfe_plan* plan, int32_t fault);
+
 /* Copy the counters of the plan's last run. */
 int bfe_plan_stats(const bfe_plan* plan, bfe_stats* out);
 
