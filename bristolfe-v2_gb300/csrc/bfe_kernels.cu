@@ -448,6 +448,13 @@ int batched_candidates(int precision, int R, bool have_groups, int max_bs, int* 
   return k;
 }
 
+int settled_variant(int precision, int64_t R, bool have_groups, int max_bs) {
+  if (!have_groups) return 0;
+  if (precision == 0) return R % 16 ? 0 : R % 32 ? 3 : R % 64 ? 2 : 1;
+  if (max_bs <= 2 && (R % 64 == 0 || R == 16 || R == 32)) return 20;
+  return R % 64 ? 0 : 13;
+}
+
 // Prefetching pays where the three states do not fit in L2, so that a step's
 // first touch of a row is a DRAM miss in a node's chain of loads; below that
 // the requests are only extra work. Us per step without / with, FP32: coupled

@@ -310,7 +310,11 @@ int march_on_chip(bfe_plan* pl, RunSpec& rs, bfe::StepArgs a, unsigned char* con
 
 }  // namespace
 
-int execute(bfe_plan* pl, RunSpec& rs, cudaStream_t st) {
+namespace {
+
+// One march. settled: by the kernels whose outputs a non-finite march keeps
+// (execute); again is set when this march has to be made once more by them.
+int march(bfe_plan* pl, RunSpec& rs, TimeLimit& limit, bool settled, bool& again, cudaStream_t st) {
   const int64_t n = pl->n, R = rs.R;
   const int prec = pl->prec;
   const size_t es = elem_size(prec);
@@ -349,8 +353,6 @@ int execute(bfe_plan* pl, RunSpec& rs, cudaStream_t st) {
     ~EvGuard() { for (auto e : *a) cudaEventDestroy(e); for (auto e : *b) cudaEventDestroy(e); }
   } guard{&ev_step, &ev_aux};
   const bool timing = pl->timing;
-  TimeLimit limit;
-  CUDA_TRY(limit.start(pl->time_limit_s));
   // Autotuner: on the first batched run with a given operator shape and R,
   // time each candidate kernel (bfe::batched_candidates) on a few steps of
   // the real operator - the state is still zero, and the march that follows
@@ -364,12 +366,13 @@ int execute(bfe_plan* pl, RunSpec& rs, cudaStream_t st) {
   if (!pl->d_flag.p) CUDA_TRY(pl->d_flag.alloc(2));
   CUDA_TRY(cudaMemsetAsync(pl->d_flag.p, 0, 2 * sizeof(int), st));
   bool on_chip = false;
-  if (R > 1) {
+  if (R > 1 && !settled) {
     const int rc1 = march_on_chip_multi(pl, rs, a, U, st, on_chip);
     if (rc1) return rc1;
     if (!on_chip) CUDA_TRY(cudaMemsetAsync(pl->d_flag.p, 0, 2 * sizeof(int), st));
   }
   int variant = 0;
+  bool other_zeros = false;          // rows summed in another form than the settled kernel's
   const bfe::GroupArgs* grp = pl->have_groups ? &pl->groups : nullptr;
   if (R > 1 && !on_chip) {
     CUDA_TRY(cudaMemsetAsync(d_u.p, 0, 3 * state_bytes, st));
@@ -380,8 +383,9 @@ int execute(bfe_plan* pl, RunSpec& rs, cudaStream_t st) {
     const TuneKey key{pl->device, prec, max_bs, n, pl->nnz_operator, R};
     auto it = pl->variant_of_R.find(R);
     const char* force = getenv("BFE_VARIANT");
+    const int keep = bfe::settled_variant(prec, R, pl->have_groups, max_bs);
     bool cached = false;
-    if (!force && it == pl->variant_of_R.end()) {
+    if (!force && !settled && it == pl->variant_of_R.end()) {
       std::lock_guard<std::mutex> lock(g_tune_mutex);
       auto c = g_tune_cache.find(key);
       if (c != g_tune_cache.end()) {
@@ -392,6 +396,8 @@ int execute(bfe_plan* pl, RunSpec& rs, cudaStream_t st) {
     }
     if (force) {
       variant = atoi(force);
+    } else if (settled) {
+      variant = keep;
     } else if (it != pl->variant_of_R.end()) {
       variant = it->second;
     } else if (!cached && nc > 1 && rs.ti_start < rs.n_t) {
@@ -424,6 +430,7 @@ int execute(bfe_plan* pl, RunSpec& rs, cudaStream_t st) {
       std::lock_guard<std::mutex> lock(g_tune_mutex);
       g_tune_cache[key] = variant;
     }
+    other_zeros = !force && keep == 0 && variant != 0;
   }
   stt.variant = variant;
   int v5_flip = 0;
@@ -449,7 +456,7 @@ int execute(bfe_plan* pl, RunSpec& rs, cudaStream_t st) {
   // Element fields are reduced afterwards from raw frames kept on the device.
   if (R == 1) {
     DevBuf<double> d_raw;
-    const int rc1 = march_on_chip(pl, rs, a, U, frames, st, d_raw, on_chip);
+    const int rc1 = settled ? BFE_OK : march_on_chip(pl, rs, a, U, frames, st, d_raw, on_chip);
     if (rc1) return rc1;
     if (on_chip) {
       iprev = 0, icur = 1, inew = 2;
@@ -590,6 +597,10 @@ int execute(bfe_plan* pl, RunSpec& rs, cudaStream_t st) {
     stt.aux_ms += ms;
   }
   CUDA_TRY(cudaStreamSynchronize(st));
+  if (nonfinite && !settled && !limit.expired && (on_chip || other_zeros)) {
+    again = true;
+    return BFE_OK;
+  }
   if (nonfinite)
     return fail(BFE_ERR_UNSTABLE, "the march produced non-finite values by sample %lld of %lld (time step above "
                 "the stability limit, or non-finite forcing)", (long long)ti, (long long)rs.n_t);
@@ -597,6 +608,23 @@ int execute(bfe_plan* pl, RunSpec& rs, cudaStream_t st) {
     return fail(BFE_ERR_TIMEOUT, "the run exceeded its time limit of %g s: stopped after sample %lld of %lld",
                 limit.limit, (long long)ti, (long long)rs.n_t);
   return BFE_OK;
+}
+
+}  // namespace
+
+// A march, and once more if it became non-finite where rows are summed in
+// another form. Node blocks hold zeros for the entries a row lacks, and 0 x inf
+// is NaN: beside an infinite value, the marches on the chip and the any-R group
+// kernels give NaN where the row's own entries give an infinity or, in 5 of 1.2
+// million samples of a coupled run, a finite value. While the state is finite
+// both forms give the same bits, so only marches that end non-finite (their
+// outputs are returned with BFE_ERR_UNSTABLE) are made twice.
+int execute(bfe_plan* pl, RunSpec& rs, cudaStream_t st) {
+  TimeLimit limit;
+  CUDA_TRY(limit.start(pl->time_limit_s));
+  bool again = false;
+  const int rc = march(pl, rs, limit, false, again, st);
+  return rc == BFE_OK && again ? march(pl, rs, limit, true, again, st) : rc;
 }
 
 // Statuses after which a run's outputs are still copied to the caller.
