@@ -137,7 +137,8 @@ int group_max_bs(const GroupArgs& g);
 cudaError_t launch_step_batched(const StepArgs& a, const GroupArgs* gr, int precision, int max_slice_entries,
                                 int variant, cudaStream_t s);                         // any R
 size_t batched_smem_bytes(int precision, int max_slice_entries);
-cudaError_t set_batched_smem_limit(int precision, size_t smem);
+constexpr size_t kBatchedSmem = 227 * 1024;            // most that a slice's staged rows may take
+cudaError_t set_batched_smem_limit(int precision);
 cudaError_t launch_interface_fixup(const StepArgs& a, int precision, cudaStream_t s);
 // Sets *flag to 1 if any of the count values at u (FP64 for precision 0,
 // FP32 otherwise) is NaN or infinite; leaves it alone otherwise.
@@ -178,6 +179,14 @@ struct PackArgs {
 };
 cudaError_t launch_pack_count(const PackArgs& p, int precision, cudaStream_t s);
 cudaError_t launch_pack_write(const PackArgs& p, int precision, cudaStream_t s);
+
+// Shared memory a march's CTA may use, less a margin for the kernels' static
+// part, and the bitmap words of one that builds a partition. A function's
+// shared-memory limit belongs to the process: it is always set to the same
+// maximum, never to a plan's own need, which another thread with a larger plan
+// could find lowered between its setting and its launch.
+constexpr int kOnchipSmem = 232448 - 256;
+constexpr int kOnchipMaxWords = 50000;
 
 // One-source march that keeps state and operator on the chip (bfe_onchip.cu).
 // Device data of a plan's partition; the forcing, monitor and interface lists

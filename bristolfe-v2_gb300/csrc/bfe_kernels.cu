@@ -512,14 +512,15 @@ cudaError_t launch_step_batched(const StepArgs& a, const GroupArgs* gr, int prec
   return cudaGetLastError();
 }
 
-cudaError_t set_batched_smem_limit(int precision, size_t smem) {
+cudaError_t set_batched_smem_limit(int precision) {
+  const int smem = (int)kBatchedSmem;
   cudaError_t e;
   if (precision == 0) {
-    e = cudaFuncSetAttribute(step_batched<double, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = cudaFuncSetAttribute(step_batched<double, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   } else {
-    e = cudaFuncSetAttribute(step_batched<float, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = cudaFuncSetAttribute(step_batched<float, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(step_batched<float, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      e = cudaFuncSetAttribute(step_batched<float, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   }
   return e;
 }

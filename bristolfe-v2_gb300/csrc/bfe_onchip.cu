@@ -778,9 +778,13 @@ __global__ void __launch_bounds__(256) oc_reorder(OnchipReorder r) {
 
 template <typename T>
 cudaError_t build_t(const OnchipBuild& b, cudaStream_t st) {
-  const size_t words = (size_t)((b.max_words + kRankWords - 1) / kRankWords) * kRankWords;
-  const size_t smem = words * 4 + words / kRankWords * 4;
-  cudaError_t e = cudaFuncSetAttribute(oc_columns<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  auto smem_of = [](int max_words) {
+    const int words = (max_words + kRankWords - 1) / kRankWords * kRankWords;
+    return words * 4 + words / kRankWords * 4;
+  };
+  const int smem = smem_of(b.max_words);
+  cudaError_t e =
+      cudaFuncSetAttribute(oc_columns<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_of(kOnchipMaxWords));
   if (e != cudaSuccess) return e;
   oc_columns<T><<<b.n_parts, 1024, smem, st>>>(b);
   const int pairs = b.n_parts * b.n_parts;
@@ -793,7 +797,7 @@ template <typename T, bool INT, bool V5, int NT>
 cudaError_t launch_t(const OnchipArgs& o, const StepArgs& a, const V5Args& v, int64_t ti0, int64_t n_steps, int fresh,
                      cudaStream_t st) {
   auto* kern = march_onchip<T, INT, V5, NT>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, o.smem);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kOnchipSmem);
   if (e != cudaSuccess) return e;
   OnchipArgs oo = o;
   StepArgs aa = a;

@@ -7,8 +7,7 @@ using namespace bfe_host;
 
 namespace {
 
-// Shared memory a CTA may use, less a margin for the kernel's static part.
-constexpr int64_t kSmemLimit = 232448 - 256;
+constexpr int64_t kSmemLimit = bfe::kOnchipSmem;
 // Slices per part below which a part is not split further: one warp of rows
 // for each of an SM's four schedulers.
 constexpr int64_t kMinSlices = 4;
@@ -243,7 +242,7 @@ static int build_parts(bfe_plan* pl, std::unique_ptr<Onchip>& holder, const Part
   b.n = (int32_t)n;
   b.n_parts = (int32_t)P;
   b.max_part_slices = (int32_t)max_slices;
-  b.max_words = (int32_t)std::min<int64_t>((n + 31) / 32 + 1, 50000);
+  b.max_words = (int32_t)std::min<int64_t>((n + 31) / 32 + 1, bfe::kOnchipMaxWords);
   b.max_window = (int32_t)max_window;
   b.halo_cap = (int32_t)std::min<int64_t>(max_window, n + P);
   b.n_int = pl->n_int;

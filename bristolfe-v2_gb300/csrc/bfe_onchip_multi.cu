@@ -437,7 +437,7 @@ template <typename T>
 cudaError_t launch_t(const OnchipArgs& o, const StepArgs& a, const OnchipMulti& m, int64_t n_steps, int fresh,
                      cudaStream_t st) {
   auto* kern = march_onchip_multi<T>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, o.smem);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kOnchipSmem);
   if (e != cudaSuccess) return e;
   OnchipArgs oo = o;
   StepArgs aa = a;

@@ -114,8 +114,8 @@ int prepare_run(bfe_plan* pl, std::vector<ForceEntry>& frc, const std::vector<in
   if (pl->n_int) CUDA_TRY(ra.vint.alloc((size_t)pl->n_int * bfe::padded_sources(prec, R, pl->have_groups) * es));
   if (R > 1) {
     const size_t smem = bfe::batched_smem_bytes(prec, pl->max_slice_entries);
-    if (smem > 227 * 1024) return fail(BFE_ERR_UNSUPPORTED, "operator rows too long for the batched kernel");
-    CUDA_TRY(bfe::set_batched_smem_limit(prec, std::max<size_t>(smem, 1)));
+    if (smem > bfe::kBatchedSmem) return fail(BFE_ERR_UNSUPPORTED, "operator rows too long for the batched kernel");
+    CUDA_TRY(bfe::set_batched_smem_limit(prec));
   }
   a = bfe::StepArgs{};
   a.n = (int32_t)n;
