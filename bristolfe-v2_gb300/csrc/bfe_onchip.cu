@@ -186,14 +186,17 @@ __global__ void __launch_bounds__(NT, 1) march_onchip(OnchipArgs o, StepArgs a, 
   int64_t to_issue = 0;
   int waiting = 0, w_slot = 0, i_slot = 0;              // copies in flight, slot to read, slot to fill
   uint32_t w_parity = 0;
+  bool bad = false;                                     // a wait of this thread ran out
   if (stream)
     for (int j = warp; j < ns; j += nw)
       if (!(sd[j].y & kSlResident)) {
         const int kd = sl_kind(sd[j].y), cu = chunk_units<T>(kd);
         to_issue += max(1, (sl_units<T>(sd[j].y) + cu - 1) / cu) * n_steps;
       }
+  // Only lane 0 copies, and none after a wait of its own ran out: its counts
+  // are those of the copies in flight.
   auto issue = [&]() {
-    if (to_issue == 0) return;
+    if (to_issue == 0 || bad) return;
     while (sd[ij].y & kSlResident) {
       ij += nw;
       if (ij >= ns) ij = warp;
@@ -215,10 +218,12 @@ __global__ void __launch_bounds__(NT, 1) march_onchip(OnchipArgs o, StepArgs a, 
   for (int k = 0; k < o.depth && stream; ++k) issue();
   // the slot just read is free again: fill it, go on to the next
   auto next_slot = [&]() {
-    --waiting;
-    if (++w_slot == o.depth) {
-      w_slot = 0;
-      w_parity ^= 1;
+    if (!bad) {
+      --waiting;
+      if (++w_slot == o.depth) {
+        w_slot = 0;
+        w_parity ^= 1;
+      }
     }
     __syncwarp();
     issue();
@@ -298,7 +303,6 @@ __global__ void __launch_bounds__(NT, 1) march_onchip(OnchipArgs o, StepArgs a, 
   __syncthreads();
 
   uint32_t au = 0, bu = (uint32_t)(W * sizeof(T));      // byte offsets of u_n and of u_{n-1} / u_{n+1}
-  bool bad = false;
   for (int64_t k = 0; k <= n_steps; ++k) {
     const T* A = reinterpret_cast<const T*>(sm + au);
     T* B = reinterpret_cast<T*>(sm + bu);
@@ -379,25 +383,26 @@ __global__ void __launch_bounds__(NT, 1) march_onchip(OnchipArgs o, StepArgs a, 
       const unsigned char* blk = cache + d.x;
       if (!resident) {
         blk = ring + (warp * o.depth + w_slot) * o.slot_bytes;
-        bad |= !bar_wait(bars + warp * o.depth + w_slot, w_parity, o.err);
+        bad = bad || !bar_wait(bars + warp * o.depth + w_slot, w_parity, o.err);
       }
       const T rc = reinterpret_cast<const T*>(blk)[lane];
       blk += coef_bytes<T>();
       T acc = T(0);
+      // the indices of a chunk that did not come are not followed
       if (!(d.y & kSlChunks)) {
-        acc = row_sum(acc, blk, lane, kind, sl_width(d.y), sm, au, ref);
+        acc = row_sum(acc, blk, lane, kind, bad ? 0 : sl_width(d.y), sm, au, ref);
       } else {
         // FP64 counts entries (an odd last one is not paired), FP32 units
         const int cu = chunk_units<T>(kind), full = sizeof(T) == 8 ? 2 * cu : cu, step = units_bytes<T>(kind, cu);
         for (int left = sl_width(d.y);;) {
-          acc = row_sum(acc, blk, lane, kind, min(left, full), sm, au, ref);
+          acc = row_sum(acc, blk, lane, kind, bad ? 0 : min(left, full), sm, au, ref);
           left -= full;
           if (left <= 0) break;
           blk += step;
           if (!resident) {
             next_slot();
             blk = ring + (warp * o.depth + w_slot) * o.slot_bytes;
-            bad |= !bar_wait(bars + warp * o.depth + w_slot, w_parity, o.err);
+            bad = bad || !bar_wait(bars + warp * o.depth + w_slot, w_parity, o.err);
           }
         }
       }
@@ -434,7 +439,7 @@ __global__ void __launch_bounds__(NT, 1) march_onchip(OnchipArgs o, StepArgs a, 
     }
     if (k + 1 < n_steps) bad |= !receive(xu, hrow, H, hx, tag, B + rpad, tid, nt, o.err);
     if (__syncthreads_or(bad)) {
-      for (; waiting > 0; --waiting) {                  // no copy may outlive the CTA
+      for (; lane == 0 && waiting > 0; --waiting) {     // no copy may outlive the CTA
         if (!bar_wait(bars + warp * o.depth + w_slot, w_parity, o.err)) break;
         if (++w_slot == o.depth) {
           w_slot = 0;
