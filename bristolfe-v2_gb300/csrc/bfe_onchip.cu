@@ -16,7 +16,7 @@
 // gather is one shared-memory load.
 //
 // Exchange: after computing a row that others read, its owner writes the
-// value to a global buffer together with the step number, in one store per 4
+// value to a global buffer together with the step number, as 64-bit words of 4
 // bytes of value and 4 of step number; readers poll the value itself. One L2
 // round trip replaces data, fence, flag, poll, read. Two buffers by step
 // parity suffice: a CTA publishes step t + 2 only after it has read step

@@ -20,35 +20,38 @@ constexpr uint32_t kOcCut = 7, kOcMaxInt = 511;
 __device__ __forceinline__ bool is_slot(uint32_t f) { return !(f & kOcInterface) && (f >> kOcIntShift); }
 
 // ---------------------------------------------------------------------------
-// Exchange words: value and step number travel in the same 8 bytes.
+// Exchange words. 4 bytes of a value and the step number are the halves of one
+// 64-bit word, and every access is of whole 64-bit scalars (as .v2 where two
+// words lie side by side), which memory never tears: a reader that sees the
+// step number has the value too. Relaxed: nothing else is published by them.
+__device__ __forceinline__ uint64_t word(uint32_t v, uint32_t tag) { return (uint64_t)tag << 32 | v; }
+__device__ __forceinline__ void put_words(void* p, uint64_t a, uint64_t b) {
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1,%2};" ::"l"(p), "l"(a), "l"(b) : "memory");
+}
+__device__ __forceinline__ bool get_words(const void* p, uint32_t tag, uint32_t& lo, uint32_t& hi) {
+  uint64_t a, b;
+  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0,%1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+  lo = (uint32_t)a;
+  hi = (uint32_t)b;
+  return (uint32_t)(a >> 32) == tag && (uint32_t)(b >> 32) == tag;
+}
 __device__ __forceinline__ void xput(double* base, size_t i, double v, uint32_t tag) {
-  const uint32_t lo = (uint32_t)__double2loint(v), hi = (uint32_t)__double2hiint(v);
-  asm volatile("st.volatile.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(reinterpret_cast<uint4*>(base) + i), "r"(lo),
-               "r"(tag), "r"(hi), "r"(tag)
-               : "memory");
+  put_words(base + 2 * i, word((uint32_t)__double2loint(v), tag), word((uint32_t)__double2hiint(v), tag));
 }
 __device__ __forceinline__ void xput(float* base, size_t i, float v, uint32_t tag) {
-  asm volatile("st.volatile.global.v2.u32 [%0], {%1,%2};" ::"l"(reinterpret_cast<uint2*>(base) + i),
-               "r"(__float_as_uint(v)), "r"(tag)
-               : "memory");
+  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(base + 2 * i), "l"(word(__float_as_uint(v), tag)) : "memory");
 }
 __device__ __forceinline__ bool xtry(const double* base, size_t i, uint32_t tag, double& v) {
-  uint32_t a, b, c, d;
-  asm volatile("ld.volatile.global.v4.u32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(a), "=r"(b), "=r"(c), "=r"(d)
-               : "l"(reinterpret_cast<const uint4*>(base) + i)
-               : "memory");
-  v = __hiloint2double((int)c, (int)a);
-  return b == tag && d == tag;
+  uint32_t lo, hi;
+  const bool ok = get_words(base + 2 * i, tag, lo, hi);
+  v = __hiloint2double((int)hi, (int)lo);
+  return ok;
 }
 __device__ __forceinline__ bool xtry(const float* base, size_t i, uint32_t tag, float& v) {
-  uint32_t a, b;
-  asm volatile("ld.volatile.global.v2.u32 {%0,%1}, [%2];"
-               : "=r"(a), "=r"(b)
-               : "l"(reinterpret_cast<const uint2*>(base) + i)
-               : "memory");
-  v = __uint_as_float(a);
-  return b == tag;
+  uint64_t a;
+  asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(a) : "l"(base + 2 * i) : "memory");
+  v = __uint_as_float((uint32_t)a);
+  return (uint32_t)(a >> 32) == tag;
 }
 
 // About two seconds of the SM clock: far above any wait of a running march.

@@ -65,18 +65,16 @@ __device__ __forceinline__ float2 e_update(float2 acc, float2 ui, float2 up, flo
 
 // Exchange words of 16 bytes: an element, each half with the step number.
 __device__ __forceinline__ void wput(uint4* w, float2 v, uint32_t tag) {
-  asm volatile("st.volatile.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(w), "r"(__float_as_uint(v.x)), "r"(tag),
-               "r"(__float_as_uint(v.y)), "r"(tag)
-               : "memory");
+  put_words(w, word(__float_as_uint(v.x), tag), word(__float_as_uint(v.y), tag));
 }
 __device__ __forceinline__ void wput(uint4* w, double v, uint32_t tag) {
   xput(reinterpret_cast<double*>(w), 0, v, tag);
 }
 __device__ __forceinline__ bool wtry(const uint4* w, uint32_t tag, float2& v) {
-  uint32_t a, b, c, d;
-  asm volatile("ld.volatile.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "l"(w) : "memory");
-  v = make_float2(__uint_as_float(a), __uint_as_float(c));
-  return b == tag && d == tag;
+  uint32_t lo, hi;
+  const bool ok = get_words(w, tag, lo, hi);
+  v = make_float2(__uint_as_float(lo), __uint_as_float(hi));
+  return ok;
 }
 __device__ __forceinline__ bool wtry(const uint4* w, uint32_t tag, double& v) {
   return xtry(reinterpret_cast<const double*>(w), 0, tag, v);
