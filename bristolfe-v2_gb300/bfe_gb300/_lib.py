@@ -39,6 +39,8 @@ BFE_PREC_SINGLE = 1
 BFE_PLAN_ONE_SOURCE = 1
 BFE_MARCH_FAULT_NONE = 0
 BFE_MARCH_FAULT_LAUNCH = 1
+BFE_MARCH_FAULT_WAIT = 2
+BFE_MARCH_FAULT_MEMORY = 3
 
 I64 = ctypes.c_int64
 I32 = ctypes.c_int32
@@ -79,6 +81,11 @@ class BfeStats(ctypes.Structure):
                 ("nnz_padded", I64), ("n_interface", I64), ("n_direct_rows", I64),
                 ("variant", I64), ("n_nodes", I64), ("n_groups", I64), ("adjoint_segments", I64),
                 ("adjoint_kept", I64)]
+
+
+class BfeMarchInfo(ctypes.Structure):
+    """bfe_march_info: what a plan keeps for marches on the chip (bfe_plan_march_info)."""
+    _fields_ = [("partition_bytes", I64)]
 
 
 SIGNATURES = {
@@ -124,6 +131,7 @@ SIGNATURES = {
     "bfe_plan_set_timing": (I32, [VP, I32]),
     "bfe_plan_set_time_limit": (I32, [VP, ctypes.c_double]),
     "bfe_plan_set_march_fault": (I32, [VP, I32]),
+    "bfe_plan_march_info": (I32, [VP, ctypes.POINTER(BfeMarchInfo)]),
     "bfe_plan_stats": (I32, [VP, ctypes.POINTER(BfeStats)]),
     "bfe_last_error": (ctypes.c_char_p, []),
     "bfe_version": (I32, [PI32, PI32, PI32]),

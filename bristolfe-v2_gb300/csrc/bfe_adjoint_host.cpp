@@ -183,7 +183,8 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
     CUDA_TRY(cudaMemcpy(&e, pl->d_flag.p + 1, sizeof(int), cudaMemcpyDeviceToHost));
     yes = e != 0;
     if (yes) {
-      oc->state = -1;
+      onchip_give_up(pl, oc);
+      oc = nullptr;
       CUDA_TRY(cudaMemsetAsync(pl->d_flag.p, 0, 2 * sizeof(int), st));
     }
     return BFE_OK;
@@ -196,7 +197,7 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
   bfe::StepArgs afc = af;                           // the forward inputs as the chip's parts have them
   if (chip) onchip_multi_rows(*oc, frc, hidx, lf);
   chip = chip && onchip_multi_fit(pl, *oc, af, lf.frows, lf.mrows, false, st, of);
-  if (chip && (rc = onchip_multi_lists(pl, *oc, frc, lf, afc))) return rc;
+  if (chip && ((rc = onchip_multi_lists(pl, *oc, frc, lf, afc)) || (rc = onchip_meet_fault(pl, *oc)))) return rc;
   // With ckpt_every = 0, every forward state stays on the device when the
   // steps + 2 states and the adjoint's c + 2 segment slots fit in 3/4 of the
   // free memory: state u_t sits in slot t - ti0 + 2 of d_all (slots 0 and 1

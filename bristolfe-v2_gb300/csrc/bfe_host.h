@@ -143,6 +143,7 @@ struct Onchip {
   DevBuf<uint4> xchm;               // exchange words of marches with several sources
   std::vector<int32_t> halo_cnt;
   DevBuf<ushort4> lref;
+  int64_t device_bytes() const;
 };
 
 }  // namespace bfe_host
@@ -280,6 +281,11 @@ void onchip_multi_rows(const Onchip& oc, const std::vector<ForceEntry>& frc, con
                        MultiLists& L);
 int onchip_multi_lists(const bfe_plan* pl, const Onchip& oc, const std::vector<ForceEntry>& frc, MultiLists& L,
                        bfe::StepArgs& a);
+// Frees a partition whose march gave up (the stream is idle) and keeps the plan
+// from building it again.
+void onchip_give_up(bfe_plan* pl, const Onchip* oc);
+// BFE_MARCH_FAULT_WAIT: one row of the partition is published no more.
+int onchip_meet_fault(const bfe_plan* pl, Onchip& oc);
 // Whether that is worth building the partition for.
 bool onchip_multi_may_fit(const bfe_plan* pl, int64_t R, bool against_graph);
 // Step numbers for n steps that the exchange buffers do not hold yet.

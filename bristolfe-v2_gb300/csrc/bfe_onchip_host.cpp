@@ -179,10 +179,10 @@ static int64_t max_parts(int64_t slices) {
 }
 
 
-// Builds the partition of holder; parts already in part_slice are kept.
-static int build_parts(bfe_plan* pl, std::unique_ptr<Onchip>& holder, const PartView& view,
-                       const std::vector<uint32_t>& h_base, cudaStream_t st) {
-  Onchip& oc = *holder;
+// Builds the partition oc; parts already in part_slice are kept. Its state
+// becomes 1 when it fits.
+static int build_parts(bfe_plan* pl, Onchip& oc, const PartView& view, const std::vector<uint32_t>& h_base,
+                       cudaStream_t st) {
   const int64_t n = pl->n, S = pl->n_slices;
   const int prec = pl->prec;
   const int64_t es = (int64_t)elem_size(prec);
@@ -258,6 +258,7 @@ static int build_parts(bfe_plan* pl, std::unique_ptr<Onchip>& holder, const Part
   CUDA_TRY(oc.flags.alloc(n));
   CUDA_TRY(oc.order.alloc(S));
   CUDA_TRY(oc.blocks.alloc(off));
+  if (pl->march_fault == BFE_MARCH_FAULT_MEMORY) return fail(BFE_ERR_OOM, "no memory for a partition (injected)");
   if (prec == BFE_PREC_SINGLE) {
     CUDA_TRY(oc.lref.alloc(n));
     CUDA_TRY(base.upload(h_base));
@@ -326,11 +327,7 @@ static int build_parts(bfe_plan* pl, std::unique_ptr<Onchip>& holder, const Part
     max_halo = std::max<int64_t>(max_halo, cnt[p]);
     if (need > kSmemLimit || rp + cnt[p] > max_window) failed = true;
   }
-  if (failed) {
-    holder.reset(new Onchip());
-    holder->state = -1;
-    return BFE_OK;
-  }
+  if (failed) return BFE_OK;
   oc.op_bytes = obytes;
   oc.halo_cnt = cnt;
   bfe::OnchipArgs& o = oc.args;
@@ -365,17 +362,68 @@ static int build_parts(bfe_plan* pl, std::unique_ptr<Onchip>& holder, const Part
   return BFE_OK;
 }
 
+static void discard(std::unique_ptr<Onchip>& holder) {
+  holder.reset(new Onchip());
+  holder->state = -1;
+}
+
+void onchip_give_up(bfe_plan* pl, const Onchip* oc) {
+  for (auto* holder : {&pl->tiled, &pl->onchip})
+    if (holder->get() == oc) discard(*holder);
+}
+
+// Builds a partition once per plan. Nothing is kept of one that does not fit
+// or could not be built.
+template <typename Build>
+static int prepare(std::unique_ptr<Onchip>& holder, cudaStream_t st, Build&& build) {
+  if (holder->state) return BFE_OK;
+  int rc;
+  try {
+    rc = build();
+  } catch (const std::bad_alloc&) {
+    rc = fail(BFE_ERR_OOM, "host allocation failed while building a partition");
+  }
+  if (rc == BFE_OK && holder->state == 1) return BFE_OK;
+  if (rc) {
+    cudaStreamSynchronize(st);                         // work on the buffers about to go
+    cudaGetLastError();
+  }
+  discard(holder);
+  return rc;
+}
+
 int onchip_prepare(bfe_plan* pl, cudaStream_t st) {
-  if (pl->onchip->state) return BFE_OK;
-  pl->onchip->state = -1;
-  const PartView view{&pl->h_slice_ptr, pl->slice_ptr.p, pl->col.p, pl->val.p, pl->rowc.p};
-  return build_parts(pl, pl->onchip, view, pl->h_base, st);
+  return prepare(pl->onchip, st, [&] {
+    const PartView view{&pl->h_slice_ptr, pl->slice_ptr.p, pl->col.p, pl->val.p, pl->rowc.p};
+    return build_parts(pl, *pl->onchip, view, pl->h_base, st);
+  });
+}
+
+int64_t Onchip::device_bytes() const {
+  int64_t b = 0;
+  auto add = [&](const auto& d) { if (d.p) b += (int64_t)(d.n * sizeof(*d.p)); };
+  for (auto* d : {&d_part, &d_off, &d_word, &d_bytes, &d_cnt, &d_halo, &d_vptr, &d_vhalo, &row_of}) add(*d);
+  for (auto* d : {&flags, &order, &z_lcol}) add(*d);
+  for (auto* d : {&blocks, &xch, &xchv}) add(*d);
+  add(xchm);
+  add(lref);
+  return b;
+}
+
+int onchip_meet_fault(const bfe_plan* pl, Onchip& oc) {
+  if (pl->march_fault != BFE_MARCH_FAULT_WAIT) return BFE_OK;
+  std::vector<uint16_t> f(oc.flags.n);
+  CUDA_TRY(cudaMemcpy(f.data(), oc.flags.p, f.size() * sizeof(uint16_t), cudaMemcpyDeviceToHost));
+  auto it = std::find_if(f.begin(), f.end(), [](uint16_t x) { return x & 1; });     // bit 0: other parts read the row
+  if (it == f.end()) return BFE_OK;
+  *it &= (uint16_t)~1u;
+  CUDA_TRY(cudaMemcpy(oc.flags.p, f.data(), f.size() * sizeof(uint16_t), cudaMemcpyHostToDevice));
+  CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
+  return BFE_OK;
 }
 
 // The tiled partition, if the model has one.
-static int prepare_tiled(bfe_plan* pl, cudaStream_t st) {
-  if (pl->tiled->state) return BFE_OK;
-  pl->tiled->state = -1;
+static int build_tiled(bfe_plan* pl, cudaStream_t st) {
   Onchip& oc = *pl->tiled;
   const int64_t n = pl->n, S = pl->n_slices;
   std::vector<int32_t> perm;
@@ -412,20 +460,14 @@ static int prepare_tiled(bfe_plan* pl, cudaStream_t st) {
                        slice_ptr.p, col.p, val.p, rowc.p};
   CUDA_TRY(bfe::launch_onchip_reorder(r, pl->prec, st));
   const PartView view{&sp, slice_ptr.p, col.p, val.p, rowc.p};
-  return build_parts(pl, pl->tiled, view, base, st);     // synchronises before it returns
+  return build_parts(pl, oc, view, base, st);            // synchronises before it returns
 }
 
 Onchip* onchip_for_several(bfe_plan* pl, cudaStream_t st) {
-  for (auto* oc : {&pl->tiled, &pl->onchip}) {
-    if ((oc == &pl->tiled ? prepare_tiled(pl, st) : onchip_prepare(pl, st)) != BFE_OK) {
-      if ((*oc)->state == 0) (*oc)->state = -1;
-      cudaStreamSynchronize(st);
-      cudaGetLastError();
-      g_last_error.clear();
-    }
-    if ((*oc)->state == 1) return oc->get();
-  }
-  return nullptr;
+  if (prepare(pl->tiled, st, [&] { return build_tiled(pl, st); }) != BFE_OK) g_last_error.clear();
+  if (pl->tiled->state == 1) return pl->tiled.get();
+  if (onchip_prepare(pl, st) != BFE_OK) g_last_error.clear();
+  return pl->onchip->state == 1 ? pl->onchip.get() : nullptr;
 }
 
 bool onchip_fit(bfe_plan* pl, const std::vector<ForceEntry>& frc, const std::vector<int64_t>& v5_bytes,

@@ -323,8 +323,15 @@ int bfe_plan_set_time_limit(bfe_plan* plan, double seconds) {
 
 int bfe_plan_set_march_fault(bfe_plan* plan, int32_t fault) {
   if (!plan) return fail(BFE_ERR_ARG, "plan is NULL");
-  if (fault < BFE_MARCH_FAULT_NONE || fault > BFE_MARCH_FAULT_LAUNCH) return fail(BFE_ERR_ARG, "unknown fault %d", fault);
+  if (fault < BFE_MARCH_FAULT_NONE || fault > BFE_MARCH_FAULT_MEMORY) return fail(BFE_ERR_ARG, "unknown fault %d", fault);
   plan->march_fault = fault;
+  return BFE_OK;
+}
+
+int bfe_plan_march_info(const bfe_plan* plan, bfe_march_info* out) {
+  if (!plan || !out) return fail(BFE_ERR_ARG, "NULL argument");
+  *out = bfe_march_info{};
+  out->partition_bytes = plan->onchip->device_bytes() + plan->tiled->device_bytes();
   return BFE_OK;
 }
 

@@ -178,6 +178,7 @@ int march_on_chip_multi(bfe_plan* pl, RunSpec& rs, bfe::StepArgs a, unsigned cha
   onchip_multi_rows(*oc, rs.frc, rs.hist_idx, L);
   if (!onchip_multi_fit(pl, *oc, a, L.frows, L.mrows, true, st, o)) return BFE_OK;
   if (const int rc = onchip_multi_lists(pl, *oc, rs.frc, L, a)) return rc;
+  if (const int rc = onchip_meet_fault(pl, *oc)) return rc;
   o.err = pl->d_flag.p + 1;
   int prev = 2, cur = 0, next = 1;
   for (int64_t ti = rs.ti_start; ti < rs.n_t; ti += kOnchipLaunchSteps) {
@@ -203,7 +204,7 @@ int march_on_chip_multi(bfe_plan* pl, RunSpec& rs, bfe::StepArgs a, unsigned cha
   CUDA_TRY(cudaMemcpyAsync(&gave_up, o.err, sizeof(int), cudaMemcpyDeviceToHost, st));
   CUDA_TRY(cudaStreamSynchronize(st));
   if (gave_up) {
-    oc->state = -1;
+    onchip_give_up(pl, oc);
     return BFE_OK;
   }
   if (cur != 1)
@@ -227,7 +228,6 @@ int march_on_chip(bfe_plan* pl, RunSpec& rs, bfe::StepArgs a, unsigned char* con
   if (raw && pl->n * n_frames * (int64_t)sizeof(double) > kRawFrameBytes) return BFE_OK;
   if (onchip_prepare(pl, st) || (raw && d_raw.alloc((size_t)pl->n * n_frames) != cudaSuccess)) {
     // no memory for the partition or the raw frames: not an error of the run
-    if (pl->onchip->state == 0) pl->onchip->state = -1;
     cudaGetLastError();
     g_last_error.clear();
     return BFE_OK;
@@ -267,6 +267,7 @@ int march_on_chip(bfe_plan* pl, RunSpec& rs, bfe::StepArgs a, unsigned char* con
     a.dt = pl->dt;
   }
   int rct;
+  if ((rct = onchip_meet_fault(pl, *pl->onchip))) return rct;
   if ((rct = onchip_tags(*pl->onchip, rs.n_t, st, o.tag0))) return rct;
   o.err = pl->d_flag.p + 1;
   int prev = 2, cur = 0, next = 1;
@@ -291,7 +292,7 @@ int march_on_chip(bfe_plan* pl, RunSpec& rs, bfe::StepArgs a, unsigned char* con
   CUDA_TRY(cudaMemcpyAsync(&gave_up, o.err, sizeof(int), cudaMemcpyDeviceToHost, st));
   CUDA_TRY(cudaStreamSynchronize(st));
   if (gave_up) {                   // CTAs were not running together: march step by step
-    pl->onchip->state = -1;
+    onchip_give_up(pl, pl->onchip.get());
     return BFE_OK;
   }
   if (cur != 1)

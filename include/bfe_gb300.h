@@ -444,9 +444,18 @@ int bfe_plan_set_time_limit(bfe_plan* plan, double seconds);
  */
 enum {
   BFE_MARCH_FAULT_NONE = 0,
-  BFE_MARCH_FAULT_LAUNCH = 1   /* the launch of a march's second piece of 8,192 steps is refused */
+  BFE_MARCH_FAULT_LAUNCH = 1,  /* the launch of a march's second piece of 8,192 steps is refused */
+  BFE_MARCH_FAULT_WAIT = 2,    /* one value is never passed on: the waits for it run out (two seconds) */
+  BFE_MARCH_FAULT_MEMORY = 3   /* an allocation of the march's partition fails */
 };
 int bfe_plan_set_march_fault(bfe_plan* plan, int32_t fault);
+
+/* What a plan keeps for marches that stay on the chip (no reference
+ * counterpart). */
+typedef struct bfe_march_info {
+  int64_t partition_bytes;     /* device memory of its partitions of the operator */
+} bfe_march_info;
+int bfe_plan_march_info(const bfe_plan* plan, bfe_march_info* out);
 
 /* Copy the counters of the plan's last run. */
 int bfe_plan_stats(const bfe_plan* plan, bfe_stats* out);

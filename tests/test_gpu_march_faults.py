@@ -69,3 +69,83 @@ def test_v5_starts_again_from_rest_when_a_later_launch_is_refused(bfe, models, p
     monkeypatch.setenv("BFE_NO_GRAPH", "1")
     off, _ = _v5(bfe, m, prec, LONG, _lib.BFE_MARCH_FAULT_NONE)
     assert _same(on, off)
+
+
+def _info(bfe, plan):
+    import ctypes
+    from bfe_gb300 import _lib
+    info = _lib.BfeMarchInfo()
+    _lib.check(bfe.load().bfe_plan_march_info(plan._h, ctypes.byref(info)))
+    return info
+
+
+def _march(bfe, models, route, prec, nt, faults):
+    """Two runs of one plan, with the given faults: outputs, launches and what
+    is kept after each."""
+    from bfe_gb300 import model
+    name = dict(run="plate", coupled="coupled", brick="brick", v5="damped", batch="plate").get(route)
+    if route.startswith("adjoint"):
+        a = model.steel_plate_adjoint(W=2e-3, H=1e-3, h=0.1e-3, n_src=3, n_rec=4, abs_wavelengths=0.3)
+        t, s = modelgen.pulse(nt, a["dt"])
+        hi = model.global_indices(a["gl"], a["rec_nodes"], 2)
+        srcs = [model.global_indices(a["gl"], x, 2) for x in a["src_nodes"]]
+        obs = np.asfortranarray(np.broadcast_to(1e-13 * s[None, :, None], (hi.size, nt, 3)))
+        make = lambda: bfe.Plan(a["K"], a["C"], a["M"], a["dt"], bfe.VEL_CURRENT, prec, a["gl"])   # noqa: E731
+        every = dict(adjoint=0, adjoint_kept=0, adjoint_segments=nt - 100)[route]
+        go = lambda p: p.adjoint_gradient(a["element_data"], t, srcs, s, hi, obs, ckpt_every=every,  # noqa: E731
+                                          return_history=True)[1:]
+    else:
+        m, dof = models[name]
+        t, s = modelgen.pulse(nt, m["dt"])
+        fi = modelgen.gi_of(m["gl"], [m["frc_nd"]], dof)
+        n = m["K"].shape[0]
+        hi = np.arange(1, n + 1, 7)
+        make = lambda: bfe.Plan(m["K"], m["C"], m["M"], m["dt"], bfe.V5 if route == "v5" else bfe.VEL_CURRENT,  # noqa: E731
+                                prec, m["gl"], one_source=route != "batch")
+        srcs = [fi, fi + 2, np.array([1]), np.array([n])]
+        di = modelgen.gi_of(m["gl"], np.nonzero(np.isclose(m["mod"]["nds"][:, 0], 0.0))[0] + 1, 2) if route == "v5" else None
+        go = (lambda p: (p.run_batched(t, srcs, s, hi),)) if route == "batch" else \
+            (lambda p: p.run_v5(t, fi, s, di, 1e-9 * np.outer(np.linspace(0.5, 1.0, di.size), s), hi, nt // 9)[:3]) \
+            if route == "v5" else (lambda p: p.run(t, fi, s, hi, nt // 9, True)[:2])
+    out = []
+    with make() as plan:
+        for f in faults:
+            _fault(bfe, plan, f)
+            r = go(plan)
+            out.append((r, plan.stats()["step_launches"], _info(bfe, plan)))
+    return out
+
+
+ROUTES = ["run", "coupled", "brick", "v5", "batch", "adjoint", "adjoint_segments"]
+
+
+@pytest.mark.parametrize("fault", ["BFE_MARCH_FAULT_WAIT", "BFE_MARCH_FAULT_MEMORY"])
+@pytest.mark.parametrize("route,prec", [(r, "single") for r in ROUTES] + [("run", "double"), ("batch", "double")])
+def test_given_up_marches_step_and_keep_nothing(bfe, models, route, prec, fault, monkeypatch):
+    """A wait that runs out, and no memory for the partition: the same bits
+    from step kernels, no partition kept, and none built for the next run."""
+    from bfe_gb300 import _lib
+    monkeypatch.delenv("BFE_NO_GRAPH", raising=False)
+    nt = 400
+    (sane, _, info), = _march(bfe, models, route, prec, nt, [0])
+    assert info.partition_bytes > 0
+    for r, launches, info in _march(bfe, models, route, prec, nt, [getattr(_lib, fault), 0]):
+        assert info.partition_bytes == 0
+        assert launches >= nt
+        assert _same(r, sane)
+
+
+@pytest.mark.parametrize("fault", [0, 1])
+@pytest.mark.parametrize("route,prec", [("run", "double"), ("run", "single"), ("coupled", "single"), ("brick", "single"),
+                                        ("v5", "double"), ("batch", "double"), ("batch", "single"),
+                                        ("adjoint_kept", "single"), ("adjoint_segments", "single")])
+def test_marches_of_more_than_one_launch(bfe, models, route, prec, fault, monkeypatch):
+    """More samples than one launch marches: the second goes on from the states,
+    frames, histories and velocities of the first, or is refused."""
+    monkeypatch.delenv("BFE_NO_GRAPH", raising=False)
+    (on, launches, _), = _march(bfe, models, route, prec, LONG, [fault])
+    forward = LONG if route == "adjoint_segments" else 0           # checkpoints are made step by step
+    assert launches < forward + 300 if fault == 0 else launches > forward + LONG - 100
+    monkeypatch.setenv("BFE_NO_GRAPH", "1")
+    (off, _, _), = _march(bfe, models, route, prec, LONG, [0])
+    assert _same(on, off)
