@@ -85,7 +85,7 @@ class BfeStats(ctypes.Structure):
 
 class BfeMarchInfo(ctypes.Structure):
     """bfe_march_info: what a plan keeps for marches on the chip (bfe_plan_march_info)."""
-    _fields_ = [("partition_bytes", I64)]
+    _fields_ = [("partition_bytes", I64), ("partitions_built", I64)]
 
 
 SIGNATURES = {

@@ -183,6 +183,7 @@ struct bfe_plan {
   bool timing = false;
   double time_limit_s = 0.0;        // wall-clock limit of a run (0 = none)
   int32_t march_fault = 0;          // BFE_MARCH_FAULT_*, for tests
+  int64_t partitions_built = 0;     // on-chip partitions begun
   bfe_host::DevBuf<int> d_flag;     // non-finite flag of the last run, and a march's wait-ran-out flag
   bfe_stats last{};
   // autotuned batched-kernel variant per R (chosen on the first run with that R)

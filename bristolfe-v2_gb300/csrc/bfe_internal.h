@@ -270,6 +270,7 @@ struct OnchipReorder {
 };
 cudaError_t launch_onchip_reorder(const OnchipReorder& r, int precision, cudaStream_t s);
 int onchip_block_bound(int precision, int width);    // most bytes of a slice of this width
+int onchip_block_least(int width, int dofs);         // FP32: least, with nodes of up to so many DOFs
 cudaError_t launch_onchip_build(const OnchipBuild& b, int precision, cudaStream_t s);
 // n_steps steps from ti0. fresh: from rest, else from a.u_n, a.u_prev. The
 // newest state is written to a.u_new, the one before it to a.u_prev. v: the

@@ -818,6 +818,15 @@ int onchip_block_bound(int precision, int width) {
   return precision == 0 ? block_bound<double>(width) : block_bound<float>(width);
 }
 
+int onchip_block_least(int width, int dofs) {
+  int least = block_bytes<float>(1, slice_units(1, width));
+  for (int kind = 2; kind <= dofs; ++kind) {
+    const int b = block_bytes<float>(kind, (width + kind - 1) / kind);
+    if (b < least) least = b;
+  }
+  return least;
+}
+
 cudaError_t launch_onchip_reorder(const OnchipReorder& r, int precision, cudaStream_t st) {
   const int blocks = (r.n_slices * 32 + 255) / 256;
   if (precision == 0) oc_reorder<double><<<blocks, 256, 0, st>>>(r);

@@ -332,6 +332,7 @@ int bfe_plan_march_info(const bfe_plan* plan, bfe_march_info* out) {
   if (!plan || !out) return fail(BFE_ERR_ARG, "NULL argument");
   *out = bfe_march_info{};
   out->partition_bytes = plan->onchip->device_bytes() + plan->tiled->device_bytes();
+  out->partitions_built = plan->partitions_built;
   return BFE_OK;
 }
 

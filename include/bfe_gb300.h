@@ -454,6 +454,7 @@ int bfe_plan_set_march_fault(bfe_plan* plan, int32_t fault);
  * counterpart). */
 typedef struct bfe_march_info {
   int64_t partition_bytes;     /* device memory of its partitions of the operator */
+  int64_t partitions_built;    /* partitions it began to build, used or not */
 } bfe_march_info;
 int bfe_plan_march_info(const bfe_plan* plan, bfe_march_info* out);
 

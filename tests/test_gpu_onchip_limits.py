@@ -1,0 +1,46 @@
+"""Models that the on-chip marches leave to the step kernels: nothing is built
+for them."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import modelgen
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def bfe():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    from bfe_gb300 import build
+    build.build()
+    import bfe_gb300
+    bfe_gb300.load()
+    return bfe_gb300
+
+
+def _first_run(bfe, m, prec, nt, R=1):
+    from bfe_gb300 import _lib
+    t, s = modelgen.pulse(nt, m["dt"])
+    s[0] = 1e-3
+    n = m["K"].shape[0]
+    with bfe.Plan(m["K"], m["C"], m["M"], m["dt"], bfe.VEL_CURRENT, prec, m["gl"], one_source=R == 1) as plan:
+        if R == 1:
+            plan.run(t, [n // 2], s, [1, n])
+        else:
+            plan.run_batched(t, [np.array([n // 2 + r]) for r in range(R)], s, [1, n])
+        info = _lib.BfeMarchInfo()
+        _lib.check(bfe.load().bfe_plan_march_info(plan._h, ctypes.byref(info)))
+        return plan.stats()["step_launches"], info
+
+
+@pytest.mark.parametrize("prec", ["double", "single"])
+def test_operators_over_the_limit(bfe, prec):
+    """444,000 DOF in 3D: blocks of 330 MB in FP64 and at least 150 MB in FP32."""
+    from bfe_gb300 import model
+    launches, info = _first_run(bfe, model.steel_block_3d(13e-3, 13e-3, 6.6e-3, 0.2e-3, n_mon=4), prec, 400)
+    assert launches == 400
+    assert info.partitions_built == 0 and info.partition_bytes == 0
