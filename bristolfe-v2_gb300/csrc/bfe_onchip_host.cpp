@@ -19,6 +19,15 @@ constexpr int64_t kMinSlices = 4;
 // 492,579 DOF (52 MB) took 14.2 against 19.3.
 constexpr int64_t kMaxOperator = (int64_t)96 << 20, kMaxOperator64 = (int64_t)88 << 20;
 
+// FP32 rows of many entries (3D) whose blocks alone exceed the SMs' shared
+// memory (35 MB) stream too much of them: the step kernel is faster as long as
+// its operator, 8 bytes an entry, comes from L2. Us per step on chip / step
+// kernels, bricks: 73,872 DOF (blocks of 24 MB) 6.6 / 10.9, 100,800 DOF (34) 7.7
+// / 11.5, 105,903 DOF (35.4) 11.9 / 11.1, 122,034 DOF (39; 65 MB of entries) 12.6
+// / 11.2, 133,584 DOF (76 MB) 13.1 / 14.5, 202,878 DOF 14.7 / 29.0. Rows of a few
+// entries gain either way: coupled 961,641 DOF (50 MB) 10.8 / 17.
+constexpr int64_t kStepOperator = (int64_t)70 << 20, kWideRow = 32;
+
 inline int64_t align2(int64_t x) { return (x + 1) & ~(int64_t)1; }
 
 // Lists of the interface correction: which interface values each part reads
@@ -255,6 +264,9 @@ static int build_parts(bfe_plan* pl, Onchip& oc, const PartView& view, const std
   if (prec == BFE_PREC_DOUBLE && off > kMaxOperator64) return BFE_OK;
   if (prec == BFE_PREC_SINGLE && off > kMaxOperator && least_operator(sp, h_base) > kMaxOperator) return BFE_OK;
   if (max_slices * bfe::kSlice > max_window) return BFE_OK;
+  if (prec == BFE_PREC_SINGLE && off > P * kSmemLimit && sp[S] >= n * kWideRow && (int64_t)sp[S] * 8 <= kStepOperator &&
+      least_operator(sp, h_base) > P * kSmemLimit)
+    return BFE_OK;
   InterfaceLists L;
   if (pl->n_int && !interface_lists(pl, oc.part_slice, L)) return BFE_OK;
 

@@ -44,3 +44,13 @@ def test_operators_over_the_limit(bfe, prec):
     launches, info = _first_run(bfe, model.steel_block_3d(13e-3, 13e-3, 6.6e-3, 0.2e-3, n_mon=4), prec, 400)
     assert launches == 400
     assert info.partitions_built == 0 and info.partition_bytes == 0
+
+
+@pytest.mark.parametrize("side,kept", [(7.0e-3, True), (8.0e-3, False), (8.4e-3, False), (9.0e-3, True)])
+def test_bricks_that_stream_only_where_that_is_faster(bfe, side, kept):
+    """73,872 DOF fit in the SMs' shared memory, 152,352 stream against a step
+    kernel that is out of L2; between them the step kernel is faster."""
+    from bfe_gb300 import model
+    launches, info = _first_run(bfe, model.steel_block_3d(side, side, side / 2, 0.2e-3, n_mon=4), "single", 400)
+    assert launches == (1 if kept else 400)
+    assert info.partitions_built == (1 if kept else 0) and (info.partition_bytes > 0) == kept
