@@ -183,19 +183,13 @@ static int64_t most_sources(int prec, bool against_graph) {
   return !against_graph ? 16 : prec == BFE_PREC_DOUBLE ? 8 : 64;
 }
 
-// Least bytes of an FP32 operator's blocks: every slice in the smallest form
-// its rows' node blocks allow, no node short of entries.
-static int64_t least_operator(const std::vector<int32_t>& sp, const std::vector<uint32_t>& base) {
-  const int64_t n = (int64_t)base.size(), S = (int64_t)sp.size() - 1;
+// Least bytes of an FP32 operator's blocks, from the slices' widths alone: every
+// slice in the smallest form (3D rows: three entries a node, else two), no node
+// short of entries.
+static int64_t least_operator(const std::vector<int32_t>& sp, bool wide) {
   int64_t total = 0;
-  for (int64_t s = 0; s < S; ++s) {
-    int most = 3;                                      // DOFs of a node that one index may serve
-    for (int64_t i = s * bfe::kSlice; i < std::min(n, (s + 1) * bfe::kSlice); ++i) {
-      const int64_t b = base[i];
-      while (most > 1 && (b + most > n || base[b + most - 1] != (uint32_t)b)) --most;
-    }
-    total += bfe::onchip_block_least((sp[s + 1] - sp[s]) / bfe::kSlice, most);
-  }
+  for (size_t s = 0; s + 1 < sp.size(); ++s)
+    total += bfe::onchip_block_least((sp[s + 1] - sp[s]) / bfe::kSlice, wide ? 3 : 2);
   return total;
 }
 
@@ -258,14 +252,15 @@ static int build_parts(bfe_plan* pl, Onchip& oc, const PartView& view, const std
     off += bfe::onchip_block_bound(prec, (sp[s + 1] - sp[s]) / bfe::kSlice);
     if (off / 16 > INT32_MAX) return BFE_OK;
   }
+  const bool wide = sp[S] >= n * kWideRow;
   // What cannot fit is not built: blocks, halo lists and exchange words of a
   // 1,560,753-DOF brick in FP32 cost 3.4 ms of a plan's first run. FP64 sizes
   // are exact.
   if (prec == BFE_PREC_DOUBLE && off > kMaxOperator64) return BFE_OK;
-  if (prec == BFE_PREC_SINGLE && off > kMaxOperator && least_operator(sp, h_base) > kMaxOperator) return BFE_OK;
+  if (prec == BFE_PREC_SINGLE && off > kMaxOperator && least_operator(sp, wide) > kMaxOperator) return BFE_OK;
   if (max_slices * bfe::kSlice > max_window) return BFE_OK;
-  if (prec == BFE_PREC_SINGLE && off > P * kSmemLimit && sp[S] >= n * kWideRow && (int64_t)sp[S] * 8 <= kStepOperator &&
-      least_operator(sp, h_base) > P * kSmemLimit)
+  if (prec == BFE_PREC_SINGLE && off > P * kSmemLimit && wide && (int64_t)sp[S] * 8 <= kStepOperator &&
+      least_operator(sp, wide) > P * kSmemLimit)
     return BFE_OK;
   InterfaceLists L;
   if (pl->n_int && !interface_lists(pl, oc.part_slice, L)) return BFE_OK;
