@@ -184,6 +184,7 @@ struct bfe_plan {
   double time_limit_s = 0.0;        // wall-clock limit of a run (0 = none)
   int32_t march_fault = 0;          // BFE_MARCH_FAULT_*, for tests
   int64_t partitions_built = 0;     // on-chip partitions begun
+  int64_t steps_marched = 0;        // towards the first (onchip_due)
   bfe_host::DevBuf<int> d_flag;     // non-finite flag of the last run, and a march's wait-ran-out flag
   bfe_stats last{};
   // autotuned batched-kernel variant per R (chosen on the first run with that R)
@@ -287,6 +288,9 @@ int onchip_multi_lists(const bfe_plan* pl, const Onchip& oc, const std::vector<F
 void onchip_give_up(bfe_plan* pl, const Onchip* oc);
 // BFE_MARCH_FAULT_WAIT: one row of the partition is published no more.
 int onchip_meet_fault(const bfe_plan* pl, Onchip& oc);
+// Whether the plan has decided about its partition, or has marched enough steps
+// with these to build it.
+bool onchip_due(bfe_plan* pl, int64_t steps, bool several);
 // Whether that is worth building the partition for.
 bool onchip_multi_may_fit(const bfe_plan* pl, int64_t R, bool against_graph);
 // Step numbers for n steps that the exchange buffers do not hold yet.

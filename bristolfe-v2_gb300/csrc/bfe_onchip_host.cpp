@@ -51,16 +51,16 @@ bool interface_lists(const bfe_plan* pl, const std::vector<int32_t>& part, Inter
     for (int32_t t = L.first[p]; t < L.first[p + 1]; ++t) owner[t] = p;
   std::vector<std::vector<int32_t>> need(P);
   std::vector<char> adj((size_t)P * P, 0);
+  std::vector<int32_t> at(ni, -1);   // the last part that noted a column, later its local number there
   for (int p = 0; p < P; ++p) {
-    for (int32_t t = L.first[p]; t < L.first[p + 1]; ++t)
-      for (int32_t e = pl->h_z_ptr[t]; e < pl->h_z_ptr[t + 1]; ++e) {
-        const int32_t c = pl->h_z_col[e];
-        if (owner[c] == p) continue;
-        need[p].push_back(c);
-        adj[(size_t)p * P + owner[c]] = 1;
-      }
+    for (int32_t e = pl->h_z_ptr[L.first[p]]; e < pl->h_z_ptr[L.first[p + 1]]; ++e) {
+      const int32_t c = pl->h_z_col[e];
+      if (owner[c] == p || at[c] == p) continue;
+      at[c] = p;
+      need[p].push_back(c);
+      adj[(size_t)p * P + owner[c]] = 1;
+    }
     std::sort(need[p].begin(), need[p].end());
-    need[p].erase(std::unique(need[p].begin(), need[p].end()), need[p].end());
   }
   std::vector<size_t> real(P);
   for (int p = 0; p < P; ++p) real[p] = need[p].size();
@@ -76,12 +76,11 @@ bool interface_lists(const bfe_plan* pl, const std::vector<int32_t>& part, Inter
     L.ptr.push_back((int32_t)L.list.size());
     const int32_t own = L.first[p + 1] - L.first[p];
     if (own + (int64_t)need[p].size() > 65535) return false;
-    const auto b = need[p].begin(), r = b + real[p];
-    for (int32_t t = L.first[p]; t < L.first[p + 1]; ++t)
-      for (int32_t e = pl->h_z_ptr[t]; e < pl->h_z_ptr[t + 1]; ++e) {
-        const int32_t c = pl->h_z_col[e];
-        L.z_lcol[e] = (uint16_t)(owner[c] == p ? c - L.first[p] : own + (int32_t)(std::lower_bound(b, r, c) - b));
-      }
+    for (size_t k = 0; k < real[p]; ++k) at[need[p][k]] = own + (int32_t)k;
+    for (int32_t e = pl->h_z_ptr[L.first[p]]; e < pl->h_z_ptr[L.first[p + 1]]; ++e) {
+      const int32_t c = pl->h_z_col[e];
+      L.z_lcol[e] = (uint16_t)(owner[c] == p ? c - L.first[p] : at[c]);
+    }
   }
   return true;
 }
@@ -496,6 +495,23 @@ Onchip* onchip_for_several(bfe_plan* pl, cudaStream_t st) {
   if (pl->tiled->state == 1) return pl->tiled.get();
   if (onchip_prepare(pl, st) != BFE_OK) g_last_error.clear();
   return pl->onchip->state == 1 ? pl->onchip.get() : nullptr;
+}
+
+// Steps a plan marches before its partition is built: about as many as win back
+// what that costs, so that a plan of one short run does not pay for it and one
+// of many short runs soon has it. One source: 0.3 to 1.4 ms, for 2 to 5 us a
+// step and 0.3 ms a run (no graph). Samples at which a first run breaks even:
+// plate of 161,202 DOF FP32 115, coupled 241,579 DOF FP64 165, 961,641 DOF FP32
+// 215 (96 samples there: 3.28 ms on the chip, 2.71 in steps). Several sources:
+// 0.6 ms at 10,000 DOF, 1.0 at 40,602, 1.5 at 90,902, for 3.4 to 5.7 us a step:
+// 40,602 DOF R = 16 breaks even at 200 samples, 90,902 DOF R = 4 at 270. Rows of
+// many entries (3D) gain up to 30 us a step and break even below 96.
+bool onchip_due(bfe_plan* pl, int64_t steps, bool several) {
+  if (pl->onchip->state || (several && pl->tiled->state)) return true;
+  pl->steps_marched += steps;
+  const int64_t n = pl->n;
+  const bool wide = pl->h_slice_ptr.back() >= n * kWideRow;
+  return pl->steps_marched >= (wide ? 0 : several ? 70 + n / 350 : 80 + n / 4500);
 }
 
 bool onchip_fit(bfe_plan* pl, const std::vector<ForceEntry>& frc, const std::vector<int64_t>& v5_bytes,

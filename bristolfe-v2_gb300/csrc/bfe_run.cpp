@@ -156,8 +156,9 @@ int prepare_run(bfe_plan* pl, std::vector<ForceEntry>& frc, const std::vector<in
 
 namespace {
 
-// Steps below which a run is not worth the partition's setup, and steps of
-// one launch (bounds how long one kernel runs).
+// Steps below which a run takes the step kernels in any case (onchip_due has the
+// rule for the first runs of a plan), and steps of one launch (bounds how long
+// one kernel runs).
 constexpr int64_t kOnchipMinSteps = 96, kOnchipLaunchSteps = 8192;
 // Device memory for raw frames that an element field is reduced from.
 constexpr int64_t kRawFrameBytes = (int64_t)1 << 31;
@@ -170,7 +171,7 @@ int march_on_chip_multi(bfe_plan* pl, RunSpec& rs, bfe::StepArgs a, unsigned cha
   if (pl->timing || pl->time_limit_s > 0.0 || steps < kOnchipMinSteps || rs.n_t >= ((int64_t)1 << 30) || pl->n_int ||
       getenv("BFE_NO_GRAPH") || getenv("BFE_VARIANT"))
     return BFE_OK;
-  if (!onchip_multi_may_fit(pl, a.R, true)) return BFE_OK;
+  if (!onchip_multi_may_fit(pl, a.R, true) || !onchip_due(pl, steps, true)) return BFE_OK;
   Onchip* oc = onchip_for_several(pl, st);
   if (!oc) return BFE_OK;
   MultiLists L;
@@ -226,6 +227,7 @@ int march_on_chip(bfe_plan* pl, RunSpec& rs, bfe::StepArgs a, unsigned char* con
   const int64_t n_frames = frames ? (rs.n_t + rs.every_n - 1) / rs.every_n : 0;
   const bool raw = frames && rs.field;
   if (raw && pl->n * n_frames * (int64_t)sizeof(double) > kRawFrameBytes) return BFE_OK;
+  if (!onchip_due(pl, steps, false)) return BFE_OK;
   if (onchip_prepare(pl, st) || (raw && d_raw.alloc((size_t)pl->n * n_frames) != cudaSuccess)) {
     // no memory for the partition or the raw frames: not an error of the run
     cudaGetLastError();

@@ -54,3 +54,23 @@ def test_bricks_that_stream_only_where_that_is_faster(bfe, side, kept):
     launches, info = _first_run(bfe, model.steel_block_3d(side, side, side / 2, 0.2e-3, n_mon=4), "single", 400)
     assert launches == (1 if kept else 400)
     assert info.partitions_built == (1 if kept else 0) and (info.partition_bytes > 0) == kept
+
+
+@pytest.mark.parametrize("R", [1, 4])
+def test_short_runs_build_once_it_pays(bfe, R):
+    """The first 100 samples of a plan of 40,602 DOF and four sources, and of one
+    of 161,202 DOF and one, take the step kernels, later ones the chip."""
+    from bfe_gb300 import model
+    m = model.steel_plate(20e-3, 10e-3, 0.1e-3, 16) if R > 1 else model.steel_plate(40e-3, 20e-3, 0.1e-3, 16)
+    t, s = modelgen.pulse(100, m["dt"])
+    s[0] = 1e-3
+    n = m["K"].shape[0]
+    launches, out = [], []
+    with bfe.Plan(m["K"], m["C"], m["M"], m["dt"], bfe.VEL_CURRENT, "double", m["gl"], one_source=R == 1) as plan:
+        for _ in range(4):
+            out.append(plan.run(t, [n // 2], s, [n // 2, n])[0] if R == 1 else
+                       plan.run_batched(t, [np.array([n // 2 + r]) for r in range(R)], s, [n // 2, n]))
+            launches.append(plan.stats()["step_launches"])
+    assert launches == [100, 1, 1, 1]
+    for x in out[1:]:
+        assert np.abs(x).max() > 0 and np.array_equal(x, out[0])

@@ -30,7 +30,7 @@ def test_marches_on_three_threads(bfe, R, monkeypatch):
     jobs = []
     for W, H in ((1e-3, 0.6e-3), (9e-3, 6e-3), (0.4e-3, 0.3e-3)):
         m = modelgen.solid_plate(W=W, H=H, h=0.1e-3)
-        t, s = modelgen.pulse(100, m["dt"])
+        t, s = modelgen.pulse(160, m["dt"])
         n = m["K"].shape[0]
         srcs = [np.array([1 + (7 * r) % n]) for r in range(R)]
         plan = bfe.Plan(m["K"], m["C"], m["M"], m["dt"], bfe.VEL_CURRENT, "single", m["gl"], one_source=R == 1)
