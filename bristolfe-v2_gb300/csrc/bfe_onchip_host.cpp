@@ -97,6 +97,29 @@ struct PartView {
   const void *val, *rowc;
 };
 
+// How P parts of S slices are cut from M mesh columns of len nodes: px strips of
+// py parts, and the halo nodes of the largest. A row costs about twice what a
+// halo row does. py = 1: tiles are not worth it.
+struct TileCut {
+  int64_t px, py, halo;
+};
+TileCut tile_cut(int64_t S, int64_t P, int64_t M, double len, int64_t bs) {
+  auto halo = [&](int64_t px, int64_t py) {
+    const double w = (double)M / (double)px, h = len / (double)py;
+    return (px > 1 ? 2 * h : 0) + (py > 1 ? 2 * w : 0) + 4;
+  };
+  auto cost = [&](int64_t px, int64_t py) {
+    return (double)((S + px * py - 1) / (px * py) * bfe::kSlice) + 0.5 * halo(px, py) * (double)bs;
+  };
+  int64_t px = P, py = 1;
+  for (int64_t x = 1; x <= std::min(P, M); ++x)
+    for (int64_t y = 1; x * y <= P && y <= (int64_t)len; ++y)
+      if (cost(x, y) < cost(px, py)) px = x, py = y;
+  if (cost(px, py) > 0.9 * cost(P, 1)) px = P, py = 1;
+  const int64_t w = (M + px - 1) / px, h = (int64_t)std::ceil(len / (double)py);
+  return {px, py, (px > 1 ? 2 * h : 0) + (py > 1 ? 2 * w : 0) + 4};
+}
+
 // Tiles for a 2D model. Contiguous ranges of the caller's node order (column
 // by column) are strips of a mesh column or two when a part is small, and then
 // all of their rows are read by other parts. Here the nodes are put in an
@@ -137,18 +160,9 @@ bool tile_order(const bfe_plan* pl, int64_t P, std::vector<int32_t>& perm, std::
       break;
     }
   }
-  // px strips of py parts: a row costs about twice what a halo row does
-  const double len = (double)N / (double)M;
-  auto cost = [&](int64_t px, int64_t py) {
-    const double w = (double)M / (double)px, h = len / (double)py;
-    const double halo = (px > 1 ? 2 * h : 0) + (py > 1 ? 2 * w : 0) + 4;
-    return (double)((S + px * py - 1) / (px * py) * bfe::kSlice) + 0.5 * halo * (double)bs;
-  };
-  int64_t px = P, py = 1;
-  for (int64_t x = 1; x <= std::min(P, M); ++x)
-    for (int64_t y = 1; x * y <= P && y <= (int64_t)len; ++y)
-      if (cost(x, y) < cost(px, py)) px = x, py = y;
-  if (py == 1 || cost(px, py) > 0.9 * cost(P, 1)) return false;
+  const TileCut cut = tile_cut(S, P, M, (double)N / (double)M, bs);
+  const int64_t px = cut.px, py = cut.py;
+  if (py == 1) return false;
   perm.resize(pl->n);
   parts.assign(1, 0);
   std::vector<int32_t> first, node;
@@ -620,10 +634,40 @@ int onchip_v5(bfe_plan* pl, const V5Lists& L, OnchipV5& d, bool& fits) {
   return BFE_OK;
 }
 
+// Whether the exchange of so many halo rows takes longer than a step from a graph
+// (the figures are in onchip_multi_fit).
+static bool too_many_words(int prec, int64_t R, int64_t halo) {
+  return halo * (prec == BFE_PREC_DOUBLE ? R : R / 2) > 3300 && R > (prec == BFE_PREC_DOUBLE ? 4 : 8);
+}
+
 bool onchip_multi_may_fit(const bfe_plan* pl, int64_t R, bool against_graph) {
   if (pl->n_int || R < 2 || R > most_sources(pl->prec, against_graph) || R % bfe::onchip_multi_rv(pl->prec)) return false;
   // the states alone must fit in the SMs' shared memory
-  return 2 * (double)pl->n * (double)R * (double)elem_size(pl->prec) <= (double)kSmemLimit * bfe::sm_count();
+  const int64_t es = (int64_t)elem_size(pl->prec);
+  if (2 * (double)pl->n * (double)R * (double)es > (double)kSmemLimit * bfe::sm_count()) return false;
+  // On a 2D model whose tiles are not cut yet, what onchip_multi_fit would
+  // find: tiles cost 1 to 2 ms, and 161,202 DOF, R = 16 had them cut in vain in
+  // every plan's first run (3.1 -> 5.3 ms for 200 samples). A mesh column is as
+  // long as a node in the middle is far from its last neighbour, and other nodes
+  // have as many neighbours.
+  const auto& g = pl->groups;
+  if (pl->tiled->state || !pl->have_groups || g.n_groups != 1 || g.bs[0] > 2 || (int64_t)g.n_nodes[0] * g.bs[0] != pl->n)
+    return true;
+  const int64_t bs = g.bs[0], N = g.n_nodes[0], q = N / 2, S = pl->n_slices, P = max_parts(S);
+  // (a part of a few rows fits with twice its rows as halo)
+  const int64_t most = 3 * ((S + P - 1) / P) * bfe::kSlice;
+  if (2 * R * most * es <= kSmemLimit / 2 && !(against_graph && too_many_words(pl->prec, R, most))) return true;
+  int32_t at[2] = {0, 0}, last = 0;
+  if (cudaMemcpy(at, pl->g_nptr[0].p + q, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost) != cudaSuccess || at[1] <= at[0] ||
+      cudaMemcpy(&last, pl->g_nrow[0].p + at[1] - 1, sizeof(int32_t), cudaMemcpyDeviceToHost) != cudaSuccess)
+    return true;
+  const int64_t len = std::max<int64_t>(1, last / bs - q), M = (N + len - 1) / len;
+  const TileCut cut = tile_cut(S, P, M, (double)len, bs);
+  const int64_t rows = (S + cut.px * cut.py - 1) / (cut.px * cut.py) * bfe::kSlice, halo = cut.halo * bs;
+  const int width = es == 8 ? (int)(pl->h_slice_ptr[S] / (S * bfe::kSlice)) : (at[1] - at[0]) * (int)bs;
+  const int64_t block = es == 8 ? bfe::onchip_block_bound(pl->prec, width) : bfe::onchip_block_least(width, (int)bs);
+  return 2 * R * (rows + halo) * es + 6 * rows + 4 * halo + rows / bfe::kSlice * block <= kSmemLimit &&
+         !(against_graph && too_many_words(pl->prec, R, halo));
 }
 
 void onchip_multi_rows(const Onchip& oc, const std::vector<ForceEntry>& frc, const std::vector<int64_t>& hist_idx,
@@ -703,7 +747,7 @@ bool onchip_multi_fit(bfe_plan* pl, Onchip& oc, const bfe::StepArgs& a, const st
   // 40,602 DOF R = 16 9.3 / 9.1 (3,232 words), R = 32 14.1 / 9.9. One launch
   // per step, which the adjoint would make, is slower wherever this fits up to
   // R = 16 (17 us per step of 90,902 DOF, R = 16, against 7.5).
-  if (against_graph && words > 3300 && R > (es == 8 ? 4 : 8)) return false;
+  if (against_graph && too_many_words(pl->prec, R, words / wpr)) return false;
   const int64_t turns = (tasks + 31) / 32, warps = (tasks + turns - 1) / turns;
   o.threads = (int32_t)std::max<int64_t>({128, warps * 32, std::min<int64_t>(1024, (words / 4 + 31) / 32 * 32)});
   for (int p = 0; p < P; ++p)

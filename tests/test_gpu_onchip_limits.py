@@ -74,3 +74,15 @@ def test_short_runs_build_once_it_pays(bfe, R):
     assert launches == [100, 1, 1, 1]
     for x in out[1:]:
         assert np.abs(x).max() > 0 and np.array_equal(x, out[0])
+
+
+@pytest.mark.parametrize("W,H,R,kept", [(20e-3, 10e-3, 48, True), (20e-3, 10e-3, 64, False), (30e-3, 15e-3, 24, True),
+                                        (30e-3, 15e-3, 36, False), (40e-3, 20e-3, 12, True), (40e-3, 20e-3, 16, False),
+                                        (200e-3, 2e-3, 24, True)])
+def test_tiles_are_cut_only_for_source_counts_that_fit(bfe, W, H, R, kept):
+    """Plates of 40,602, 90,902 and 161,202 DOF on both sides of what fits, and a
+    thin one, whose parts have few neighbours."""
+    from bfe_gb300 import model
+    launches, info = _first_run(bfe, model.steel_plate(W, H, 0.1e-3, 16), "single", 700, R)
+    assert (launches == 1) == kept
+    assert info.partitions_built == (1 if kept else 0)
