@@ -97,7 +97,8 @@ __global__ void __launch_bounds__(256, MINB) step_f32_group2(StepArgs a, GroupAr
 // FP64 group block-sparse kernel (direct form, the reference's arithmetic):
 // u_new = sum over the node's blocks (its own included) of B_block u_n
 // + D u_{n-1} + forcing, summed in column order like the one-source kernel.
-// LPN lanes per node, VEC doubles (right-hand sides) per lane and pass.
+// LPN lanes per node, VEC doubles (right-hand sides) per lane and pass; UNROLL
+// neighbours in flight (0: the compiler's choice).
 template <int BS, int VEC, int UNROLL>
 __device__ __forceinline__ void group64_node(const StepArgs& a, const GroupArgs& gr, int gi, int node,
                                              int c0, int stride) {
@@ -114,8 +115,7 @@ __device__ __forceinline__ void group64_node(const StepArgs& a, const GroupArgs&
     for (int k = 0; k < BS; ++k)
 #pragma unroll
       for (int v = 0; v < VEC; ++v) acc[k][v] = 0.0;
-#pragma unroll UNROLL
-    for (int e = p0; e < p1; ++e) {
+    auto add = [&](int e) {
       const double* nb = un + (size_t)__ldg(nrow + e) * rs + c;
       double g[BS][VEC];
 #pragma unroll
@@ -135,6 +135,12 @@ __device__ __forceinline__ void group64_node(const StepArgs& a, const GroupArgs&
         for (int k = 0; k < BS; ++k)
 #pragma unroll
           for (int v = 0; v < VEC; ++v) acc[k][v] = fma(cv[k * BS + l], g[l][v], acc[k][v]);
+    };
+    if constexpr (UNROLL == 0) {
+      for (int e = p0; e < p1; ++e) add(e);
+    } else {
+#pragma unroll UNROLL
+      for (int e = p0; e < p1; ++e) add(e);
     }
     double* unew = static_cast<double*>(a.u_new);
     const double* upv = static_cast<const double*>(a.u_prev);
@@ -173,7 +179,7 @@ __device__ __forceinline__ void group64_node(const StepArgs& a, const GroupArgs&
   }
 }
 
-template <int LPN, int VEC, int MINB, int MAXBS, int UNROLL = 1>
+template <int LPN, int VEC, int MINB, int MAXBS, int UNROLL = 0>
 __global__ void __launch_bounds__(128, MINB) step_f64_group(StepArgs a, GroupArgs gr) {
   const int b = blockIdx.x;
   int gi = 0;
@@ -196,7 +202,11 @@ __global__ void __launch_bounds__(128, MINB) step_f64_group(StepArgs a, GroupArg
 // (us per step, slice kernel / variant 4: coupled 241,579 DOF R = 5 154.5 /
 // 35.1, R = 21 157.5 / 111.5; the FP64 pipe bounds both). Skipping the absent
 // entries of a block (one in seven) by a branch made variant 1 slower, 359 us
-// against 272 at R = 64.
+// against 272 at R = 64. One neighbour at a time suits variants 1 and 2 on 2D
+// nodes (us per step with the compiler's choice / one: coupled 241,579 DOF R = 64
+// 286.4 / 283.2); variant 3 and 3D nodes want the compiler's choice (bricks of
+// 14,553 DOF R = 48 100.9 / 102.5, R = 64 129.8 / 131.7, plate of 40,602 DOF R = 48
+// 57.7 / 58.4).
 static cudaError_t launch_group64(const StepArgs& a, const GroupArgs& gr, int variant, cudaStream_t st) {
   const int pairs = a.R / 2, passes = (pairs + 15) / 16;
   const int lpn = variant >= 4 ? (pairs + passes - 1) / passes : variant == 3 ? 8 : 16;
@@ -211,16 +221,16 @@ static cudaError_t launch_group64(const StepArgs& a, const GroupArgs& gr, int va
   int maxbs = 1;
   for (int k = 0; k < g.n_groups; ++k) maxbs = g.bs[k] > maxbs ? g.bs[k] : maxbs;
   if (maxbs <= 2) {
-    if (variant == 1) step_f64_group<16, 4, 8, 2><<<blocks, 128, 0, st>>>(a, g);
-    else if (variant == 2) step_f64_group<16, 2, 10, 2><<<blocks, 128, 0, st>>>(a, g);
+    if (variant == 1) step_f64_group<16, 4, 8, 2, 1><<<blocks, 128, 0, st>>>(a, g);
+    else if (variant == 2) step_f64_group<16, 2, 10, 2, 1><<<blocks, 128, 0, st>>>(a, g);
     else if (variant == 3) step_f64_group<8, 2, 10, 2><<<blocks, 128, 0, st>>>(a, g);
-    else if (variant == 4) step_f64_group<0, 2, 8, 2><<<blocks, 128, 0, st>>>(a, g);
+    else if (variant == 4) step_f64_group<0, 2, 8, 2, 1><<<blocks, 128, 0, st>>>(a, g);
     else step_f64_group<0, 2, 6, 2, 2><<<blocks, 128, 0, st>>>(a, g);
   } else {
     if (variant == 1) step_f64_group<16, 4, 6, 3><<<blocks, 128, 0, st>>>(a, g);
     else if (variant == 2) step_f64_group<16, 2, 8, 3><<<blocks, 128, 0, st>>>(a, g);
     else if (variant == 3) step_f64_group<8, 2, 8, 3><<<blocks, 128, 0, st>>>(a, g);
-    else if (variant == 4) step_f64_group<0, 2, 6, 3><<<blocks, 128, 0, st>>>(a, g);
+    else if (variant == 4) step_f64_group<0, 2, 6, 3, 1><<<blocks, 128, 0, st>>>(a, g);
     else step_f64_group<0, 2, 4, 3, 2><<<blocks, 128, 0, st>>>(a, g);
   }
   return cudaGetLastError();

@@ -360,8 +360,9 @@ int march(bfe_plan* pl, RunSpec& rs, TimeLimit& limit, bool settled, bool& again
   // time each candidate kernel (bfe::batched_candidates) on a few steps of
   // the real operator - the state is still zero, and the march that follows
   // starts from rest again - and keep the fastest. The default (first)
-  // candidate stays unless another is at least 3 % faster, so that near-ties
-  // do not flip between runs. The choice is kept in the plan and for the
+  // candidate stays unless another is at least 2 % faster, so that near-ties
+  // do not flip between runs (3 % kept the FP64 group kernel on all-solid plates
+  // of 161,202 DOF, R = 64, where the slice kernel takes 255.3 us of 261.0). The choice is kept in the plan and for the
   // process (g_tune_cache). BFE_VARIANT=<k> forces variant k (sweeps).
   auto launch_batched = [&](const bfe::GroupArgs* grpp, int v) -> cudaError_t {
     return bfe::launch_step_batched(a, grpp, prec, pl->max_slice_entries, v, st);
@@ -425,7 +426,7 @@ int march(bfe_plan* pl, RunSpec& rs, TimeLimit& limit, bool settled, bool& again
         if (k == 0) t_default = ms;
         if (ms < best) { best = ms; variant = v; }
       }
-      if (best > 0.97f * t_default) variant = cand[0];
+      if (best > 0.98f * t_default) variant = cand[0];
       cudaEventDestroy(e0);
       cudaEventDestroy(e1);
       CUDA_TRY(cudaMemsetAsync(d_u.p, 0, 3 * state_bytes, st));
