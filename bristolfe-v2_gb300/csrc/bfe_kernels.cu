@@ -406,8 +406,8 @@ size_t batched_smem_bytes(int precision, int max_slice_entries) {
 //   24 - 26  the float4 form for any R and block size, one, two or four
 //            neighbours in flight
 //   9 - 14   packed warp-per-node kernel step_f32_group2 (unroll 1, 2, 4;
-//            occupancy hints 4, 6, 8 CTAs): 3-DOF node blocks (3D), R a
-//            multiple of 64
+//            occupancy hints 4, 6, 8 CTAs), R a multiple of 64: only when forced,
+//            slower than 24 - 26 on every model
 // The first candidate is the default; the autotuner keeps it unless another
 // is clearly faster on the live operator.
 int batched_candidates(int precision, int R, bool have_groups, int max_bs, int* out) {
@@ -436,10 +436,9 @@ int batched_candidates(int precision, int R, bool have_groups, int max_bs, int* 
     for (int v : {20, 22}) out[k++] = v;
     return k;
   }
-  if (have_groups && R % 64 == 0) {
-    for (int v : {24, 25, 13, 9}) out[k++] = v;
-    return k;
-  }
+  // (3D nodes too, us per step of 24 / 25 / 26 and the best of 9 - 14: bricks R = 64
+  // of 14,553 DOF 23.2 / 22.2 / 18.5, 21.1; 46,128 DOF 36.5 / 37.0 / 34.4, 45.6;
+  // 202,878 DOF 123.8 / 139.8 / 135.8, 195.8)
   if (have_groups) {
     for (int v : {24, 25, 26}) out[k++] = v;
     return k;
