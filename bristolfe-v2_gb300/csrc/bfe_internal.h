@@ -417,17 +417,20 @@ void set_last_error(const char* msg);
 int exception_status() noexcept;
 
 // Number of SMs of the current device (queried once per device, thread-safe).
-inline int sm_count() {
+template <cudaDeviceAttr ATTR>
+inline int device_attribute() {
   static std::atomic<int> cache[64];
   int dev = 0;
   cudaGetDevice(&dev);
   int c = (dev >= 0 && dev < 64) ? cache[dev].load(std::memory_order_relaxed) : 0;
   if (c == 0) {
-    cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&c, ATTR, dev);
     if (dev >= 0 && dev < 64) cache[dev].store(c, std::memory_order_relaxed);
   }
   return c;
 }
+inline int sm_count() { return device_attribute<cudaDevAttrMultiProcessorCount>(); }
+inline int l2_bytes() { return device_attribute<cudaDevAttrL2CacheSize>(); }
 
 // True the first time it is called for the current device with this flag
 // set (for per-device, per-function attributes; thread-safe).

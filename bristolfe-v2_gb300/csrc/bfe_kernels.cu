@@ -457,25 +457,31 @@ int settled_variant(int precision, int64_t R, bool have_groups, int max_bs) {
 // Prefetching pays where the three states do not fit in L2, so that a step's
 // first touch of a row is a DRAM miss in a node's chain of loads; below that
 // the requests are only extra work. Us per step without / with, FP32: coupled
-// 961,641 DOF R = 16 65.7 / 63.4, R = 32 107.2 / 97.9, R = 64 166.7 / 150.0,
-// R = 128 299.8 / 270.1; bricks of 1,778,478 DOF R = 8 268.2 / 258.7, R = 24
-// 571.9 / 534.8, of 202,878 R = 64 132.1 / 121.4; states of 139 to 186 MB gain
-// 1 to 10 %. Where it loses: fewer than 16 right-hand sides of one- and two-DOF
-// nodes (R = 8, 2,674,573 DOF: 96.8 / 98.4: a request costs as much as the
-// load), several uneven passes over R (R = 96, 241,579 DOF: 82.0 / 84.7), and
-// it does nothing for FP64, which the FP64 pipe bounds (R = 64 271.2 / 272.4).
-// The distance is long enough for a DRAM miss and short enough that the data
-// are still in L2: 800 of 1,824 resident CTAs (400: 156.7, 1,200: 150.6, 2,000:
-// 161 at R = 64); the wide blocks of three-DOF nodes want 200 (R = 16,
-// 1,778,478 DOF: 363 us, 400: 379, 800: 429).
+// 961,641 DOF R = 16 65.7 / 63.4, R = 32 107.2 / 97.9, R = 64 166.7 / 150.0; bricks
+// of 1,778,478 DOF R = 8 268.2 / 258.7, R = 24 571.9 / 534.8, of 202,878 R = 64
+// 132.4 / 120.3, R = 256 453.5 / 443.3; states of 139 to 186 MB gain 1 to 10 %.
+// Where it loses: fewer than 16 right-hand sides of one- and two-DOF nodes
+// (R = 8, 2,674,573 DOF: 96.8 / 98.4: a request costs as much as the load),
+// several uneven passes over R (R = 96, 241,579 DOF: 91.6 / 93.4), and it does
+// nothing for FP64, which the FP64 pipe bounds (R = 64 271.2 / 272.4). The
+// distance is long enough for a DRAM miss and short enough that the data are
+// still in L2: 800 CTAs of 1,824 resident (400: 156.7, 1,200: 150.6, 2,000: 161 at
+// R = 64); the wide blocks of three-DOF nodes want 200 (R = 16, 1,778,478 DOF: 363
+// us, 400: 379, 800: 429).
+// Above 64 right-hand sides a CTA's rows are as many times larger, and the
+// distance shorter. None / 400 / 800: R = 128 plate of 161,202 DOF 61.3 / 61.5 /
+// 63.0, coupled 241,579 DOF 101.5 / 98.8 / 102.8, 961,641 DOF 325 / 295 / 296; R = 192
+// 161,202 DOF (371 MB of states) 90.8 / 94.4 / 100.1, 241,579 DOF (557 MB) 141.2 /
+// 139.0 / 144.4, plate of 1,003,002 DOF 514 / 464 / 527. R = 256 none / 200 / 800:
+// plate of 361,802 DOF (1.1 GB) 238.4 / 239.6 / 274.4, 961,641 DOF 644 / 600 / 641.
+// R = 320 only loses (361,802 DOF 295.5 / 306.5 at 200; bricks of 46,128 DOF 157.6 /
+// 161.6).
 int group_ahead(const StepArgs& a, const GroupArgs& g) {
-  int dev = 0, l2 = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess)
-    return 0;
-  if (3 * (size_t)a.n * (size_t)a.R * sizeof(float) <= (size_t)l2) return 0;
-  if (a.R > 64 && a.R % 64 != 0) return 0;
-  const bool wide = group_max_bs(g) > 2;
-  return a.R < (wide ? 8 : 16) ? 0 : wide ? 200 : 800;
+  const size_t state = 3 * (size_t)a.n * (size_t)a.R * sizeof(float), l2 = (size_t)l2_bytes();
+  if (l2 == 0 || state <= l2 || (a.R > 64 && a.R % 64 != 0) || a.R > 256) return 0;
+  if (group_max_bs(g) > 2) return a.R < 8 ? 0 : 200;
+  if (a.R <= 128) return a.R < 16 ? 0 : a.R <= 64 ? 800 : 400;
+  return a.R == 192 ? (state >= 4 * l2 ? 400 : 0) : (state >= 12 * l2 ? 200 : 0);
 }
 
 int group_max_bs(const GroupArgs& g) {
