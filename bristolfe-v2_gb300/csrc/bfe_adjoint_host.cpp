@@ -121,12 +121,10 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
   if ((rc = prepare_run(pl, frc, hidx, R, n_t, n_sig, d_sig.p, d_hist.p, st, rf, af))) return rc;
   const int64_t Rp = af.R;           // right-hand sides of the states, padding included
   const bfe::GroupArgs* grp = pl->have_groups ? &pl->groups : nullptr;
-  // the variant the forward runs chose for this R, else the default candidate
+  // the variant the forward runs chose for this R, else the usual best
   int variant = 0;
   if (R > 1) {
-    int cand[8];
-    bfe::batched_candidates(prec, (int)Rp, pl->have_groups, grp ? bfe::group_max_bs(*grp) : 0, cand);
-    variant = cand[0];
+    variant = bfe::untimed_candidate(prec, (int)Rp, (int)n, pl->have_groups, grp ? bfe::group_max_bs(*grp) : 1);
     auto it = pl->variant_of_R.find(R);
     if (it != pl->variant_of_R.end()) variant = it->second;
   }

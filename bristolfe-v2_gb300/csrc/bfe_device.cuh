@@ -34,6 +34,29 @@ __device__ __forceinline__ T forcing_sum(const StepArgs& a, int i, int r) {
   return f;
 }
 
+// The same for N consecutive right-hand sides from r0, in one pass over the
+// row's entries, which are sorted by right-hand side. A receiver of the adjoint
+// is forced in every source, and a pass for each right-hand side of a lane was a
+// chain of loads that a step waits for: 6,642 DOF FP32 R = 24, 600 samples 24.2 ->
+// 21.1 ms. (In the FP64 group kernels it costs registers: coupled 241,579 DOF R =
+// 64 281 -> 309 us per step.)
+template <typename T, int N>
+__device__ __forceinline__ void forcing_sums(const StepArgs& a, int i, int r0, T (&f)[N]) {
+  const T* coef = static_cast<const T*>(a.frc_coef);
+  const T* sig = static_cast<const T*>(a.sig) + (size_t)step_index(a) * a.n_sig;
+#pragma unroll
+  for (int j = 0; j < N; ++j) f[j] = T(0);
+  for (int e = lower_bound_i32(a.frc_row, a.n_frc, i); e < a.n_frc && __ldg(a.frc_row + e) == i; ++e) {
+    const int k = __ldg(a.frc_rhs + e) - r0;
+    if (k >= N) break;
+    if (k < 0) continue;
+    const T c = __ldg(coef + e), s = __ldg(sig + __ldg(a.frc_sig + e));
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      if (j == k) f[j] += c * s;
+  }
+}
+
 __device__ __forceinline__ void write_history(const StepArgs& a, int i, int r, double v) {
   if (r >= a.R_out) return;
   for (int k = lower_bound_i32(a.mon_row, a.n_mon, i); k < a.n_mon && __ldg(a.mon_row + k) == i; ++k) {

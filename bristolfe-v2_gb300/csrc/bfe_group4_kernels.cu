@@ -92,9 +92,11 @@ __device__ __forceinline__ void finish4(const StepArgs& a, int row, int c, float
     float2 d, err;
     two_sum2(u, make_float2(-p.x, -p.y), d, err);
     float2 inc = __ffma2_rn(q2, d, ac);                        // q d - Lp u
-    if (info & kRowForced)
-      inc = __fadd2_rn(inc, make_float2(forcing_sum<float>(a, row, c + 2 * h),
-                                        forcing_sum<float>(a, row, c + 2 * h + 1)));
+    if (info & kRowForced) {
+      float f[2];
+      forcing_sums(a, row, c + 2 * h, f);
+      inc = __fadd2_rn(inc, make_float2(f[0], f[1]));
+    }
     inc = __ffma2_rn(q2, err, inc);
     res[h] = __fadd2_rn(u, inc);
     vin[h] = a.int_base_prev ? __fadd2_rn(__fadd2_rn(d, err), inc) : __fadd2_rn(d, err);

@@ -121,6 +121,8 @@ cudaError_t launch_step(const StepArgs& a, int precision, cudaStream_t s);      
 // Kernel variants a batched run of (precision, R) may use, the default
 // first; writes them to out (at most 8) and returns their number.
 int batched_candidates(int precision, int R, bool have_groups, int max_bs, int* out);
+// The candidate of a march whose kernels are not timed.
+int untimed_candidate(int precision, int R, int n, bool have_groups, int max_bs);
 // The kernel whose outputs a non-finite march of R sources keeps: the group
 // form where R fills its lanes, else the slice kernel.
 int settled_variant(int precision, int64_t R, bool have_groups, int max_bs);

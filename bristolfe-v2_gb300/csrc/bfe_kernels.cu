@@ -447,6 +447,18 @@ int batched_candidates(int precision, int R, bool have_groups, int max_bs, int* 
   return k;
 }
 
+// A step of one wave of CTAs waits for its chains of loads, and more neighbours
+// in flight shorten them: adjoint of 6,642 DOF FP32 R = 24, 600 samples 21.1 ms
+// with variant 24, 19.6 with 26 (20.3 in the slice kernel), 26,082 DOF R = 40, 400
+// samples 21.8 / 20.6; 90,902 DOF R = 52 (5 waves of 12 CTAs per SM) 23.7 / 23.8,
+// 361,802 DOF 49.8 / 53.0.
+int untimed_candidate(int precision, int R, int n, bool have_groups, int max_bs) {
+  int cand[8];
+  batched_candidates(precision, R, have_groups, max_bs, cand);
+  const int64_t lanes = (int64_t)(n / max_bs) * ((R + 3) / 4);
+  return cand[0] == 24 && lanes <= (int64_t)sm_count() * 12 * 128 ? 26 : cand[0];
+}
+
 int settled_variant(int precision, int64_t R, bool have_groups, int max_bs) {
   if (!have_groups) return 0;
   if (precision == 0) return R % 16 ? 0 : R % 32 ? 3 : R % 64 ? 2 : 1;
