@@ -84,8 +84,8 @@ class BfeStats(ctypes.Structure):
 
 
 class BfeMarchInfo(ctypes.Structure):
-    """bfe_march_info: what a plan keeps for marches on the chip (bfe_plan_march_info)."""
-    _fields_ = [("partition_bytes", I64), ("partitions_built", I64)]
+    """bfe_march_info: how a plan was made, what it keeps for marches on the chip (bfe_plan_march_info)."""
+    _fields_ = [("partition_bytes", I64), ("partitions_built", I64), ("packed_on_gpu", I64)]
 
 
 SIGNATURES = {

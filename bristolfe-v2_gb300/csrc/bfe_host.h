@@ -184,6 +184,7 @@ struct bfe_plan {
   double time_limit_s = 0.0;        // wall-clock limit of a run (0 = none)
   int32_t march_fault = 0;          // BFE_MARCH_FAULT_*, for tests
   int64_t partitions_built = 0;     // on-chip partitions begun
+  bool packed_on_gpu = false;       // the sliced-ELL operator (bfe_pack.cu)
   int64_t steps_marched = 0;        // towards the first (onchip_due)
   bfe_host::DevBuf<int> d_flag;     // non-finite flag of the last run, and a march's wait-ran-out flag
   bfe_stats last{};

@@ -333,6 +333,7 @@ int bfe_plan_march_info(const bfe_plan* plan, bfe_march_info* out) {
   *out = bfe_march_info{};
   out->partition_bytes = plan->onchip->device_bytes() + plan->tiled->device_bytes();
   out->partitions_built = plan->partitions_built;
+  out->packed_on_gpu = plan->packed_on_gpu;
   return BFE_OK;
 }
 
@@ -580,6 +581,7 @@ int create_plan(Csr K, Csr C, Csr M, double dt, int32_t solver_mode, int32_t pre
                              stored, direct_rows)))
       return rc;
     total = pl->h_slice_ptr.back();
+    pl->packed_on_gpu = true;
   }
   const int n_pack = Kv ? 1 : plan_threads(n_slices, 1024);
   std::vector<Piece> pieces(n_pack);
@@ -935,15 +937,15 @@ int bfe_plan_create_ex(const bfe_sparse* Kv, const bfe_sparse* Cv, const bfe_spa
   Csr K, C, M;
   int rc;
   // A one-source plan packs K on the GPU (a v5 plan keeps K on the host).
-  // Whatever that path does not take or cannot do is left to the path below,
-  // which reports errors in its own order.
+  // What that path does not take, inputs it refuses or memory it lacks are left
+  // to the path below, which reports errors in its own order; a CUDA error of
+  // another kind is one.
   if ((flags & BFE_PLAN_ONE_SOURCE) && solver_mode != BFE_MODE_V5 && Kv && Kv->format == BFE_CSR && Kv->n_rows > 0 &&
       Kv->n_rows == Kv->n_cols && Kv->n_rows <= bfe::kMaxDof && Kv->nnz >= 0 && Kv->ptr && (Kv->nnz == 0 || (Kv->idx && Kv->val)) &&
       Kv->ptr[0] == 0 && Kv->ptr[Kv->n_rows] == Kv->nnz && to_csr(Cv, "C", C) == BFE_OK && to_csr(Mv, "M", M) == BFE_OK) {
     K.n = K.m = Kv->n_rows;
-    if (create_plan(std::move(K), std::move(C), std::move(M), dt, solver_mode, precision, dof_node, dof_type, flags, out,
-                    Kv) == BFE_OK)
-      return BFE_OK;
+    rc = create_plan(std::move(K), std::move(C), std::move(M), dt, solver_mode, precision, dof_node, dof_type, flags, out, Kv);
+    if (rc == BFE_OK || rc == BFE_ERR_CUDA) return rc;
     cudaGetLastError();
     *out = nullptr;
     K = Csr();

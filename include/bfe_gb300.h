@@ -450,11 +450,12 @@ enum {
 };
 int bfe_plan_set_march_fault(bfe_plan* plan, int32_t fault);
 
-/* What a plan keeps for marches that stay on the chip (no reference
- * counterpart). */
+/* How a plan was made, and what it keeps for marches that stay on the chip (no
+ * reference counterpart). */
 typedef struct bfe_march_info {
   int64_t partition_bytes;     /* device memory of its partitions of the operator */
   int64_t partitions_built;    /* partitions it began to build, used or not */
+  int64_t packed_on_gpu;       /* 1: its operator was packed on the GPU (one-source plans), 0: on the host */
 } bfe_march_info;
 int bfe_plan_march_info(const bfe_plan* plan, bfe_march_info* out);
 
