@@ -1,8 +1,6 @@
-// Group block-sparse step kernels (sm_103a): the packed-math warp-per-node
-// form (step_f32_group2, 3D and bs > 2) and the FP64 direct form
-// (step_f64_group), with the launchers the batched dispatch in
-// bfe_kernels.cu calls by variant number. The half-warp float4 form is in
-// bfe_group4_kernels.cu.
+// The FP64 group block-sparse step kernels (sm_103a, step_f64_group), with the
+// launcher the batched dispatch in bfe_kernels.cu calls by variant number. The
+// FP32 forms are in bfe_group4_kernels.cu.
 #include <cuda_runtime.h>
 #include <cstdint>
 
@@ -10,89 +8,6 @@
 #include "bfe_internal.h"
 
 namespace bfe {
-
-// ---------------------------------------------------------------------------
-// FP32 group block-sparse kernel, packed-math form (R a multiple of 64).
-// One warp per node of a group, each lane owns two right-hand sides held as
-// a float2 and every arithmetic operation is one packed FP32x2 instruction
-// (__ffma2_rn / __fadd2_rn: IEEE round-to-nearest per component, the same
-// results as two scalar operations). Coefficients are stored as pre-broadcast
-// float2 pairs ({c, c}). The neighbour differences are formed as
-// (u_own - u_nbr), so the accumulator holds -Lp u and the compensated update
-// needs no negation (f2sub, two_sum2: bfe_device.cuh).
-
-template <int BS, int UNROLL>
-__device__ __forceinline__ void group2_node(const StepArgs& a, const GroupArgs& gr, int gi,
-                                            int node, int lane) {
-  const int row0 = __ldg(gr.row0[gi] + node);
-  const int p0 = __ldg(gr.nptr[gi] + node), p1 = __ldg(gr.nptr[gi] + node + 1);
-  const int32_t* nrow = gr.nrow[gi];
-  const float2* coef = gr.coef2[gi];
-  const int R = a.R;
-  const size_t rstride = (size_t)R * sizeof(float);
-  for (int c = lane * 2; c < R; c += 64) {
-    const char* ub = reinterpret_cast<const char*>(static_cast<const float*>(a.u_n) + c);
-    float2 uo[BS], acc[BS];
-#pragma unroll
-    for (int k = 0; k < BS; ++k) {
-      uo[k] = __ldg(reinterpret_cast<const float2*>(ub + (size_t)(row0 + k) * rstride));
-      acc[k] = make_float2(0.f, 0.f);
-    }
-#pragma unroll UNROLL
-    for (int e = p0; e < p1; ++e) {
-      const char* nb = ub + (size_t)__ldg(nrow + e) * rstride;
-      const float2* cb = coef + (size_t)e * (BS * BS);
-#pragma unroll
-      for (int l = 0; l < BS; ++l) {
-        const float2 g = __ldg(reinterpret_cast<const float2*>(nb + l * rstride));
-        const float2 dn = f2sub(uo[l], g);                      // u_own - u_nbr
-#pragma unroll
-        for (int k = 0; k < BS; ++k) acc[k] = __ffma2_rn(__ldg(cb + k * BS + l), dn, acc[k]);
-      }
-    }
-    float* unew = static_cast<float*>(a.u_new);
-#pragma unroll
-    for (int k = 0; k < BS; ++k) {
-      const int row = row0 + k;
-      const uint32_t info = __ldg(a.rowinfo + row);
-      const float q = __ldg(static_cast<const float*>(a.rowc) + row);
-      const size_t o = (size_t)row * R + c;
-      const float2 up = __ldcs(reinterpret_cast<const float2*>(static_cast<const float*>(a.u_prev) + o));
-      float2 d, err;
-      two_sum2(uo[k], make_float2(-up.x, -up.y), d, err);
-      const float2 q2 = make_float2(q, q);
-      float2 inc = __ffma2_rn(q2, d, acc[k]);                    // q d - Lp u
-      if (info & kRowForced)
-        inc = __fadd2_rn(inc, make_float2(forcing_sum<float>(a, row, c), forcing_sum<float>(a, row, c + 1)));
-      inc = __ffma2_rn(q2, err, inc);
-      const float2 r = __fadd2_rn(uo[k], inc);
-      *reinterpret_cast<float2*>(unew + o) = r;
-      if (info & kRowInterface) {
-        const int t = lower_bound_i32(a.int_row, a.n_int, row);
-        const float2 vi = a.int_base_prev ? __fadd2_rn(__fadd2_rn(d, err), inc) : __fadd2_rn(d, err);
-        *reinterpret_cast<float2*>(static_cast<float*>(a.v_int) + (size_t)t * R + c) = vi;
-      } else if (info & kRowMonitored) {
-        write_history(a, row, c, (double)r.x);
-        write_history(a, row, c + 1, (double)r.y);
-      }
-    }
-  }
-}
-
-template <int MAXBS, int UNROLL, int MINB>
-__global__ void __launch_bounds__(256, MINB) step_f32_group2(StepArgs a, GroupArgs gr) {
-  const int lane = threadIdx.x & 31;
-  const int b = blockIdx.x;
-  int gi = 0;
-#pragma unroll
-  for (int k = 1; k < kMaxGroups; ++k)
-    if (k < gr.n_groups && b >= gr.blk_begin[k]) gi = k;
-  const int node = (b - gr.blk_begin[gi]) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (node >= gr.n_nodes[gi]) return;
-  if (gr.bs[gi] == 1) group2_node<1, UNROLL * 2>(a, gr, gi, node, lane);
-  else if (MAXBS == 2 || gr.bs[gi] == 2) group2_node<(MAXBS >= 2 ? 2 : 1), UNROLL>(a, gr, gi, node, lane);
-  else group2_node<MAXBS, UNROLL>(a, gr, gi, node, lane);
-}
 
 // FP64 group block-sparse kernel (direct form, the reference's arithmetic):
 // u_new = sum over the node's blocks (its own included) of B_block u_n
@@ -233,25 +148,6 @@ static cudaError_t launch_group64(const StepArgs& a, const GroupArgs& gr, int va
     else if (variant == 4) step_f64_group<0, 2, 6, 3, 1><<<blocks, 128, 0, st>>>(a, g);
     else step_f64_group<0, 2, 4, 3, 2><<<blocks, 128, 0, st>>>(a, g);
   }
-  return cudaGetLastError();
-}
-
-template <int MAXBS>
-static void launch_group2(const StepArgs& a, const GroupArgs& gr, int variant, cudaStream_t st) {
-  const int grid = gr.blk_begin[gr.n_groups];
-  switch (variant) {
-    case 9: step_f32_group2<MAXBS, 1, 1><<<grid, 256, 0, st>>>(a, gr); break;
-    case 10: step_f32_group2<MAXBS, 2, 1><<<grid, 256, 0, st>>>(a, gr); break;
-    case 11: step_f32_group2<MAXBS, 4, 1><<<grid, 256, 0, st>>>(a, gr); break;
-    case 12: step_f32_group2<MAXBS, 1, 4><<<grid, 256, 0, st>>>(a, gr); break;
-    case 13: step_f32_group2<MAXBS, 1, 6><<<grid, 256, 0, st>>>(a, gr); break;
-    default: step_f32_group2<MAXBS, 1, 8><<<grid, 256, 0, st>>>(a, gr); break;
-  }
-}
-
-cudaError_t launch_group2_variant(int maxbs, const StepArgs& a, const GroupArgs& gr, int variant, cudaStream_t st) {
-  if (maxbs <= 2) launch_group2<2>(a, gr, variant, st);
-  else launch_group2<3>(a, gr, variant, st);
   return cudaGetLastError();
 }
 

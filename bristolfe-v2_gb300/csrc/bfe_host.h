@@ -194,8 +194,7 @@ struct bfe_plan {
   // group block-sparse operator (FP32 difference form)
   bool have_groups = false;
   bfe::GroupArgs groups{};
-  bfe_host::DevBuf<int32_t> g_row0[bfe::kMaxGroups], g_nptr[bfe::kMaxGroups], g_nrow[bfe::kMaxGroups];
-  bfe_host::DevBuf<float2> g_coef2[bfe::kMaxGroups];
+  bfe_host::DevBuf<int32_t> g_nptr[bfe::kMaxGroups], g_nrow[bfe::kMaxGroups];
   bfe_host::DevBuf<int4> g_rec[bfe::kMaxGroups];
   bfe_host::DevBuf<float> g_coef[bfe::kMaxGroups];
   bfe_host::DevBuf<double> g_coef64[bfe::kMaxGroups];

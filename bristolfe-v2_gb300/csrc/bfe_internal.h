@@ -105,11 +105,9 @@ struct GroupArgs {
   int32_t bs[kMaxGroups];            // block size of each group (1..3)
   int32_t n_nodes[kMaxGroups];
   int32_t blk_begin[kMaxGroups + 1];
-  const int32_t* row0[kMaxGroups];   // first row of the group block of each node
   const int32_t* nptr[kMaxGroups];   // neighbour list of each node (n_nodes + 1)
   const int32_t* nrow[kMaxGroups];   // first row of each neighbour block
   const float* coef[kMaxGroups];     // BS*BS per neighbour block, [own k][neighbour l]
-  const float2* coef2[kMaxGroups];   // the coefficients as broadcast pairs {c, c}
   const int4* rec[kMaxGroups];       // per node {first row, first neighbour block, neighbour count, 0}
   int32_t lpn;                       // lanes per node of the any-R kernels
   int32_t ahead;                     // CTAs whose data a CTA asks L2 for (0 = none)
@@ -148,7 +146,6 @@ cudaError_t launch_nonfinite_check(const void* u, int64_t count, int precision, 
 // Group block-sparse kernel families (bfe_group_kernels.cu), by batched
 // variant: packed warp-per-node for block size maxbs (2 or 3), half-warp
 // float4 with lpn lanes per node (16, 8 or 4), FP64 direct form.
-cudaError_t launch_group2_variant(int maxbs, const StepArgs& a, const GroupArgs& gr, int variant, cudaStream_t s);
 cudaError_t launch_group4_variant(int lpn, const StepArgs& a, const GroupArgs& gr, int variant, cudaStream_t s);
 cudaError_t launch_group64_variant(const StepArgs& a, const GroupArgs& gr, int variant, cudaStream_t s);
 cudaError_t launch_groupn_variant(int maxbs, const StepArgs& a, const GroupArgs& gr, int variant, cudaStream_t s);

@@ -405,9 +405,7 @@ size_t batched_smem_bytes(int precision, int max_slice_entries) {
 //            R a multiple of 64 or R = 16, 32
 //   24 - 26  the float4 form for any R and block size, one, two or four
 //            neighbours in flight
-//   9 - 14   packed warp-per-node kernel step_f32_group2 (unroll 1, 2, 4;
-//            occupancy hints 4, 6, 8 CTAs), R a multiple of 64: only when forced,
-//            slower than 24 - 26 on every model
+//            (forced numbers from 9 on that name no kernel run 24)
 // The first candidate is the default; the autotuner keeps it unless another
 // is clearly faster on the live operator.
 int batched_candidates(int precision, int R, bool have_groups, int max_bs, int* out) {
@@ -436,9 +434,10 @@ int batched_candidates(int precision, int R, bool have_groups, int max_bs, int* 
     for (int v : {20, 22}) out[k++] = v;
     return k;
   }
-  // (3D nodes too, us per step of 24 / 25 / 26 and the best of 9 - 14: bricks R = 64
-  // of 14,553 DOF 23.2 / 22.2 / 18.5, 21.1; 46,128 DOF 36.5 / 37.0 / 34.4, 45.6;
-  // 202,878 DOF 123.8 / 139.8 / 135.8, 195.8)
+  // (3D nodes too, us per step of 24 / 25 / 26, bricks R = 64: 14,553 DOF 23.2 / 22.2
+  // / 18.5, 46,128 DOF 36.5 / 37.0 / 34.4, 202,878 DOF 123.8 / 139.8 / 135.8; the best
+  // of a warp-per-node form with packed pairs of coefficients took 21.1, 45.6 and
+  // 195.8 there)
   if (have_groups) {
     for (int v : {24, 25, 26}) out[k++] = v;
     return k;
@@ -463,7 +462,7 @@ int settled_variant(int precision, int64_t R, bool have_groups, int max_bs) {
   if (!have_groups) return 0;
   if (precision == 0) return R % 16 ? 0 : R % 32 ? 3 : R % 64 ? 2 : 1;
   if (max_bs <= 2 && (R % 64 == 0 || R == 16 || R == 32)) return 20;
-  return R % 64 ? 0 : 13;
+  return R % 64 ? 0 : 24;
 }
 
 // Prefetching pays where the three states do not fit in L2, so that a step's
@@ -518,9 +517,8 @@ cudaError_t launch_step_batched(const StepArgs& a, const GroupArgs* gr, int prec
     launch_groupn_variant(maxbs, a, *gr, variant, st);
   } else if (gr && half_warp && maxbs <= 2 && (r64 || r1632)) {
     launch_group4_variant(r64 ? 16 : a.R == 32 ? 8 : 4, a, *gr, variant, st);
-  } else if (gr && r64 && ((variant >= 9 && variant <= 14) || half_warp)) {
-    // 3-DOF node blocks take the warp-per-node form
-    launch_group2_variant(maxbs <= 2 ? 2 : 3, a, *gr, half_warp ? 14 : variant, st);
+  } else if (gr && variant >= 9) {                    // 20 and 22 where they do not apply
+    launch_groupn_variant(maxbs, a, *gr, 24, st);
   } else if (r64) {
     step_batched<float, 2><<<a.n_slices, threads, smem, st>>>(a);
   } else {

@@ -847,7 +847,6 @@ int create_plan(Csr K, Csr C, Csr M, double dt, int32_t solver_mode, int32_t pre
         pl->groups.n_nodes[gi] = (int32_t)row0s[gi].size();
         pl->groups.blk_begin[gi] = blocks;
         blocks += (int32_t)((row0s[gi].size() + 7) / 8);
-        CUDA_TRY(pl->g_row0[gi].upload(row0s[gi]));
         CUDA_TRY(pl->g_nptr[gi].upload(nptr));
         CUDA_TRY(pl->g_nrow[gi].upload(nrow));
         std::vector<int4> rec(row0s[gi].size());
@@ -855,7 +854,6 @@ int create_plan(Csr K, Csr C, Csr M, double dt, int32_t solver_mode, int32_t pre
           rec[a0] = make_int4(row0s[gi][a0], nptr[a0], nptr[a0 + 1] - nptr[a0], 0);
         CUDA_TRY(pl->g_rec[gi].upload(rec));
         pl->groups.rec[gi] = pl->g_rec[gi].p;
-        pl->groups.row0[gi] = pl->g_row0[gi].p;
         pl->groups.nptr[gi] = pl->g_nptr[gi].p;
         pl->groups.nrow[gi] = pl->g_nrow[gi].p;
         if (f64) {
@@ -864,17 +862,6 @@ int create_plan(Csr K, Csr C, Csr M, double dt, int32_t solver_mode, int32_t pre
           continue;
         }
         CUDA_TRY(pl->g_coef[gi].upload(coef));
-        // the coefficients as broadcast pairs {c, c}, filled on threads
-        const int64_t n_nodes_g = (int64_t)nodes.size();
-        std::vector<float2> coef2(coef.size());
-        const int n_fill = plan_threads(n_nodes_g, 4096);
-        if (!parallel_chunks(n_nodes_g, n_fill, [&](int, int64_t q0, int64_t q1) {
-              const size_t c0 = (size_t)nptr[q0] * bs * bs, c1 = (size_t)nptr[q1] * bs * bs;
-              for (size_t k = c0; k < c1; ++k) coef2[k] = make_float2(coef[k], coef[k]);
-            }))
-          return fail(BFE_ERR_OOM, "host allocation failed while building the group operator");
-        CUDA_TRY(pl->g_coef2[gi].upload(coef2));
-        pl->groups.coef2[gi] = pl->g_coef2[gi].p;
         pl->groups.coef[gi] = pl->g_coef[gi].p;
       }
       pl->groups.blk_begin[pl->groups.n_groups] = blocks;
