@@ -756,7 +756,7 @@ def adjoint_section(torch, bfe_gb300, model, n_fd=20, n_t=4000):
     from a seeded +-5 % stiffness perturbation (1 mm Gaussian bumps),
     gradient of the misfit w.r.t. per-element stiffness scale and density
     (backward segments of sqrt(N) steps; forward states kept on the device
-    when they fit) in FP32 and FP64, FP64 central differences on n_fd random
+    when they fit, the segments then four times as long) in FP32 and FP64, FP64 central differences on n_fd random
     elements of the sensitive region."""
     m = model.steel_plate_adjoint()
     ke, mh, ch, dof = m["element_data"]
@@ -782,7 +782,7 @@ def adjoint_section(torch, bfe_gb300, model, n_fd=20, n_t=4000):
             J, gs, gr = p.adjoint_gradient((ke, mh, ch, dof), t, srcs, sig, rec, obs)
             el = time.perf_counter() - t0
             kept = p.stats()["adjoint_kept"]
-            res["segment_steps"] = int(np.ceil(n_t / p.stats()["adjoint_segments"]))
+            res["segments"] = p.stats()["adjoint_segments"]
         grads[prec] = (J, gs, gr)
         res["fp32" if prec == "single" else "fp64"] = {
             "gradient_s": el, "misfit": J,

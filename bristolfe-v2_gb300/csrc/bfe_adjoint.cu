@@ -244,7 +244,8 @@ __global__ void __launch_bounds__(256) grad_stiff_w(int64_t n_el, const int32_t*
 // blocks of 128 threads per SM leave 92 registers, with which a step's loads
 // are all in flight (90,902 DOF, 16 sources, 1,000 steps: 4.2 ms against 6.2
 // with 256 threads at 76 registers; six blocks 5.5, eight 5.8, the next step's
-// loads ahead in registers 4.6 at best).
+// loads ahead in registers 4.6 at best). Elements of 3 and 9 DOFs keep 256
+// threads: no figure asked for another shape.
 template <int NDF> constexpr int kWfThreads = NDF == 6 ? 128 : 256;
 template <int NDF> constexpr int kWfBlocks = NDF == 6 ? 5 : 1;
 template <int NDF, int RK>

@@ -207,6 +207,9 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
   // setup and the ramps of three launches (90,902 DOF, 16 sources, 1,000 steps:
   // 28.6 ms in segments of 32, 27.6 of 64, 27.3 of 125, 27.6 of 250; 6,642 DOF,
   // 400 steps 4.1 ms of 20, 3.7 of 64 and more).
+  // Four times the terms enter a segment's compensated FP32 sums: gradients of
+  // 6,642 to 90,902 DOF and 300 to 4,000 samples are as far from FP64 (1e-7 to 3e-7)
+  // in both lengths, to four digits.
   bool keep_all = false;
   if (ckpt_every <= 0) {
     size_t free_b = 0, total_b = 0;

@@ -27,7 +27,8 @@
 //
 // The arithmetic of a row is that of step_f64_r1 / step_f32_r1 and
 // interface_fixup_r1 (bfe_kernels.cu), term for term in the same order, so
-// the results are the same bits.
+// the results are the same bits while the state is finite (entries that a node
+// block lacks are zeros here; execute() in bfe_run.cpp has the rest).
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <type_traits>
@@ -41,14 +42,15 @@ namespace {
 // ---------------------------------------------------------------------------
 // The march, one CTA of NT threads or fewer per part.
 //
-// What bounds it: FP64 rows the FP64 pipe (2 multiply-adds per clock and SM);
-// FP32 rows of large models the stream of operator chunks from L2 (about 4.5
-// TB/s over all SMs) and instruction issue; small models the exchange of a
-// step, about a microsecond from a value's store to its use in another CTA.
-// Measured per step of a 500-step run against one launch per step from a
-// graph, GB300 (us): plate of 40,602 DOF FP64 2.9 / 6.2, FP32 2.3 / 6.0;
-// coupled 241,579 DOF FP64 8.3 / 13.1, FP32 4.5 / 9.3; coupled 961,641 DOF
-// FP32 12.5 / 17.1; bricks of 202,878 DOF FP32 15.7 / 29.8.
+// What bounds it (ncu): FP64 rows the FP64 pipe (coupled 241,579 DOF: 65 % of
+// active cycles; plate of 40,602 DOF 37 %, the rest waits for the exchange, about
+// a microsecond from a value's store to its use in another CTA); FP32 rows of
+// large models instruction issue (coupled 961,641 DOF: 69 % of the issue slots,
+// beside 3.7 TB/s of operator chunks from L2); 3D ones that chunk stream (bricks of
+// 73,872 DOF: 3.1 TB/s, 40 % of the slots). Measured per step of a 500-step run
+// against one launch per step from a graph, GB300 (us): plate of 40,602 DOF FP64
+// 2.9 / 6.2, FP32 2.3 / 6.0; coupled 241,579 DOF FP64 8.3 / 13.1, FP32 4.5 / 9.3;
+// coupled 961,641 DOF FP32 12.5 / 17.1; bricks of 202,878 DOF FP32 15.7 / 29.8.
 //
 // Per step: rows (interface and exported slices first, so that
 // their values travel while the others are computed), interface correction,

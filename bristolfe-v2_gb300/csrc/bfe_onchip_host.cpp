@@ -15,8 +15,10 @@ constexpr int64_t kMinSlices = 4;
 // streamed chunks come from HBM as the step kernels' operator does: FP64
 // bricks of 202,878 DOF (163 MB) took 39 us per step against 35.5 with one
 // launch per step. FP64, whose blocks are known before they are built, stops
-// a little lower: coupled 961,641 DOF (96 MB) took 27.6 us against 25.6, while
-// 492,579 DOF (52 MB) took 14.2 against 19.3.
+// a little lower. Us per step on chip / step kernels (MB of 2^20): coupled
+// 592,202 DOF (57 MB) 14.8 / 18.0, 696,719 (67) 18.0 / 20.2, plate of 642,402 DOF (78)
+// 18.0 / 19.4, bricks of 122,034 DOF (83) 25.5 / 27.4, coupled 961,641 DOF (92) 27.6 /
+// 25.6.
 constexpr int64_t kMaxOperator = (int64_t)96 << 20, kMaxOperator64 = (int64_t)88 << 20;
 
 // FP32 rows of many entries (3D) whose blocks alone exceed the SMs' shared

@@ -19,7 +19,9 @@
 // written to global memory, [n][R] at m.out + k m.out_stride.
 //
 // Arithmetic and order are those of the group kernels (step_f32_groupn,
-// step_f64_group), so the results are the same bits.
+// step_f64_group), so the results are the same bits while the state is finite.
+// 90,902 DOF, R = 16 in tiles (ncu): 60 % of the issue slots, 46 % of the
+// shared-memory pipe.
 #include <cuda_runtime.h>
 #include <cstdint>
 
@@ -115,9 +117,9 @@ __device__ __forceinline__ void row_sums(double (&acc)[kRe], const unsigned char
   }
 }
 // Slices whose nodes all start at an even place of the window: both DOFs of a
-// neighbour (kind 2) come with one 16-byte load. Shared-memory reads bound the
-// rows (two lanes of a node read the same words, so 16 distinct ones per load
-// either way): 6.5 instead of 10.5 wavefronts a neighbour, 90,902 DOF R = 16
+// neighbour (kind 2) come with one 16-byte load, fewer instructions and
+// shared-memory wavefronts (two lanes of a node read the same words, so 16
+// distinct ones per load either way): 6.5 instead of 10.5 wavefronts a neighbour, 90,902 DOF R = 16
 // 16,000 -> 13,700 clocks of rows per step. Eight right-hand sides per lane in
 // place of four: no faster at R = 16 (12.3 us per step both), slower at R = 8
 // (6.7 / 5.7).
