@@ -186,6 +186,7 @@ struct bfe_plan {
   int64_t partitions_built = 0;     // on-chip partitions begun
   bool packed_on_gpu = false;       // the sliced-ELL operator (bfe_pack.cu)
   int64_t steps_marched = 0;        // towards the first (onchip_due)
+  int32_t mid_neighbours = 0, mid_last = 0;   // of the first group's middle node: neighbours, first row of the last
   bfe_host::DevBuf<int> d_flag;     // non-finite flag of the last run, and a march's wait-ran-out flag
   bfe_stats last{};
   // autotuned batched-kernel variant per R (chosen on the first run with that R)

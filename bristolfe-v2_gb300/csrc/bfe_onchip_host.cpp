@@ -659,14 +659,11 @@ bool onchip_multi_may_fit(const bfe_plan* pl, int64_t R, bool against_graph) {
   // (a part of a few rows fits with twice its rows as halo)
   const int64_t most = 3 * ((S + P - 1) / P) * bfe::kSlice;
   if (2 * R * most * es <= kSmemLimit / 2 && !(against_graph && too_many_words(pl->prec, R, most))) return true;
-  int32_t at[2] = {0, 0}, last = 0;
-  if (cudaMemcpy(at, pl->g_nptr[0].p + q, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost) != cudaSuccess || at[1] <= at[0] ||
-      cudaMemcpy(&last, pl->g_nrow[0].p + at[1] - 1, sizeof(int32_t), cudaMemcpyDeviceToHost) != cudaSuccess)
-    return true;
-  const int64_t len = std::max<int64_t>(1, last / bs - q), M = (N + len - 1) / len;
+  if (pl->mid_neighbours == 0) return true;
+  const int64_t len = std::max<int64_t>(1, pl->mid_last / bs - q), M = (N + len - 1) / len;
   const TileCut cut = tile_cut(S, P, M, (double)len, bs);
   const int64_t rows = (S + cut.px * cut.py - 1) / (cut.px * cut.py) * bfe::kSlice, halo = cut.halo * bs;
-  const int width = es == 8 ? (int)(pl->h_slice_ptr[S] / (S * bfe::kSlice)) : (at[1] - at[0]) * (int)bs;
+  const int width = es == 8 ? (int)(pl->h_slice_ptr[S] / (S * bfe::kSlice)) : pl->mid_neighbours * (int)bs;
   const int64_t block = es == 8 ? bfe::onchip_block_bound(pl->prec, width) : bfe::onchip_block_least(width, (int)bs);
   return 2 * R * (rows + halo) * es + 6 * rows + 4 * halo + rows / bfe::kSlice * block <= kSmemLimit &&
          !(against_graph && too_many_words(pl->prec, R, halo));

@@ -849,6 +849,11 @@ int create_plan(Csr K, Csr C, Csr M, double dt, int32_t solver_mode, int32_t pre
         blocks += (int32_t)((row0s[gi].size() + 7) / 8);
         CUDA_TRY(pl->g_nptr[gi].upload(nptr));
         CUDA_TRY(pl->g_nrow[gi].upload(nrow));
+        const size_t mid = row0s[gi].size() / 2;
+        if (gi == 0 && mid + 1 < nptr.size() && nptr[mid + 1] > nptr[mid]) {
+          pl->mid_neighbours = nptr[mid + 1] - nptr[mid];
+          pl->mid_last = nrow[nptr[mid + 1] - 1];
+        }
         std::vector<int4> rec(row0s[gi].size());
         for (size_t a0 = 0; a0 < rec.size(); ++a0)
           rec[a0] = make_int4(row0s[gi][a0], nptr[a0], nptr[a0 + 1] - nptr[a0], 0);

@@ -357,7 +357,7 @@ int march(bfe_plan* pl, RunSpec& rs, TimeLimit& limit, bool settled, bool& again
   } guard{&ev_step, &ev_aux};
   const bool timing = pl->timing;
   // Autotuner: on the first batched run with a given operator shape and R,
-  // time each candidate kernel (bfe::batched_candidates) on a few steps of
+  // time each candidate kernel (bfe::batched_candidates) on a step or a few of
   // the real operator - the state is still zero, and the march that follows
   // starts from rest again - and keep the fastest. The default (first)
   // candidate stays unless another is at least 2 % faster, so that near-ties
@@ -416,13 +416,18 @@ int march(bfe_plan* pl, RunSpec& rs, TimeLimit& limit, bool settled, bool& again
       for (int k = 0; k < nc; ++k) {
         const int v = cand[k];
         CUDA_TRY(launch_batched(grp, v));   // warm
-        CUDA_TRY(cudaEventRecord(e0, st));
-        for (int r = 0; r < 3; ++r) CUDA_TRY(launch_batched(grp, v));
-        CUDA_TRY(cudaEventRecord(e1, st));
-        CUDA_TRY(cudaEventSynchronize(e1));
+        stt.aux_launches++;
+        // of a long kernel one launch says enough, of a short one three
         float ms = 0;
-        CUDA_TRY(cudaEventElapsedTime(&ms, e0, e1));
-        stt.aux_launches += 4;
+        for (int count = 1; count <= 3 && ms < 0.3f; count += 2) {
+          CUDA_TRY(cudaEventRecord(e0, st));
+          for (int r = 0; r < count; ++r) CUDA_TRY(launch_batched(grp, v));
+          CUDA_TRY(cudaEventRecord(e1, st));
+          CUDA_TRY(cudaEventSynchronize(e1));
+          CUDA_TRY(cudaEventElapsedTime(&ms, e0, e1));
+          ms /= (float)count;
+          stt.aux_launches += count;
+        }
         if (k == 0) t_default = ms;
         if (ms < best) { best = ms; variant = v; }
       }
