@@ -362,8 +362,9 @@ int march(bfe_plan* pl, RunSpec& rs, TimeLimit& limit, bool settled, bool& again
   // starts from rest again - and keep the fastest. The default (first)
   // candidate stays unless another is at least 2 % faster, so that near-ties
   // do not flip between runs (3 % kept the FP64 group kernel on all-solid plates
-  // of 161,202 DOF, R = 64, where the slice kernel takes 255.3 us of 261.0). The choice is kept in the plan and for the
-  // process (g_tune_cache). BFE_VARIANT=<k> forces variant k (sweeps).
+  // of 161,202 DOF, R = 64, where the slice kernel takes 255.3 us of 261.0). The
+  // choice is kept in the plan and for the process (g_tune_cache).
+  // BFE_VARIANT=<k> forces variant k (sweeps).
   auto launch_batched = [&](const bfe::GroupArgs* grpp, int v) -> cudaError_t {
     return bfe::launch_step_batched(a, grpp, prec, pl->max_slice_entries, v, st);
   };
