@@ -473,8 +473,10 @@ int settled_variant(int precision, int64_t R, bool have_groups, int max_bs) {
 // 132.4 / 120.3, R = 256 453.5 / 443.3; states of 139 to 186 MB gain 1 to 10 %.
 // Where it loses: fewer than 16 right-hand sides of one- and two-DOF nodes
 // (R = 8, 2,674,573 DOF: 96.8 / 98.4: a request costs as much as the load),
-// several uneven passes over R (R = 96, 241,579 DOF: 91.6 / 93.4), and it does
-// nothing for FP64, which the FP64 pipe bounds (R = 64 271.2 / 272.4). The
+// several uneven passes over R on models of up to 360,000 DOF (R = 80 plate of
+// 161,202 DOF 51.1 / 55.1, R = 96 coupled 241,579 DOF 91.6 / 93.4; 961,641 DOF would
+// gain, 312 / 297, as bricks of 202,878 DOF, 207 / 200 at 200), and it does nothing
+// for FP64, which the FP64 pipe bounds (R = 64 271.2 / 272.4). The
 // distance is long enough for a DRAM miss and short enough that the data are
 // still in L2: 800 CTAs of 1,824 resident (400: 156.7, 1,200: 150.6, 2,000: 161 at
 // R = 64); the wide blocks of three-DOF nodes want 200 (R = 16, 1,778,478 DOF: 363
