@@ -176,17 +176,6 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
     }
     return true;
   };
-  auto gave_up = [&](bool& yes) -> int {            // after a synchronisation point
-    int e = 0;
-    CUDA_TRY(cudaMemcpy(&e, pl->d_flag.p + 1, sizeof(int), cudaMemcpyDeviceToHost));
-    yes = e != 0;
-    if (yes) {
-      onchip_give_up(pl, oc);
-      oc = nullptr;
-      CUDA_TRY(cudaMemsetAsync(pl->d_flag.p, 0, 2 * sizeof(int), st));
-    }
-    return BFE_OK;
-  };
   bfe::OnchipArgs of, oa;
   bool chip = onchip_multi_may_fit(pl, Rp, false) && c >= 8 && !pl->timing && !getenv("BFE_NO_GRAPH") && n_t < ((int64_t)1 << 30);
   // two marches of these steps (26,082 DOF, 60 samples: 7 to 14 us won back a
@@ -232,41 +221,49 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
   stt.adjoint_segments = n_seg;
   stt.adjoint_kept = keep_all ? 1 : 0;
   DevBuf<unsigned char> d_u, d_ck, d_all;
-  auto forward_steps = [&]() -> int {
-    for (int64_t t = ti0; t < n_t; ++t) {
-      af.ti = t;
-      af.u_prev = d_all.p + (size_t)(t - ti0) * sb;
-      af.u_n = d_all.p + (size_t)(t - ti0 + 1) * sb;
-      af.u_new = d_all.p + (size_t)(t - ti0 + 2) * sb;
-      if (int r = step(af)) return r;
-    }
-    return BFE_OK;
-  };
   if (keep_all) {
     CUDA_TRY(d_all.alloc((size_t)(steps + 2) * sb));
-    CUDA_TRY(cudaMemsetAsync(d_all.p, 0, 2 * sb, st));
-    chip = chip && chip_march(of, afc, ti0, 1, steps, true, nullptr, nullptr, d_all.p + 2 * sb);
-    if (!chip && (rc = forward_steps())) return rc;
   } else {
     CUDA_TRY(d_u.alloc(3 * sb));
-    CUDA_TRY(cudaMemsetAsync(d_u.p, 0, 3 * sb, st));
     CUDA_TRY(d_ck.alloc(2 * sb * n_seg));
-    unsigned char* U[3] = {d_u.p, d_u.p + sb, d_u.p + 2 * sb};
-    int ip = 0, ic = 1, iw = 2;
-    for (int64_t t = ti0; t < n_t; ++t) {
-      if ((t - ti0) % c == 0) {
-        const int64_t j = (t - ti0) / c;
-        CUDA_TRY(cudaMemcpyAsync(d_ck.p + 2 * sb * j, U[ip], sb, cudaMemcpyDeviceToDevice, st));
-        CUDA_TRY(cudaMemcpyAsync(d_ck.p + 2 * sb * j + sb, U[ic], sb, cudaMemcpyDeviceToDevice, st));
-      }
-      af.ti = t;
-      af.u_prev = U[ip];
-      af.u_n = U[ic];
-      af.u_new = U[iw];
-      if ((rc = step(af))) return rc;
-      const int tt = ip; ip = ic; ic = iw; iw = tt;
-    }
   }
+  // The forward march, and a check of its newest state for non-finite values.
+  auto forward = [&]() -> int {
+    unsigned char* newest;
+    if (keep_all) {
+      newest = d_all.p + (size_t)(steps + 1) * sb;
+      CUDA_TRY(cudaMemsetAsync(d_all.p, 0, 2 * sb, st));
+      chip = chip && chip_march(of, afc, ti0, 1, steps, true, nullptr, nullptr, d_all.p + 2 * sb);
+      for (int64_t t = ti0; t < n_t && !chip; ++t) {
+        af.ti = t;
+        af.u_prev = d_all.p + (size_t)(t - ti0) * sb;
+        af.u_n = d_all.p + (size_t)(t - ti0 + 1) * sb;
+        af.u_new = d_all.p + (size_t)(t - ti0 + 2) * sb;
+        if (int r = step(af)) return r;
+      }
+    } else {
+      CUDA_TRY(cudaMemsetAsync(d_u.p, 0, 3 * sb, st));
+      unsigned char* U[3] = {d_u.p, d_u.p + sb, d_u.p + 2 * sb};
+      int ip = 0, ic = 1, iw = 2;
+      for (int64_t t = ti0; t < n_t; ++t) {
+        if ((t - ti0) % c == 0) {
+          const int64_t j = (t - ti0) / c;
+          CUDA_TRY(cudaMemcpyAsync(d_ck.p + 2 * sb * j, U[ip], sb, cudaMemcpyDeviceToDevice, st));
+          CUDA_TRY(cudaMemcpyAsync(d_ck.p + 2 * sb * j + sb, U[ic], sb, cudaMemcpyDeviceToDevice, st));
+        }
+        af.ti = t;
+        af.u_prev = U[ip];
+        af.u_n = U[ic];
+        af.u_new = U[iw];
+        if (int r = step(af)) return r;
+        const int tt = ip; ip = ic; ic = iw; iw = tt;
+      }
+      newest = U[ic];
+    }
+    CUDA_TRY(bfe::launch_nonfinite_check(newest, n * Rp, prec, pl->d_flag.p, st));
+    return BFE_OK;
+  };
+  if ((rc = forward())) return rc;
   // element data on the device, prepared on the host while the forward
   // march runs (the plan's stream does not wait for the legacy stream)
   DevBuf<int32_t> d_dof;
@@ -343,15 +340,26 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
   std::vector<double> hist(hist_n);
   CUDA_TRY(cudaMemcpyAsync(hist.data(), d_hist.p, hist_n * sizeof(double), cudaMemcpyDeviceToHost, st));
   CUDA_TRY(cudaStreamSynchronize(st));
-  if (chip && keep_all) {
-    bool yes = false;
-    if ((rc = gave_up(yes))) return rc;
-    if (yes) {
-      chip = false;
-      if ((rc = forward_steps())) return rc;
-      CUDA_TRY(cudaMemcpyAsync(hist.data(), d_hist.p, hist_n * sizeof(double), cudaMemcpyDeviceToHost, st));
-      CUDA_TRY(cudaStreamSynchronize(st));
-    }
+  // once more in steps when a wait ran out, and by the kernels whose outputs a
+  // non-finite march keeps (execute() in bfe_run.cpp) when it became one
+  int flags[2] = {0, 0};
+  CUDA_TRY(cudaMemcpy(flags, pl->d_flag.p, 2 * sizeof(int), cudaMemcpyDeviceToHost));
+  bool again = flags[1] != 0;
+  if (flags[1]) {
+    onchip_give_up(pl, oc);
+    chip = false;
+  }
+  if (flags[0] && R > 1) {
+    const int keep = bfe::settled_variant(prec, R, pl->have_groups, grp ? bfe::group_max_bs(*grp) : 0);
+    again = again || (chip && keep_all) || (keep == 0 && variant != 0);
+    chip = false;
+    if (keep == 0) variant = stt.variant = 0;
+  }
+  if (again) {
+    CUDA_TRY(cudaMemsetAsync(pl->d_flag.p, 0, 2 * sizeof(int), st));
+    if ((rc = forward())) return rc;
+    CUDA_TRY(cudaMemcpyAsync(hist.data(), d_hist.p, hist_n * sizeof(double), cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaStreamSynchronize(st));
   }
   if (hist_out) std::memcpy(hist_out, hist.data(), hist_n * sizeof(double));
   const int64_t n_rsig = q * R;
@@ -473,9 +481,12 @@ int bfe_adjoint_gradient(bfe_plan* pl, int64_t n_el, int32_t ndf, const int64_t*
   if (rc) return rc;
   if (chip) {
     CUDA_TRY(cudaStreamSynchronize(st));
-    bool yes = false;
-    if ((rc = gave_up(yes))) return rc;
-    if (yes && (rc = sweep(false))) return rc;
+    int lost = 0;
+    CUDA_TRY(cudaMemcpy(&lost, pl->d_flag.p + 1, sizeof(int), cudaMemcpyDeviceToHost));
+    if (lost) {
+      onchip_give_up(pl, oc);
+      if ((rc = sweep(false))) return rc;
+    }
   }
   stt.step_launches = launches;
   CUDA_TRY(cudaMemcpyAsync(g_stiff, d_gs.p, n_el * sizeof(double), cudaMemcpyDeviceToHost, st));

@@ -108,3 +108,34 @@ def test_prescribed_displacements(bfe, models, prec, monkeypatch):
     monkeypatch.setenv("BFE_NO_GRAPH", "1")
     for a, b in zip(on, run()):
         _equal(a, b)
+
+
+@pytest.mark.parametrize("every", [0, 60])
+@pytest.mark.parametrize("prec", ["double", "single"])
+def test_adjoint(bfe, prec, every, monkeypatch):
+    """The history of an adjoint's forward march, kept or from checkpoints, is
+    that of the slice kernel, and the gradient does not depend on the route."""
+    from bfe_gb300 import model
+    m = model.steel_plate_adjoint(W=3e-3, H=1.5e-3, h=0.1e-3, n_src=3, n_rec=9, abs_wavelengths=0.3)
+    nt, scale = (700, 2.2) if prec == "double" else (400, 1.8)
+    dt = scale * m["dt"]
+    t, k = np.arange(nt) * dt, np.arange(nt)
+    s = np.sin(k / 3.0) * np.exp(-((k - 10) / 6.0) ** 2)
+    hi = model.global_indices(m["gl"], m["rec_nodes"], 2)
+    srcs = [model.global_indices(m["gl"], x, 2) for x in m["src_nodes"]]
+    obs = np.zeros((hi.size, nt, 3), order="F")
+
+    def run():
+        with bfe.Plan(m["K"], m["C"], m["M"], dt, bfe.VEL_CURRENT, prec, m["gl"]) as plan:
+            return plan.adjoint_gradient(m["element_data"], t, srcs, s, hi, obs, ckpt_every=every, return_history=True)
+
+    monkeypatch.delenv("BFE_NO_GRAPH", raising=False)
+    on = run()
+    monkeypatch.setenv("BFE_NO_GRAPH", "1")
+    off = run()
+    for a, b in zip(on[1:3], off[1:3]):
+        assert np.array_equal(a, b, equal_nan=True)
+    _equal(on[3], off[3])
+    monkeypatch.setenv("BFE_VARIANT", "0")
+    with bfe.Plan(m["K"], m["C"], m["M"], dt, bfe.VEL_CURRENT, prec, m["gl"]) as plan:
+        _equal(on[3], _unstable(bfe, lambda: plan.run_batched(t, srcs, s, hi)))
